@@ -1,0 +1,781 @@
+// pd_tile.cu — the whole projective-dynamics solve of an outer iteration
+// (lg x [local step + Chebyshev-accelerated R2 steps as weighted-Jacobi
+// sweeps]) in one cooperative launch over compact tiles of rows.
+//
+// What bounds the solve is not bandwidth but the 31 data exchanges of every
+// local-global iteration.  So:
+//   * a tile is a compact block of rows (tile_plan.cpp): only the rows within
+//     the stencil's reach of its edge are exchanged, and most tiles' rows need
+//     nothing from outside;
+//   * an exchanged vertex is one 16-byte word that carries the phase's tag, so
+//     a reader polls the data itself: one L2 write and one L2 read per phase
+//     instead of data, a release of a flag, polls of the flag and a copy;
+//   * two CTAs share an SM, so one tile sums while the other waits;
+//   * matrix values, column offsets and both copies of the iterate stay in
+//     shared memory for the launch; the local step's neighbour differences come
+//     from the same memory (positions, or their high and low halves, occupy the
+//     two copies while no iterate does), and right-hand sides, inverse diagonals
+//     and the Chebyshev history in registers.
+//
+// Measured (GB300, one solve, before: the row-block launches of pd_persistent.cuh
+// or, FP64, one launch per sweep): mixed 16x16 0.97 -> 0.35 ms, 64x64 0.96 -> 0.49,
+// 181x181 1.31 -> 0.69, 512x512 4.35 -> 3.42, four 256x256 10.6 -> 3.4; FP32 96x96
+// 1.34 -> 0.47; FP64 64x64 2.88 -> 1.62, 257x257 9.2 -> 8.0.
+//
+// Double buffering of the exchange: in phase p a tile writes its boundary rows
+// to parity p & 1 and then reads its halo there.  It overwrites that parity in
+// phase p + 2, after it has read every neighbour's phase p + 1, which a
+// neighbour publishes only after a CTA barrier that follows its own reads of
+// phase p (the plan makes reading mutual).
+//
+// Every wait is clock-bounded: past the limit it raises kErrBarrier, the tile
+// leaves together at its next barrier, and the others' waits end on the error
+// or their own limit.
+#include <algorithm>
+#include <type_traits>
+
+#include "kernels.cuh"
+#include "svd3.cuh"
+#include "tile.h"
+
+namespace pdipc {
+
+namespace {
+
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ TileWord ld_word(const TileWord* p) {
+    TileWord w;
+    asm volatile(
+        "{\n\t.reg .b128 v;\n\t"
+        "ld.relaxed.gpu.global.b128 v, [%2];\n\t"
+        "mov.b128 {%0, %1}, v;\n\t}"
+        : "=l"(w.lo), "=l"(w.hi)
+        : "l"(p)
+        : "memory");
+    return w;
+}
+__device__ __forceinline__ void st_word(TileWord* p, unsigned long long lo, unsigned long long hi) {
+    asm volatile(
+        "{\n\t.reg .b128 v;\n\t"
+        "mov.b128 v, {%1, %2};\n\t"
+        "st.relaxed.gpu.global.b128 [%0], v;\n\t}" ::"l"(p),
+        "l"(lo), "l"(hi)
+        : "memory");
+}
+__device__ __forceinline__ unsigned long long pack2(unsigned a, unsigned b) {
+    return (unsigned long long)a | ((unsigned long long)b << 32);
+}
+
+
+// ---- the arithmetic, with its rounding spelled out: the results keep the bits
+// of the launches this solve stands in for (one per sweep in the direct form, the
+// band in the correction form), whatever the compiler would contract ----
+__device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float add_(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_(double a, double b) { return __dadd_rn(a, b); }
+// (1 - w) c + w ((s + b) / D): one weighted-Jacobi update
+template <bool kCorr, typename T>
+__device__ __forceinline__ T jacobi(T om1, T c, T w, T s, T b, T id) {
+    const T t = mul_(add_(s, b), id);
+    return kCorr ? fma_(w, t, mul_(om1, c)) : fma_(om1, c, mul_(w, t));
+}
+template <typename T>
+__device__ __forceinline__ T norm2(T x, T y, T z) {
+    return fma_(z, z, fma_(x, x, mul_(y, y)));
+}
+// Sum2 (common.cuh) with the products it adds fused
+struct Acc {
+    float s = 0.f, c = 0.f;
+    __device__ __forceinline__ void step(float t, float bp, float e) {
+        c = add_(c, add_(add_(s, -add_(t, -bp)), e));
+        s = t;
+    }
+    __device__ __forceinline__ void add(float x) {
+        const float t = add_(s, x), bp = add_(t, -s);
+        step(t, bp, add_(x, -bp));
+    }
+    __device__ __forceinline__ void add(float a, float b) {
+        const float t = fma_(a, b, s), bp = add_(t, -s);
+        step(t, bp, fma_(a, b, -bp));
+    }
+    __device__ __forceinline__ float value() const { return add_(s, c); }
+};
+
+template <typename T>
+struct alignas(2 * sizeof(T)) Pair {
+    T x, y;
+};
+
+// the values of consecutive entries of one row: 16 bytes
+template <typename T>
+struct alignas(16) Group {
+    T v[16 / sizeof(T)];
+};
+
+template <typename S>
+__device__ __forceinline__ V4<S> ldg_state(const V4<S>* p, int i) {  // written by this thread or an earlier kernel
+    return p[i];
+}
+
+// One tet's strain projection (solveVolumetricStrainConstraintKernel,
+// PdIpcGpuFunc.cu:439-599): w R G of its four vertices (three of a cloth
+// triangle's strain element) to Out.  Out of line: once per tet and
+// local-global iteration, its registers stay out of the sweeps.
+template <typename S, bool kCorr>
+__device__ __noinline__ void tile_tet(int e, const int4* __restrict__ Tets, const float* __restrict__ Idm,
+                                      const float* __restrict__ W, const V4<S>* P, const V4<float>* Ph,
+                                      const V4<float>* Pl, V4<float>* Out) {
+    const int4 q = Tets[e];
+    const bool tri = q.w < 0;
+    const int id[4] = {q.x, q.y, q.z, tri ? q.x : q.w};
+    float Ds[3][3];
+    if constexpr (kCorr) {
+        const float4 h0 = __ldcg((const float4*)Ph + id[0]), l0 = __ldcg((const float4*)Pl + id[0]);
+        for (int c = 0; c < 3; ++c) {
+            const float4 h = __ldcg((const float4*)Ph + id[c + 1]), l = __ldcg((const float4*)Pl + id[c + 1]);
+            Ds[0][c] = diff_ff(h.x, l.x, h0.x, l0.x);
+            Ds[1][c] = diff_ff(h.y, l.y, h0.y, l0.y);
+            Ds[2][c] = diff_ff(h.z, l.z, h0.z, l0.z);
+        }
+    } else {
+        const float4 x0 = __ldcg((const float4*)P + id[0]);
+        for (int c = 0; c < 3; ++c) {
+            const float4 x = __ldcg((const float4*)P + id[c + 1]);
+            Ds[0][c] = x.x - x0.x;
+            Ds[1][c] = x.y - x0.y;
+            Ds[2][c] = x.z - x0.z;
+        }
+    }
+    float idm[9];
+    for (int k = 0; k < 9; ++k) idm[k] = __ldg(Idm + 9 * (size_t)e + k);
+    float out[4][3];
+    if (tri) {
+        const float D2[3][2] = {{Ds[0][0], Ds[0][1]}, {Ds[1][0], Ds[1][1]}, {Ds[2][0], Ds[2][1]}};
+        float o3[3][3];
+        svd::tri_project<float>(D2, idm, __ldg(W + e), o3);
+        for (int c = 0; c < 3; ++c)
+            for (int r = 0; r < 3; ++r) out[c][r] = o3[c][r];
+        out[3][0] = out[3][1] = out[3][2] = 0.f;
+    } else {
+        svd::tet_project<float>(Ds, idm, __ldg(W + e), out);
+    }
+    for (int c = 0; c < 4; ++c)
+        __stcg((float4*)Out + 4 * (size_t)e + c, make_float4(out[c][0], out[c][1], out[c][2], 0.f));
+}
+
+template <typename T, typename S, bool kCorr, bool kTets, int R>
+__global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_constant__ TileArgs<T, S> a) {
+    constexpr int kW = kTileWords<T, S>;
+    constexpr int kG = kTileGroup<T>;
+    constexpr int kUnroll = R == 1 ? 2 : 1;  // two rows per thread leave no registers for more
+    extern __shared__ __align__(16) unsigned char smem[];
+    if (outer_stopped(a.gate)) return;
+    const int tile = (int)blockIdx.x + a.lo;
+    const TileInfo ti = a.tiles[tile];
+    if (a.instStop && a.instStop[ti.model]) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+
+    // ---- shared memory: values, offset patterns, two vectors of the local
+    // vertices as (x, y) pairs and z ----
+    auto a16 = [](size_t b) { return (b + 15) / 16 * 16; };
+    T* sval = reinterpret_cast<T*>(smem);
+    int16_t* spat = reinterpret_cast<int16_t*>(smem + a16((size_t)ti.nent * sizeof(T)));
+    unsigned char* vec0 =
+        smem + a16((size_t)ti.nent * sizeof(T)) + a16((size_t)ti.npat * a.patStride * sizeof(int16_t));
+    const int vecBytes = (int)a16(3 * (size_t)ti.nloc * sizeof(T));
+    auto XY = [&](int b) { return reinterpret_cast<Pair<T>*>(vec0 + b * vecBytes); };
+    auto Z = [&](int b) { return reinterpret_cast<T*>(XY(b) + ti.nloc); };
+    for (int q = threadIdx.x; q < ti.nent; q += blockDim.x) sval[q] = __ldg(a.val + ti.ent0 + q);
+    for (int q = threadIdx.x; q < ti.npat * a.patStride; q += blockDim.x)
+        spat[q] = __ldg(a.pat + (size_t)ti.pat0 * a.patStride + q);
+
+    // ---- this thread's rows: slice r nw + warp, this lane ----
+    // gr: row (-1 none); lp: its place; pe: its pattern's first element; eo/el:
+    // first entry and entries per row of its slice
+    int gr[R], lp[R], pe[R], eo[R], el[R];
+    int pub[R];
+    T id[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int s = r * nw + warp;
+        gr[r] = -1;
+        lp[r] = pe[r] = eo[r] = el[r] = 0;
+        pub[r] = 0;
+        id[r] = T(0);
+        if (s < ti.nslice) {
+            const TileSlot sl = a.slots[ti.slot0 + 32 * s + lane];
+            const TileSlice sc = a.slices[ti.slice0 + s];
+            gr[r] = sl.row;
+            lp[r] = sl.pos;
+            pe[r] = sl.pat;
+            pub[r] = sl.pub;
+            eo[r] = sc.off + kG * lane;
+            el[r] = sl.row >= 0 ? sc.len : 0;
+        }
+        if (gr[r] >= 0) id[r] = T(1) / ((a.Delastic[gr[r]] + a.Dinert[gr[r]]) + a.CollDiag[gr[r]]);
+    }
+    // the first halo row this thread polls (others through the table)
+    const TileHalo h0 = (int)threadIdx.x < ti.nhalo ? a.halo[ti.halo0 + threadIdx.x] : TileHalo{-1, 0};
+
+    auto put = [&](int b, int q, T x, T y, T z) {
+        XY(b)[q] = Pair<T>{x, y};
+        Z(b)[q] = z;
+    };
+    unsigned tag = a.epoch0;  // of the last phase published
+    auto words = [&](int w) { return a.ex + ((size_t)(tag & 1u) * kW + w) * a.nsim; };
+    // publish one vector of row g under the current tag (slot w of the phase's words)
+    auto publish = [&](int w, int g, T x, T y, T z) {
+        if constexpr (sizeof(T) == 4) {
+            st_word(words(w) + g, pack2(__float_as_uint(x), __float_as_uint(y)), pack2(__float_as_uint(z), tag));
+        } else {
+            st_word(words(0) + g, (unsigned long long)__double_as_longlong(x), tag);
+            st_word(words(1) + g, (unsigned long long)__double_as_longlong(y), tag);
+            st_word(words(2) + g, (unsigned long long)__double_as_longlong(z), tag);
+        }
+    };
+    // wait for the word at p to carry the current tag
+    auto wait_word = [&](const TileWord* p, TileWord& w) -> bool {
+        w = ld_word(p);
+        auto there = [&]() { return sizeof(T) == 4 ? (unsigned)(w.hi >> 32) == tag : (unsigned)w.hi == tag; };
+        if (there()) return true;
+        const long long t0 = clock64();
+        for (int n = 1;; ++n) {
+            w = ld_word(p);
+            if (there()) return true;
+            if (clock64() - t0 > a.timeout) {
+                atomicOr(a.err, (unsigned)kErrBarrier);
+                return false;
+            }
+            if ((n & 15) == 0 && (ld_acquire(a.err) & kErrBarrier)) return false;
+        }
+    };
+    // the halo of the current phase into vector b (and the second half into b2)
+    auto fetch_one = [&](int row, int pos, int b, int b2) -> bool {
+        TileWord w;
+        if constexpr (sizeof(T) == 4) {
+            if (!wait_word(words(0) + row, w)) return false;
+            put(b, pos, __uint_as_float((unsigned)w.lo), __uint_as_float((unsigned)(w.lo >> 32)),
+                __uint_as_float((unsigned)w.hi));
+            if (b2 >= 0) {
+                if (!wait_word(words(kW - 1) + row, w)) return false;
+                put(b2, pos, __uint_as_float((unsigned)w.lo), __uint_as_float((unsigned)(w.lo >> 32)),
+                    __uint_as_float((unsigned)w.hi));
+            }
+        } else {
+            TileWord wy, wz;
+            if (!wait_word(words(0) + row, w) || !wait_word(words(1) + row, wy) || !wait_word(words(2) + row, wz))
+                return false;
+            put(b, pos, __longlong_as_double((long long)w.lo), __longlong_as_double((long long)wy.lo),
+                __longlong_as_double((long long)wz.lo));
+        }
+        return true;
+    };
+    auto fetch = [&](int b, int b2) -> bool {
+        bool ok = h0.row < 0 || fetch_one(h0.row, h0.pos, b, b2);
+        for (int h = (int)(threadIdx.x + blockDim.x); ok && h < ti.nhalo; h += blockDim.x) {
+            const TileHalo q = a.halo[ti.halo0 + h];
+            ok = fetch_one(q.row, q.pos, b, b2);
+        }
+        return ok;
+    };
+    // end of a phase: the halo is in, every own value is written; false: the launch ends
+    auto arrive = [&](int b, int b2 = -1) -> bool {
+        if (ti.nhalo == 0) {
+            __syncthreads();
+            return true;
+        }
+        return !__syncthreads_or(!fetch(b, b2));
+    };
+    // tets only: what neighbours wrote to global memory before their same call
+    // is visible after it (release and acquire of the tiles' phase counts)
+    unsigned fl = a.flag0;
+    auto global_sync = [&]() -> bool {
+        __syncthreads();
+        ++fl;
+        if (threadIdx.x == 0) st_release(a.flags + tile, fl);
+        bool ok = true;
+        const long long t0 = clock64();
+        for (int q = (int)threadIdx.x; ok && q < ti.nnbr; q += blockDim.x) {
+            const int n = a.nbr[ti.nbr0 + q];
+            while ((int)(ld_acquire(a.flags + n) - fl) < 0) {
+                if (clock64() - t0 > a.timeout || (ld_acquire(a.err) & kErrBarrier)) {
+                    atomicOr(a.err, (unsigned)kErrBarrier);
+                    ok = false;
+                    break;
+                }
+            }
+        }
+        return !__syncthreads_or(!ok);
+    };
+
+    // sum_k N_ik z_k of owned row r over vector b, in the stored order.  Batches
+    // of entries whose loads are all in flight before the first sum: a 16-byte
+    // load brings eight offsets (one address in most warps), another the values
+    // of kG entries.
+    auto row_sum = [&](int r, int b, T& s0, T& s1, T& s2) {
+        s0 = T(0);
+        s1 = T(0);
+        s2 = T(0);
+        const Group<T>* vp = reinterpret_cast<const Group<T>*>(sval + eo[r]);
+        const uint2* pp = reinterpret_cast<const uint2*>(spat + pe[r]);
+        const Pair<T>* xy = XY(b) + lp[r];
+        const T* z = Z(b) + lp[r];
+        auto batch = [&](auto nc, const unsigned* o, const T* v) {
+            constexpr int n = decltype(nc)::value;
+            Pair<T> p[n];
+            T q[n];
+#pragma unroll
+            for (int k = 0; k < n; ++k) {
+                const int j = (k & 1) ? (int)o[k >> 1] >> 16 : (int)(short)(o[k >> 1] & 0xffffu);
+                p[k] = xy[j];
+                q[k] = z[j];
+            }
+#pragma unroll
+            for (int k = 0; k < n; ++k) {
+                s0 = fma_(v[k], p[k].x, s0);
+                s1 = fma_(v[k], p[k].y, s1);
+                s2 = fma_(v[k], q[k], s2);
+            }
+        };
+        int k = 0;
+        if constexpr (kG == 4 && R == 1) {
+            for (; k + 8 <= el[r]; k += 8) {
+                const uint4 o4 = *reinterpret_cast<const uint4*>(pp + (k >> 2));
+                const unsigned o[4] = {o4.x, o4.y, o4.z, o4.w};
+                const Group<T> va = vp[(k >> 2) * 32], vb = vp[(k >> 2) * 32 + 32];
+                T v[8];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    v[q] = va.v[q];
+                    v[4 + q] = vb.v[q];
+                }
+                batch(std::integral_constant<int, 8>(), o, v);
+            }
+        }
+#pragma unroll(kUnroll)
+        for (; k < el[r]; k += 4) {
+            const uint2 o2 = pp[k >> 2];
+            const unsigned o[2] = {o2.x, o2.y};
+            T v[4];
+#pragma unroll
+            for (int g = 0; g < 4 / kG; ++g) {
+                const Group<T> va = vp[(k / kG + g) * 32];
+#pragma unroll
+                for (int q = 0; q < kG; ++q) v[g * kG + q] = va.v[q];
+            }
+            batch(std::integral_constant<int, 4>(), o, v);
+        }
+    };
+    const T w = a.relax, om1 = T(1) - a.relax;
+
+    // ---- positions of the local vertices: own rows and halo ----
+    auto load_pos = [&](int row, int pos) {
+        if constexpr (kCorr) {
+            const V4<T> h = ldg_state(a.Ph, row), l = ldg_state(a.Pl, row);
+            put(0, pos, h.x, h.y, h.z);
+            put(1, pos, l.x, l.y, l.z);
+        } else {
+            const V4<S> x = ldg_state(a.P, row);
+            put(0, pos, x.x, x.y, x.z);
+        }
+    };
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if (gr[r] >= 0) load_pos(gr[r], lp[r]);
+    for (int h = threadIdx.x; h < ti.nhalo; h += blockDim.x) {
+        const TileHalo q = a.halo[ti.halo0 + h];
+        load_pos(q.row, q.pos);
+    }
+    __syncthreads();
+
+    int cur = 0;  // the vector that holds the positions (direct form) at the start of an iteration
+    for (int lg = 0; lg < a.lg; ++lg) {
+        if constexpr (kTets) {
+            for (int q = threadIdx.x; q < ti.ntet; q += blockDim.x)
+                tile_tet<S, kCorr>(a.tet[ti.tet0 + q], a.Tets, a.TetIdm, a.TetW, a.P, a.Ph, a.Pl, a.TetOut);
+            if (!global_sync()) return;
+        }
+        // correction form: the residual's matrix part of owned row r, in column
+        // order (the entries below the row's own block, those in it, those above)
+        auto matrix_part = [&](int r, Acc& r0, Acc& r1, Acc& r2) {
+            const T* vp = sval + eo[r];
+            const int16_t* pp = spat + pe[r];
+            const Pair<T>*hp = XY(0) + lp[r], *lpp = XY(1) + lp[r];
+            const T *hz = Z(0) + lp[r], *lz = Z(1) + lp[r];
+            const T h0x = hp[0].x, h0y = hp[0].y, h0z = hz[0], l0x = lpp[0].x, l0y = lpp[0].y, l0z = lz[0];
+            auto part = [&](int k0, int k1) {
+#pragma unroll 4
+                for (int k = k0; k < k1; ++k) {
+                    const T v = vp[32 * (k & ~(kG - 1)) + (k & (kG - 1))];
+                    const int j = pp[k];
+                    const Pair<T> p = hp[j], q = lpp[j];
+                    r0.add(v, diff_ff(p.x, q.x, h0x, l0x));
+                    r1.add(v, diff_ff(p.y, q.y, h0y, l0y));
+                    r2.add(v, diff_ff(hz[j], lz[j], h0z, l0z));
+                }
+            };
+            const int ka = (pub[r] >> 8) & 255, kb = (pub[r] >> 16) & 255;
+            part(ka, kb);
+            part(0, ka);
+            part(kb, el[r]);
+        };
+        // ---- local step: curvature vectors, springs and (correction form without
+        // a third vector) the matrix part of the residual, all from shared memory ----
+        T aq[R][3], rh[R][3], cx[R][3], px[R][3];
+        Acc acc[kCorr ? R : 1][3];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            aq[r][0] = aq[r][1] = aq[r][2] = T(0);
+            rh[r][0] = rh[r][1] = rh[r][2] = T(0);
+            cx[r][0] = cx[r][1] = cx[r][2] = T(0);
+            px[r][0] = px[r][1] = px[r][2] = T(0);
+            if (gr[r] < 0) continue;
+            const int i = gr[r];
+            const int s = r * nw + warp;
+            const int st = __ldg(a.stencil + ti.slice0 + s) + lane, nst = pub[r] >> 24;
+            const T strain = a.Strain[i];
+            T a0, a1, a2;
+            if constexpr (kCorr) {
+                Acc r0, r1, r2;
+                const V4<S> x = ldg_state(a.P, i);
+                {
+                    const V4<S> y = ldg_state(a.Rhs0, i);
+                    const T di = a.Dinert[i];
+                    r0.add(di, (T)(y.x - x.x));
+                    r1.add(di, (T)(y.y - x.y));
+                    r2.add(di, (T)(y.z - x.z));
+                }
+                const int pf = a.PinFlag[i];
+                if (pf >= 0) {
+                    const V4<S> xr = ldg_state(a.Xrest, i);
+                    const T k = a.PinK[pf];
+                    r0.add(k, (T)(xr.x - x.x));
+                    r1.add(k, (T)(xr.y - x.y));
+                    r2.add(k, (T)(xr.z - x.z));
+                }
+                {
+                    const T dc = a.CollDiag[i];
+                    if (dc != T(0)) {  // else both terms are zero
+                    const V4<T> c = ldg_state(a.CollRhs, i);
+                    const V4<S> xo = ldg_state(a.Pold, i);
+                    r0.add(c.x);
+                    r0.add(dc, (T)(xo.x - x.x));
+                    r1.add(c.y);
+                    r1.add(dc, (T)(xo.y - x.y));
+                    r2.add(c.z);
+                    r2.add(dc, (T)(xo.z - x.z));
+                    }
+                }
+                const Pair<T>*hp = XY(0) + lp[r], *lpp = XY(1) + lp[r];
+                const T *hz = Z(0) + lp[r], *lz = Z(1) + lp[r];
+                const T h0x = hp[0].x, h0y = hp[0].y, h0z = hz[0], l0x = lpp[0].x, l0y = lpp[0].y, l0z = lz[0];
+                a0 = a1 = a2 = T(0);
+#pragma unroll 4
+                for (int k = 0; k < nst; ++k) {
+                    const int j = __ldg(a.stPos + st + 32 * k);
+                    const Pair<T> hj = hp[j], lj = lpp[j];
+                    const T hjz = hz[j], ljz = lz[j];
+                    const T d0 = diff_ff(h0x, l0x, hj.x, lj.x), d1 = diff_ff(h0y, l0y, hj.y, lj.y),
+                            d2 = diff_ff(h0z, l0z, hjz, ljz);
+                    const T wl = __ldg(a.stLbo + st + 32 * k);
+                    a0 = fma_(wl, -d0, a0);
+                    a1 = fma_(wl, -d1, a1);
+                    a2 = fma_(wl, -d2, a2);
+                    const T cl = dsqrt(norm2(d0, d1, d2));
+                    const T rc = strain * (__ldg(a.stRest + st + 32 * k) / cl);
+                    r0.add(rc, d0);
+                    r1.add(rc, d1);
+                    r2.add(rc, d2);
+                }
+                if (!a.third) matrix_part(r, r0, r1, r2);
+                acc[r][0] = r0;
+                acc[r][1] = r1;
+                acc[r][2] = r2;
+            } else {
+                const Pair<T>* xp = XY(cur) + lp[r];
+                const T* xz = Z(cur) + lp[r];
+                const T x0 = xp[0].x, x1 = xp[0].y, x2 = xz[0];
+                const T l0 = a.tLbo0[i];
+                a0 = x0 * l0;
+                a1 = x1 * l0;
+                a2 = x2 * l0;
+                T t0 = T(0), t1 = T(0), t2 = T(0);
+#pragma unroll 4
+                for (int k = 0; k < nst; ++k) {
+                    const int j = __ldg(a.stPos + st + 32 * k);
+                    const Pair<T> xj = xp[j];
+                    const T xjz = xz[j];
+                    const T l = __ldg(a.stLbo + st + 32 * k);
+                    a0 = fma_(xj.x, l, a0);
+                    a1 = fma_(xj.y, l, a1);
+                    a2 = fma_(xjz, l, a2);
+                    const T d0 = x0 - xj.x, d1 = x1 - xj.y, d2 = x2 - xjz;
+                    const T cl = dsqrt(norm2(d0, d1, d2));
+                    const T rc = strain * (__ldg(a.stRest + st + 32 * k) / cl);
+                    t0 = fma_(rc, d0, t0);
+                    t1 = fma_(rc, d1, t1);
+                    t2 = fma_(rc, d2, t2);
+                }
+                rh[r][0] = t0;
+                rh[r][1] = t1;
+                rh[r][2] = t2;
+                cx[r][0] = x0;
+                cx[r][1] = x1;
+                cx[r][2] = x2;
+                if (a.tape) a.tape[(size_t)lg * a.nsim + i] = V4<T>{x0, x1, x2, T(0)};
+            }
+            const T nrm = dsqrt(norm2(a0, a1, a2));
+            if (nrm >= T(1e-10)) {
+                const T c = a.CurvNorm[i] / nrm;
+                a0 *= c;
+                a1 *= c;
+                a2 *= c;
+            }
+            aq[r][0] = a0;
+            aq[r][1] = a1;
+            aq[r][2] = a2;
+        }
+        // ---- the curvature vectors go into the third vector, or where the
+        // positions' high halves were (correction form), or into the free vector
+        // (direct form) ----
+        const int qb = kCorr ? (a.third ? 2 : 0) : cur ^ 1;
+        if (kCorr && !a.third) __syncthreads();
+        ++tag;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (gr[r] >= 0) {
+                if (pub[r] & 1) publish(0, gr[r], aq[r][0], aq[r][1], aq[r][2]);
+                put(qb, lp[r], aq[r][0], aq[r][1], aq[r][2]);
+            }
+        if (!arrive(qb)) return;
+        // ---- bending, then the right-hand side (direct) or residual (correction) ----
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (gr[r] < 0) continue;
+            const int i = gr[r];
+            const int st = __ldg(a.stencil + ti.slice0 + r * nw + warp) + lane, nst = pub[r] >> 24;
+            const Pair<T>* qp = XY(qb) + lp[r];
+            const T* qz = Z(qb) + lp[r];
+            const T b0 = a.tBend0[i];
+            if constexpr (kCorr) {
+                Acc r0 = acc[r][0], r1 = acc[r][1], r2 = acc[r][2];
+                r0.add(b0, aq[r][0]);
+                r1.add(b0, aq[r][1]);
+                r2.add(b0, aq[r][2]);
+#pragma unroll 4
+                for (int k = 0; k < nst; ++k) {
+                    const int j = __ldg(a.stPos + st + 32 * k);
+                    const T bt = __ldg(a.stBend + st + 32 * k);
+                    r0.add(bt, qp[j].x);
+                    r1.add(bt, qp[j].y);
+                    r2.add(bt, qz[j]);
+                }
+                if constexpr (kTets)
+                    for (int q = a.vtPtr[i]; q < a.vtPtr[i + 1]; ++q) {
+                        const float4 t = __ldcg((const float4*)a.TetOut + a.vtIdx[q]);
+                        r0.add(t.x);
+                        r1.add(t.y);
+                        r2.add(t.z);
+                    }
+                if (a.third) matrix_part(r, r0, r1, r2);
+                rh[r][0] = r0.value();
+                rh[r][1] = r1.value();
+                rh[r][2] = r2.value();
+            } else {
+                T t0 = rh[r][0], t1 = rh[r][1], t2 = rh[r][2];
+                t0 = fma_(b0, aq[r][0], t0);
+                t1 = fma_(b0, aq[r][1], t1);
+                t2 = fma_(b0, aq[r][2], t2);
+                const V4<S> q0 = ldg_state(a.Rhs0, i);
+                T u0 = q0.x + t0, u1 = q0.y + t1, u2 = q0.z + t2;
+#pragma unroll 4
+                for (int k = 0; k < nst; ++k) {
+                    const int j = __ldg(a.stPos + st + 32 * k);
+                    const T bt = __ldg(a.stBend + st + 32 * k);
+                    u0 = fma_(bt, qp[j].x, u0);
+                    u1 = fma_(bt, qp[j].y, u1);
+                    u2 = fma_(bt, qz[j], u2);
+                }
+                if constexpr (kTets)
+                    for (int q = a.vtPtr[i]; q < a.vtPtr[i + 1]; ++q) {
+                        const float4 t = __ldcg((const float4*)a.TetOut + a.vtIdx[q]);
+                        u0 += t.x;
+                        u1 += t.y;
+                        u2 += t.z;
+                    }
+                const V4<T> cr = ldg_state(a.CollRhs, i);
+                u0 += cr.x;
+                u1 += cr.y;
+                u2 += cr.z;
+                const V4<T> pn = ldg_state(a.PinRhs, i);
+                u0 += pn.x;
+                u1 += pn.y;
+                u2 += pn.z;
+                rh[r][0] = u0;
+                rh[r][1] = u1;
+                rh[r][2] = u2;
+            }
+        }
+
+        // ---- Chebyshev-accelerated R2 iteration as two J sweeps per step ----
+        // direct form: on x from the positions; correction form: on delta from 0
+        ++tag;
+        {
+            T y[R][3];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                T s0 = T(0), s1 = T(0), s2 = T(0);
+                if (!kCorr) row_sum(r, cur, s0, s1, s2);
+                y[r][0] = jacobi<kCorr>(om1, cx[r][0], w, s0, rh[r][0], id[r]);
+                y[r][1] = jacobi<kCorr>(om1, cx[r][1], w, s1, rh[r][1], id[r]);
+                y[r][2] = jacobi<kCorr>(om1, cx[r][2], w, s2, rh[r][2], id[r]);
+                if (pub[r] & 1) publish(0, gr[r], y[r][0], y[r][1], y[r][2]);
+            }
+            // the curvature vectors (direct form), or the positions, have been read
+            if (!kCorr || a.third) __syncthreads();
+            cur = kCorr ? 1 : cur ^ 1;
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (gr[r] >= 0) put(cur, lp[r], y[r][0], y[r][1], y[r][2]);
+        }
+        if (!arrive(cur)) return;
+        for (int it = 0; it < a.cheby; ++it) {
+            const bool last = it == a.cheby - 1;
+            const T om = a.omega[it];
+            // x = S(y), Chebyshev-combined with the step before the last
+            ++tag;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                T s0, s1, s2, n[3];
+                row_sum(r, cur, s0, s1, s2);
+                const Pair<T> yxy = XY(cur)[lp[r]];
+                const T yz = Z(cur)[lp[r]];
+                n[0] = jacobi<kCorr>(om1, yxy.x, w, s0, rh[r][0], id[r]);
+                n[1] = jacobi<kCorr>(om1, yxy.y, w, s1, rh[r][1], id[r]);
+                n[2] = jacobi<kCorr>(om1, yz, w, s2, rh[r][2], id[r]);
+                if (it > 0) {
+                    n[0] = fma_(om, add_(n[0], -px[r][0]), px[r][0]);
+                    n[1] = fma_(om, add_(n[1], -px[r][1]), px[r][1]);
+                    n[2] = fma_(om, add_(n[2], -px[r][2]), px[r][2]);
+                }
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    px[r][c] = cx[r][c];
+                    cx[r][c] = n[c];
+                }
+                if (gr[r] < 0) continue;
+                if (!(kCorr && last)) {
+                    if (pub[r] & 1) publish(0, gr[r], n[0], n[1], n[2]);
+                    put(cur ^ 1, lp[r], n[0], n[1], n[2]);
+                }
+                if (!kCorr && last && (kTets || lg == a.lg - 1)) a.P[gr[r]] = V4<S>{n[0], n[1], n[2], S(0)};
+            }
+            if (last) break;
+            cur ^= 1;
+            if (!arrive(cur)) return;
+            // y = S(x)
+            ++tag;
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                T s0, s1, s2;
+                row_sum(r, cur, s0, s1, s2);
+                const T y0 = jacobi<kCorr>(om1, cx[r][0], w, s0, rh[r][0], id[r]);
+                const T y1 = jacobi<kCorr>(om1, cx[r][1], w, s1, rh[r][1], id[r]);
+                const T y2 = jacobi<kCorr>(om1, cx[r][2], w, s2, rh[r][2], id[r]);
+                if (gr[r] < 0) continue;
+                if (pub[r] & 1) publish(0, gr[r], y0, y1, y2);
+                put(cur ^ 1, lp[r], y0, y1, y2);
+            }
+            cur ^= 1;
+            if (!arrive(cur)) return;
+        }
+        // ---- the new positions ----
+        if constexpr (kCorr) {
+            __syncthreads();  // both vectors have been read
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                if (gr[r] < 0) continue;
+                const V4<S> x = ldg_state(a.P, gr[r]);
+                const S q0 = x.x + (S)cx[r][0], q1 = x.y + (S)cx[r][1], q2 = x.z + (S)cx[r][2];
+                a.P[gr[r]] = V4<S>{q0, q1, q2, S(0)};
+                float hx, lx, hy, ly, hz, lz;
+                split_ff(q0, hx, lx);
+                split_ff(q1, hy, ly);
+                split_ff(q2, hz, lz);
+                if (kTets || lg == a.lg - 1) {
+                    a.Ph[gr[r]] = V4<T>{hx, hy, hz, T(0)};
+                    a.Pl[gr[r]] = V4<T>{lx, ly, lz, T(0)};
+                }
+                if (pub[r] & 1) {
+                    publish(0, gr[r], hx, hy, hz);
+                    publish(1, gr[r], lx, ly, lz);
+                }
+                put(0, lp[r], hx, hy, hz);
+                put(1, lp[r], lx, ly, lz);
+            }
+            if (lg == a.lg - 1) break;
+            if (!arrive(0, 1)) return;
+        } else {
+            cur ^= 1;
+            if (lg == a.lg - 1) break;
+            if (!arrive(cur)) return;
+        }
+        if constexpr (kTets)
+            if (!global_sync()) return;
+    }
+}
+
+template <typename T, typename S, bool kCorr>
+const void* tile_kernel(int R, bool tets) {
+    if constexpr (sizeof(T) == 8) {
+        if (tets || R != 1) return nullptr;
+        return (const void*)k_pd_tile<T, S, kCorr, false, 1>;
+    } else {
+        if (R != 1 && R != 2) return nullptr;
+        if (tets) return R == 1 ? (const void*)k_pd_tile<T, S, kCorr, true, 1> : (const void*)k_pd_tile<T, S, kCorr, true, 2>;
+        return R == 1 ? (const void*)k_pd_tile<T, S, kCorr, false, 1> : (const void*)k_pd_tile<T, S, kCorr, false, 2>;
+    }
+}
+
+}  // namespace
+
+template <typename T, typename S>
+int tile_residents(int R, bool tets, int threads, size_t smem, int sms) {
+    const void* f = tile_kernel<T, S, !std::is_same<T, S>::value>(R, tets);
+    if (!f || threads > kTileMaxWarps * 32) return 0;
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(smem, 1)) !=
+        cudaSuccess)
+        return 0;
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem) != cudaSuccess) return 0;
+    return per_sm * sms;
+}
+
+template <typename T, typename S>
+cudaError_t launch_pd_tile(const TileArgs<T, S>& args, int tiles, int R, bool tets, int threads, size_t smem,
+                           cudaStream_t s) {
+    const void* f = tile_kernel<T, S, !std::is_same<T, S>::value>(R, tets);
+    if (!f || tiles < 1) return cudaErrorInvalidConfiguration;
+    void* params[] = {(void*)&args};
+    return cudaLaunchCooperativeKernel(f, dim3(tiles), dim3(threads), params, smem, s);
+}
+
+#define PDIPC_INST_TILE(T, S)                                                                     \
+    template int tile_residents<T, S>(int, bool, int, size_t, int);                               \
+    template cudaError_t launch_pd_tile<T, S>(const TileArgs<T, S>&, int, int, bool, int, size_t, \
+                                              cudaStream_t);
+PDIPC_INST_TILE(float, float)
+PDIPC_INST_TILE(float, double)
+PDIPC_INST_TILE(double, double)
+
+}  // namespace pdipc

@@ -40,6 +40,7 @@ struct PlanChoice {
     bool band = false;        // the iterate's column band in shared memory (correction form)
     bool l1_gather = true;
     bool local_sync = true;
+    bool tile = false;        // compact tiles of rows (pd_tile.cu); the other fields are then fixed
 };
 
 // A launch of the plan: CTAs [cta_lo, cta_hi], rows [row0, row1).

@@ -26,6 +26,7 @@
 #include "kernels.cuh"
 #include "persistent.h"
 #include "solver.h"
+#include "tile.h"
 
 namespace pdipc {
 
@@ -80,6 +81,7 @@ public:
         const long long u = us > 0 ? (long long)us : 2000000ll;
         wait_cycles_ = std::max(1ll, u * (long long)clock_khz_ / 1000ll);
         if constexpr (std::is_same<T, float>::value) pargs_.timeout = wait_cycles_;
+        targs_.timeout = wait_cycles_;
     }
 
     pdipc_status init(const HostTables& H, const pdipc_params& p, std::string& err) override {
@@ -417,12 +419,12 @@ private:
     };
 
     void fill_tuning_record() {
-        tuning_.pd_rows_per_thread = plan_.enabled ? plan_.rows_per_thread : 0;
-        tuning_.pd_ctas = plan_.enabled ? plan_.ctas : 0;
-        tuning_.pd_launches = plan_.enabled ? (int)groups_.size() : 0;
-        tuning_.pd_band = plan_.enabled && plan_.own_max > 0;
-        tuning_.pd_l1_gather = plan_.enabled && plan_.l1_gather;
-        tuning_.pd_local_sync = plan_.enabled && plan_.local_sync;
+        tuning_.pd_rows_per_thread = tile_on_ ? tile_.rows_per_thread : plan_.enabled ? plan_.rows_per_thread : 0;
+        tuning_.pd_ctas = tile_on_ ? (int)tile_.tiles.size() : plan_.enabled ? plan_.ctas : 0;
+        tuning_.pd_launches = tile_on_ ? (int)tile_.groups.size() : plan_.enabled ? (int)groups_.size() : 0;
+        tuning_.pd_band = tile_on_ ? kCorrection : plan_.enabled && plan_.own_max > 0;
+        tuning_.pd_l1_gather = tile_on_ || (plan_.enabled && plan_.l1_gather);
+        tuning_.pd_local_sync = tile_on_ || (plan_.enabled && plan_.local_sync);
         tuning_.cand_grid = c_.cand_grid;
         tuning_.traverse_block = c_.trav_block;
         tuning_.expand_block = c_.expand_block;
@@ -430,6 +432,11 @@ private:
 
     PlanChoice current_choice() const {
         PlanChoice ch;
+        if (tile_on_) {
+            ch.rows_per_thread = tile_.rows_per_thread;
+            ch.tile = true;
+            return ch;
+        }
         if (!plan_.enabled) return ch;
         ch.rows_per_thread = plan_.rows_per_thread;
         ch.band = plan_.own_max > 0;
@@ -452,7 +459,7 @@ private:
             return e;
         };
         auto solve = [&]() -> cudaError_t {
-            if (plan_.enabled) return launch_persistent();
+            if (persistent_on()) return launch_persistent();
             enqueue_pd();
             return cudaGetLastError();
         };
@@ -472,7 +479,7 @@ private:
         PD_CK(cudaStreamSynchronize(s_));
         if (pin_->err) {  // a device wait gave up: this configuration is not usable here
             PD_CK(cudaMemsetAsync(d_.ErrFlags, 0, sizeof(unsigned int), s_));
-            PD_CK(cudaMemsetAsync(pBar_ + 1, 0, sizeof(unsigned), s_));
+            if (pBar_) PD_CK(cudaMemsetAsync(pBar_ + 1, 0, sizeof(unsigned), s_));
             *ms_out = -1.f;
             return PDIPC_OK;
         }
@@ -530,9 +537,8 @@ private:
             }
         }
         if (cached) {
-            pdipc_status r = plan_persistent(H, err, best.pd.rows_per_thread ? &best.pd : nullptr);
+            pdipc_status r = apply_choice(H, best.pd, err);
             if (r != PDIPC_OK) return r;
-            if (best.pd.rows_per_thread == 0) plan_ = PersistPlan();
             c_.cand_grid = best.cand_grid;
             c_.trav_block = best.trav_block;
             c_.expand_block = best.expand_block;
@@ -567,34 +573,35 @@ private:
         std::vector<PlanChoice> pds;
         pds.push_back(current_choice());  // the default first
         for (const PlanChoice& c : plan_choices_)
-            if (!(c.rows_per_thread == pds[0].rows_per_thread && c.band == pds[0].band &&
-                  c.l1_gather == pds[0].l1_gather && c.local_sync == pds[0].local_sync))
+            if (pds[0].tile || !(c.rows_per_thread == pds[0].rows_per_thread && c.band == pds[0].band &&
+                                 c.l1_gather == pds[0].l1_gather && c.local_sync == pds[0].local_sync))
                 pds.push_back(c);
         if (pds[0].rows_per_thread != 0) pds.push_back(PlanChoice{});  // one launch per sweep
         float bestMs = -1.f;
         for (size_t k = 0; k < pds.size(); ++k) {
-            pdipc_status r = plan_persistent(H, err, pds[k].rows_per_thread ? &pds[k] : nullptr);
+            pdipc_status r = apply_choice(H, pds[k], err);
             if (r != PDIPC_OK) return r;
-            if (pds[k].rows_per_thread == 0) plan_ = PersistPlan();
-            else if (!plan_.enabled) continue;
+            if (pds[k].rows_per_thread != 0 && !persistent_on()) continue;
             float ms = -1.f;
             r = time_pd_solve(start, startH, startL, 3, &ms, err);
             if (r != PDIPC_OK) return r;
             ++tuning_.candidates_timed;
             if (std::getenv("PDIPC_AUTOTUNE_LOG"))  // every timed PD configuration, on stderr
-                std::fprintf(stderr, "pdipc autotune: PD rows/thread %d band %d l1 %d nbr-sync %d ctas %d launches %d: %.4f ms\n",
-                             plan_.enabled ? plan_.rows_per_thread : 0, plan_.enabled && plan_.own_max > 0,
+                std::fprintf(stderr,
+                             "pdipc autotune: PD rows/thread %d tile %d band %d l1 %d nbr-sync %d ctas %d launches %d: "
+                             "%.4f ms\n",
+                             pds[k].rows_per_thread, tile_on_, plan_.enabled && plan_.own_max > 0,
                              plan_.enabled && plan_.l1_gather, plan_.enabled && plan_.local_sync,
-                             plan_.enabled ? plan_.ctas : 0, plan_.enabled ? (int)groups_.size() : 0, ms);
+                             tile_on_ ? (int)tile_.tiles.size() : plan_.enabled ? plan_.ctas : 0,
+                             tile_on_ ? (int)tile_.groups.size() : plan_.enabled ? (int)groups_.size() : 0, ms);
             if (k == 0) tuning_.pd_default_ms = ms;
             if (ms > 0.f && (bestMs < 0.f || ms < bestMs)) {
                 bestMs = ms;
                 best.pd = pds[k];
             }
         }
-        pdipc_status r = plan_persistent(H, err, best.pd.rows_per_thread ? &best.pd : nullptr);
+        pdipc_status r = apply_choice(H, best.pd, err);
         if (r != PDIPC_OK) return r;
-        if (best.pd.rows_per_thread == 0) plan_ = PersistPlan();
         tuning_.pd_solve_ms = bestMs;
         // ---- the collision kernels' launch shapes, over the current candidates ----
         PD_CK(cudaMemcpyAsync(d_.P, saveP, sizeof(V4<TC>) * ns, cudaMemcpyDeviceToDevice, s_));
@@ -757,8 +764,10 @@ public:
         s->device_bytes = bytes_;
         s->kernel_launches = launches_;
         s->device_ms = device_ms_;
-        s->pd_path = plan_.enabled ? (plan_.own_max > 0 ? 3 : plan_.matrix_in_smem ? 2 : 1) : 0;
-        s->pd_ctas = plan_.enabled ? plan_.ctas : 0;
+        s->pd_path = tile_on_ ? (kCorrection ? 3 : 2)
+                     : plan_.enabled ? (plan_.own_max > 0 ? 3 : plan_.matrix_in_smem ? 2 : 1)
+                                     : 0;
+        s->pd_ctas = tile_on_ ? (int)tile_.tiles.size() : plan_.enabled ? plan_.ctas : 0;
         s->pd_solves = pd_solves_;
         s->pd_solve_ms = pd_ms_;
         s->pd_solve_bytes = pd_bytes_;
@@ -906,7 +915,7 @@ public:
         if (r == PDIPC_OK) r = put_state(X, V, err);
         if (r != PDIPC_OK) return r;
         launch_predict(d_, (TC)c_.dt, s_);
-        if (plan_.enabled) PD_CK(launch_persistent());
+        if (persistent_on()) PD_CK(launch_persistent());
         else enqueue_pd();
         r = get_positions(out, err);
         pdipc_status r2 = put_state(saveX.data(), saveV.data(), err);
@@ -1153,6 +1162,7 @@ private:
                     om = omega_next(rho2, om);
                 }
             }
+            if (tile_on_) launch_diag(d, s_);  // the tiled solve keeps its diagonal in registers
             launch_adj_step_begin(d, invt, adj_pb_, adj_vb_, adj_r0b_, s_);
             const size_t vb = sizeof(V4<TC>) * ns;
             for (int l = adj_tape_n_ - 1; l >= 0; --l) {
@@ -1404,7 +1414,13 @@ private:
         dfree(pSCol_);
         dfree(pSVal_);
         groups_.clear();
-        if (!std::is_same<T, float>::value || !prm_.persistent || c_.cheby >= kMaxCheby) return PDIPC_OK;
+        tile_on_ = false;
+        if (!prm_.persistent || c_.cheby >= kMaxCheby) return PDIPC_OK;
+        if (force && force->tile) {
+            tile_on_ = tile_.ok;
+            return PDIPC_OK;
+        }
+        if constexpr (!std::is_same<T, float>::value) return plan_tiles(H, 0, err);
         Dev<T, TC>& d = d_;
         const int ns = d.nsim;
         int dev = 0, nsm = 0, smem_optin = 0, coop = 0;
@@ -1423,24 +1439,6 @@ private:
         for (int sl = 0; sl < nsl; ++sl) {
             for (int lane = 0; lane < kSlice; ++lane) slen[sl] = std::max(slen[sl], row_len(row_of(sl * kSlice + lane)));
             soff[sl + 1] = soff[sl] + kSlice * slen[sl];
-        }
-        {
-            std::vector<int> pcol((size_t)std::max(soff[nsl], 1), 0);
-            std::vector<T> pval((size_t)std::max(soff[nsl], 1), T(0));
-            for (int sl = 0; sl < nsl; ++sl)
-                for (int lane = 0; lane < kSlice; ++lane) {
-                    const int r = row_of(sl * kSlice + lane), len = row_len(r);
-                    for (int k = 0; k < slen[sl]; ++k) {
-                        const size_t at = (size_t)soff[sl] + (size_t)kSlice * k + lane;
-                        const int e = r < ns ? H.nPtr[r] + std::min(k, std::max(len - 1, 0)) : 0;
-                        pcol[at] = len > 0 ? H.nCol[e] : std::min(r, ns - 1);
-                        pval[at] = k < len ? (T)H.nVal[e] : T(0);
-                    }
-                }
-            PD_CK(up(pSOff_, soff));
-            PD_CK(up(pSLen_, slen));
-            PD_CK(up(pSCol_, pcol));
-            PD_CK(up(pSVal_, pval));
         }
         // distinct column-offset patterns of the rows
         int patW = 0;
@@ -1647,7 +1645,31 @@ private:
                 break;
             }
         }
+        if (!force && prm_.persistent == 1) {
+            // compact tiles where a partition fits; a row sums in the order of
+            // the configuration they stand in for, so the results keep its bits
+            pdipc_status r = plan_tiles(H, pick && pick->ch.band ? pick->spc * kSlice : 0, err);
+            if (r != PDIPC_OK || tile_on_) return r;
+        }
         if (!pick) return PDIPC_OK;
+        {
+            std::vector<int> pcol((size_t)std::max(soff[nsl], 1), 0);
+            std::vector<T> pval((size_t)std::max(soff[nsl], 1), T(0));
+            for (int sl = 0; sl < nsl; ++sl)
+                for (int lane = 0; lane < kSlice; ++lane) {
+                    const int r = row_of(sl * kSlice + lane), len = row_len(r);
+                    for (int k = 0; k < slen[sl]; ++k) {
+                        const size_t at = (size_t)soff[sl] + (size_t)kSlice * k + lane;
+                        const int e = r < ns ? H.nPtr[r] + std::min(k, std::max(len - 1, 0)) : 0;
+                        pcol[at] = len > 0 ? H.nCol[e] : std::min(r, ns - 1);
+                        pval[at] = k < len ? (T)H.nVal[e] : T(0);
+                    }
+                }
+            PD_CK(up(pSOff_, soff));
+            PD_CK(up(pSLen_, slen));
+            PD_CK(up(pSCol_, pcol));
+            PD_CK(up(pSVal_, pval));
+        }
         plan_.enabled = true;
         plan_.matrix_in_smem = pick->smem_mat;
         plan_.l1_gather = pick->ch.l1_gather;
@@ -1859,8 +1881,161 @@ private:
         return PDIPC_OK;
     }
 
+    // ---------------- tiled PD solve (pd_tile.cu) ----------------
+    bool persistent_on() const { return plan_.enabled || tile_on_; }
+
+    // A configuration of the PD solve by name (the autotuner).
+    pdipc_status apply_choice(const HostTables& H, const PlanChoice& ch, std::string& err) {
+        if (ch.rows_per_thread != 0) return plan_persistent(H, err, &ch);
+        plan_ = PersistPlan();
+        tile_on_ = false;
+        return PDIPC_OK;
+    }
+
+    // The tile partition and its tables (order_block: build_tile_plan), built
+    // once per context; leaves tile_on_ false when no partition fits.  The FP64
+    // form is built for cloths under the scene's own stopping rule.
+    pdipc_status plan_tiles(const HostTables& H, int order_block, std::string& err) {
+        constexpr bool fp64 = std::is_same<T, double>::value;
+        if (prm_.persistent != 1 || H.nsim == 0 || (fp64 && (H.ntet > 0 || prm_.instance_stop))) return PDIPC_OK;
+        int dev = 0, nsm = 0, coop = 0, sm_smem = 0, reserved = 0;
+        PD_CK(cudaGetDevice(&dev));
+        PD_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        PD_CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+        PD_CK(cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+        PD_CK(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
+        if (!coop) return PDIPC_OK;
+        TileLimits lim;
+        lim.value_bytes = (int)sizeof(T);
+        lim.vectors = kCorrection ? 3 : 2;
+        lim.max_warps = kTileMaxWarps;
+        lim.max_rows_per_thread = fp64 ? 1 : 2;
+        lim.min_rows = fp64 ? 32 : 128;
+        lim.co_resident = 2 * nsm;
+        lim.smem = (size_t)(sm_smem / 2 - reserved);
+        if (prm_.pd_group_ctas > 0) lim.group_cap = prm_.pd_group_ctas;
+        build_tile_plan(H, lim, order_block, tile_);
+        if (!tile_.ok) return PDIPC_OK;
+        const int held = tile_residents<T, TC>(tile_.rows_per_thread, H.ntet > 0, tile_.threads, tile_.smem_bytes, nsm);
+        for (const TileGroup& g : tile_.groups)
+            if (g.hi - g.lo + 1 > held) tile_.ok = false;
+        if (!tile_.ok) return PDIPC_OK;
+        Dev<T, TC>& d = d_;
+        TileArgs<T, TC>& a = targs_;
+        TileInfo* tiles = nullptr;
+        TileSlot* slots = nullptr;
+        TileSlice* slices = nullptr;
+        TileHalo* halo = nullptr;
+        T *val = nullptr, *rest = nullptr, *lbo = nullptr, *bend = nullptr;
+        int16_t *pat = nullptr, *pos = nullptr;
+        int *nbr = nullptr, *tet = nullptr, *stencil = nullptr;
+        PD_CK(up(tiles, tile_.tiles));
+        PD_CK(up(slots, tile_.slots));
+        PD_CK(up(slices, tile_.slices));
+        PD_CK(up(val, conv(tile_.val)));
+        PD_CK(up(pat, tile_.pat));
+        PD_CK(up(stencil, tile_.stencil));
+        PD_CK(up(pos, tile_.st_pos));
+        PD_CK(up(rest, conv(tile_.st_rest)));
+        PD_CK(up(lbo, conv(tile_.st_lbo)));
+        PD_CK(up(bend, conv(tile_.st_bend)));
+        PD_CK(up(halo, tile_.halo));
+        PD_CK(up(nbr, tile_.nbr));
+        PD_CK(up(tet, tile_.tet));
+        PD_CK(zeros(a.ex, 2 * (size_t)kTileWords<T, TC> * H.nsim));
+        PD_CK(zeros(a.flags, tile_.tiles.size()));
+        PD_CK(cudaStreamSynchronize(s_));
+        // the device has the tables: the host keeps the tiles and launches only
+        for (auto* v : {&tile_.val, &tile_.st_rest, &tile_.st_lbo, &tile_.st_bend}) std::vector<double>().swap(*v);
+        std::vector<TileSlot>().swap(tile_.slots);
+        std::vector<int16_t>().swap(tile_.pat);
+        std::vector<int16_t>().swap(tile_.st_pos);
+        a.nsim = H.nsim;
+        a.lg = c_.lg;
+        a.cheby = c_.cheby;
+        a.relax = (T)c_.relax;
+        T rho2 = (T)c_.rho;
+        rho2 = rho2 * rho2;
+        T om = omega_first(rho2);
+        for (int it = 0; it < kMaxCheby; ++it) a.omega[it] = T(0);
+        for (int it = 1; it < c_.cheby; ++it) {
+            a.omega[it] = om;
+            om = omega_next(rho2, om);
+        }
+        a.timeout = wait_cycles_;
+        a.P = d.P;
+        a.Ph = d.Ph;
+        a.Pl = d.Pl;
+        a.Pold = d.Pold;
+        a.Xrest = d.Xrest;
+        a.Rhs0 = d.Rhs0;
+        a.CollRhs = d.CollRhs;
+        a.PinRhs = d.PinRhs;
+        a.Delastic = d.Delastic;
+        a.Dinert = d.Dinert;
+        a.CollDiag = d.CollDiag;
+        a.PinFlag = d.PinFlag;
+        a.PinK = d.PinK;
+        a.Strain = d.Strain;
+        a.CurvNorm = d.CurvNorm;
+        a.tBend0 = d.tBend0;
+        a.tLbo0 = d.tLbo0;
+        if constexpr (!fp64) {
+            a.Tets = d.Tets;
+            a.TetIdm = d.TetIdm;
+            a.TetW = d.TetW;
+            a.TetOut = d.TetOut;
+        }
+        a.vtPtr = d.vtPtr;
+        a.vtIdx = d.vtIdx;
+        a.tet = tet;
+        a.tiles = tiles;
+        a.slots = slots;
+        a.slices = slices;
+        a.val = val;
+        a.pat = pat;
+        a.halo = halo;
+        a.patStride = tile_.pat_stride;
+        a.stencil = stencil;
+        a.stPos = pos;
+        a.stRest = rest;
+        a.stLbo = lbo;
+        a.stBend = bend;
+        a.nbr = nbr;
+        a.err = d.ErrFlags;
+        a.instStop = prm_.instance_stop ? d.InstStop : nullptr;
+        a.tape = nullptr;
+        a.third = tile_.vectors > 2;
+        tile_on_ = true;
+        return PDIPC_OK;
+    }
+
+    // One PD solve over the tiles: a launch per group of whole models.
+    cudaError_t launch_tiles(int* launched) {
+        targs_.gate = d_.Gate;
+        targs_.tape = nullptr;
+        if constexpr (kAdjoint) {
+            if (taping_) {  // positions at the start of every local-global iteration
+                if (adj_tape_n_ + c_.lg <= adj_tape_cap_) targs_.tape = adj_tape_ + (size_t)adj_tape_n_ * d_.nsim;
+                adj_tape_n_ += c_.lg;
+            }
+        }
+        for (const TileGroup& g : tile_.groups) {
+            targs_.lo = g.lo;
+            // fresh tags and phase counts: every earlier launch's lie below them
+            targs_.epoch0 = targs_.flag0 = epoch_;
+            epoch_ += tile_phases(c_.lg, c_.cheby);
+            const cudaError_t e = launch_pd_tile<T, TC>(targs_, g.hi - g.lo + 1, tile_.rows_per_thread, d_.ntet > 0,
+                                                        tile_.threads, tile_.smem_bytes, s_);
+            if (e != cudaSuccess) return e;
+            if (launched) ++*launched;
+        }
+        return cudaSuccess;
+    }
+
     // one PD solve: a launch per group, in order on the stream; returns the launches made
     cudaError_t launch_persistent(int* launched = nullptr) {
+        if (tile_on_) return launch_tiles(launched);
         if constexpr (std::is_same<T, float>::value) {
             pargs_.gate = d_.Gate;
             for (const PersistGroup& g : groups_) {
@@ -2067,7 +2242,7 @@ private:
     }
 
     pdipc_status pd_solve(std::string& err) {
-        if (plan_.enabled) {
+        if (persistent_on()) {
             int n = 0;
             PD_CK(launch_persistent(&n));
             launches_ += n;
@@ -2228,7 +2403,8 @@ private:
         launch_predict(d, dt, s_);
         ++launches_;
         const int max_outer = prm_.fixed_outer > 0 ? prm_.fixed_outer : prm_.max_outer;
-        const int ahead = plan_.enabled ? 1 : 0;
+        // (taping counts the solves that ran, so it waits too)
+        const int ahead = persistent_on() && !taping_ ? 1 : 0;
         int enq = 0, outer = 0;
         for (; enq <= ahead && enq < max_outer; ++enq) {
             pdipc_status r = enqueue_outer(enq, err);
@@ -2287,7 +2463,7 @@ private:
             pin_->err = 0;
             cudaMemsetAsync(d.ErrFlags, 0, sizeof(unsigned int), s_);
             if (e & kErrBarrier) {
-                cudaMemsetAsync(pBar_ + 1, 0, sizeof(unsigned), s_);
+                if (pBar_) cudaMemsetAsync(pBar_ + 1, 0, sizeof(unsigned), s_);
                 err = "grid barrier of the persistent solve timed out";
                 return PDIPC_ERR_CUDA;
             }
@@ -2359,6 +2535,9 @@ private:
     pdipc_tuning tuning_{};
     PersistArgs<float, TC> pargs_{};
     std::vector<PersistGroup> groups_;  // launches of one persistent PD solve
+    TilePlan tile_;                     // compact tiles (ok: their tables are on the device)
+    bool tile_on_ = false;              // the PD solve runs over them
+    TileArgs<T, TC> targs_{};
     // the matrix in SELL-32 over slots (slot_of) for the persistent solve
     int* pSOff_ = nullptr;
     int* pSLen_ = nullptr;

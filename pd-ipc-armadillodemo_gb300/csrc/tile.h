@@ -1,0 +1,106 @@
+// tile.h — arguments and launch of the tiled persistent PD solve (pd_tile.cu).
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "common.cuh"
+#include "persistent.h"
+#include "tile_plan.h"
+
+namespace pdipc {
+
+constexpr int kTileMaxWarps = 14;  // row warps per CTA; two CTAs share an SM (72 registers per thread)
+
+// A published value: 16 bytes read and written as one, the phase's tag in the
+// last word.  A vertex is one word in FP32 (x, y, z, tag) and three in FP64
+// ((value, tag) per component).
+struct alignas(16) TileWord {
+    unsigned long long lo, hi;
+};
+
+// T: solver scalar; S: state scalar (T in the direct form, double in the
+// correction form).
+template <typename T, typename S>
+struct TileArgs {
+    int nsim;
+    int lg;
+    int cheby;
+    T relax;
+    T omega[kMaxCheby];
+    long long timeout;  // limit of a wait in clock cycles
+    // state, as in PersistArgs
+    V4<S>* P;
+    V4<T>* Ph;
+    V4<T>* Pl;
+    const V4<S>* Pold;
+    const V4<S>* Xrest;
+    const V4<S>* Rhs0;
+    const V4<T>* CollRhs;
+    const V4<T>* PinRhs;
+    const T* Delastic;
+    const T* Dinert;
+    const T* CollDiag;
+    const int* PinFlag;
+    const T* PinK;
+    const T* Strain;
+    const T* CurvNorm;
+    const T* tBend0;
+    const T* tLbo0;
+    // tets (as in PersistArgs; tile t projects tet[tet0 .. tet0 + ntet))
+    const int4* Tets;
+    const T* TetIdm;
+    const T* TetW;
+    V4<T>* TetOut;
+    const int* vtPtr;
+    const int* vtIdx;
+    const int* tet;
+    // tiles
+    const TileInfo* tiles;
+    const TileSlot* slots;
+    const TileSlice* slices;
+    const T* val;
+    const int16_t* pat;
+    const TileHalo* halo;
+    int patStride;
+    // stencils by slot: neighbour k of a row of slice s at stencil[s] + 32 k +
+    // lane (place relative to the row's own, weights)
+    const int* stencil;
+    const int16_t* stPos;
+    const T* stRest;  // spring rest length
+    const T* stLbo;
+    const T* stBend;  // transposed bending weight
+    // exchange: ex[(parity * kWords + w) * nsim + row], tags from epoch0 + 1
+    TileWord* ex;
+    unsigned epoch0;
+    // tets only: phase counts of the tiles and the tiles each waits for
+    unsigned* flags;
+    const int* nbr;
+    unsigned flag0;
+    unsigned* err;
+    const OuterGate* gate;
+    const unsigned* instStop;  // per-instance stopping: tiles of a stopped model return at entry
+    V4<T>* tape;               // direct form: the positions at the start of every local-global iteration, or null
+    int lo;                    // first tile of this launch
+    int third;                 // correction form: the tiles hold a third vector
+};
+
+// Words of one vertex in a phase: the correction form publishes the two halves
+// of its positions in the same phase.
+template <typename T, typename S>
+constexpr int kTileWords = sizeof(T) == 8 ? 3 : sizeof(S) == 8 ? 2 : 1;
+// Entries of a row whose values lie together (16 bytes).
+template <typename T>
+constexpr int kTileGroup = 16 / (int)sizeof(T);
+// Tags and flags one launch uses at most.
+inline unsigned tile_phases(int lg, int cheby) { return (unsigned)(lg * (2 * cheby + 1) + 2); }
+
+// Residents: CTAs of the variant one cooperative launch can hold (0: no such variant).
+template <typename T, typename S>
+int tile_residents(int rows_per_thread, bool tets, int threads, size_t smem, int sms);
+template <typename T, typename S>
+cudaError_t launch_pd_tile(const TileArgs<T, S>& args, int tiles, int rows_per_thread, bool tets, int threads,
+                           size_t smem, cudaStream_t s);
+
+}  // namespace pdipc

@@ -19,9 +19,9 @@ INC = os.path.join(ROOT, "include")
 OUT = os.path.join(PKG, "libpdipc.so")
 OBJ = os.path.join(PKG, "_build")
 
-SOURCES = ["pd_kernels.cu", "pd_persistent.cu", "pd_persistent_band.cu", "collision_kernels.cu", "penalty_kernels.cu", "primitives.cu",
+SOURCES = ["pd_kernels.cu", "pd_persistent.cu", "pd_persistent_band.cu", "pd_tile.cu", "collision_kernels.cu", "penalty_kernels.cu", "primitives.cu",
            "adjoint_kernels.cu", "solver.cu",
-           "host_tables.cpp", "capi.cpp", "scene_io.cpp"]
+           "host_tables.cpp", "tile_plan.cpp", "capi.cpp", "scene_io.cpp"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 # host code must not fuse multiply-adds: the patch grid is computed in FP32 exactly as
 # the reference does, and an Arm host compiler contracts a*b+c by default

@@ -1,0 +1,70 @@
+"""The tiled persistent solve against one launch per sweep, where its partition
+changes shape: one tile and the first size of several, one and two rows per
+thread, several models, launches of groups, and a differentiated FP64 rollout
+(whose replay tapes the positions inside the tiled solve).
+
+In the direct form (FP32, FP64) a row sums its columns in ascending order in
+every path, so the two solves are the same numbers; in the mixed form the order
+differs and the correction form absorbs it (1e-6 m on one solve, as for the
+other persistent paths)."""
+import numpy as np
+import pytest
+
+import pdipc
+from pdipc import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def _solve(sc, prec, **kw):
+    sim = pdipc.Simulator(sc, prec, **kw)
+    X = sc.initial_positions()
+    V = np.random.default_rng(5).uniform(-0.1, 0.1, (sc.n_sim, 3))
+    x = sim.stage_pd(X, V)
+    return x, sim.tuning()
+
+
+# 21^2 = 441 rows: one tile; 22^2: several; 65: odd edges; 224 and 330: two
+# tiles per SM, with one and (FP32) two rows per thread
+@pytest.mark.parametrize("prec,n", [(p, n) for p in ("fp32", "fp64") for n in (2, 21, 22, 65, 224)] +
+                         [("fp32", 430), ("mixed", 21), ("mixed", 22), ("mixed", 430)])
+def test_tiled_solve_against_one_launch_per_sweep(prec, n, built_lib):
+    sc = scenes.cloth_drop(n, 1, with_sphere=False, lg=3)
+    a, t = _solve(sc, prec)
+    b, u = _solve(sc, prec, persistent=0)
+    assert t["pd_rows_per_thread"] == (2 if n == 430 else 1) and u["pd_rows_per_thread"] == 0
+    assert t["pd_ctas"] == 1 if n == 2 else t["pd_ctas"] > 1 if n > 21 else t["pd_ctas"] <= 2
+    if prec == "mixed":
+        assert np.abs(a - b).max() < 1e-6
+    else:
+        assert np.array_equal(a, b)
+
+
+def test_tiled_groups_and_stopped_models_give_the_bits_of_one_launch(built_lib):
+    sc = scenes.batched(5, 20, 40, seed=11)
+    for prec, stop in (("fp32", 1), ("mixed", 1), ("fp64", 0)):
+        one = pdipc.Simulator(sc, prec, instance_stop=stop)
+        many = pdipc.Simulator(sc, prec, instance_stop=stop, pd_group_ctas=one.tuning()["pd_ctas"] // 2)
+        assert one.tuning()["pd_launches"] == 1 and many.tuning()["pd_launches"] > 1
+        for _ in range(3):
+            one.step(1)
+            many.step(1)
+            assert np.array_equal(one.positions(), many.positions()), prec
+
+
+def test_differentiated_rollout_is_the_same_over_tiles_and_sweeps(built_lib):
+    sc = scenes.cloth_drop(24, 1, with_sphere=False)
+    rng = np.random.default_rng(3)
+    x0 = sc.initial_positions()
+    v0 = rng.uniform(-0.1, 0.1, x0.shape)
+    g = rng.normal(size=x0.shape)
+    out = []
+    for persistent in (1, 0):
+        sim = pdipc.Simulator(sc, "fp64", fixed_outer=2, persistent=persistent)
+        assert (sim.stats()["pd_path"] > 0) == (persistent == 1)
+        sim.set_state(x0, v0)
+        sim.adjoint_record(2)
+        sim.step(3)
+        out.append((sim.positions(),) + sim.adjoint_backward(g))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
