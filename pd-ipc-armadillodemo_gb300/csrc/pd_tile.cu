@@ -199,37 +199,50 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
     for (int q = threadIdx.x; q < ti.npat * a.patStride; q += blockDim.x)
         spat[q] = __ldg(a.pat + (size_t)ti.pat0 * a.patStride + q);
 
-    // ---- this thread's rows: slice r nw + warp, this lane ----
-    // gr: row (-1 none); lp: its place; pe: its pattern's first element; eo/el:
-    // first entry and entries per row of its slice
-    int gr[R], lp[R], pe[R], eo[R], el[R];
-    int pub[R];
+    // ---- this thread's rows: slice r nw + warp, this lane.  Packed, two rows per
+    // thread leave few registers: gp = row (negative: none), bit 30: published;
+    // lpe = place | pattern's first element << 16; eol = first entry | entries
+    // per row << 20 ----
+    int gp[R];
+    unsigned lpe[R], eol[R];
     T id[R];
+    auto slot = [&](int r) { return ti.slot0 + 32 * (r * nw + warp) + lane; };
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int s = r * nw + warp;
-        gr[r] = -1;
-        lp[r] = pe[r] = eo[r] = el[r] = 0;
-        pub[r] = 0;
+        gp[r] = -1;
+        lpe[r] = eol[r] = 0u;
         id[r] = T(0);
         if (s < ti.nslice) {
-            const TileSlot sl = a.slots[ti.slot0 + 32 * s + lane];
+            const TileSlot sl = a.slots[slot(r)];
             const TileSlice sc = a.slices[ti.slice0 + s];
-            gr[r] = sl.row;
-            lp[r] = sl.pos;
-            pe[r] = sl.pat;
-            pub[r] = sl.pub;
-            eo[r] = sc.off + kG * lane;
-            el[r] = sl.row >= 0 ? sc.len : 0;
+            if (sl.row >= 0) {
+                gp[r] = sl.row | ((sl.pub & 1) << 30);
+                lpe[r] = (unsigned)sl.pos | ((unsigned)sl.pat << 16);
+                eol[r] = (unsigned)(sc.off + kG * lane) | ((unsigned)sc.len << 20);
+                id[r] = T(1) / ((a.Delastic[sl.row] + a.Dinert[sl.row]) + a.CollDiag[sl.row]);
+            }
         }
-        if (gr[r] >= 0) id[r] = T(1) / ((a.Delastic[gr[r]] + a.Dinert[gr[r]]) + a.CollDiag[gr[r]]);
     }
+    auto live = [&](int r) { return gp[r] >= 0; };
+    auto row = [&](int r) { return gp[r] & 0x3fffffff; };
+    auto pub = [&](int r) { return gp[r] >= 0x40000000; };
+    auto lp = [&](int r) { return (int)(lpe[r] & 0xffffu); };
+    auto pe = [&](int r) { return (int)(lpe[r] >> 16); };
+    auto eo = [&](int r) { return (int)(eol[r] & 0xfffffu); };
+    auto el = [&](int r) { return (int)(eol[r] >> 20); };
     // the first halo row this thread polls (others through the table)
     const TileHalo h0 = (int)threadIdx.x < ti.nhalo ? a.halo[ti.halo0 + threadIdx.x] : TileHalo{-1, 0};
 
     auto put = [&](int b, int q, T x, T y, T z) {
         XY(b)[q] = Pair<T>{x, y};
         Z(b)[q] = z;
+    };
+    auto own = [&](int b, int r, T& x, T& y, T& z) {
+        const Pair<T> p = XY(b)[lp(r)];
+        x = p.x;
+        y = p.y;
+        z = Z(b)[lp(r)];
     };
     unsigned tag = a.epoch0;  // of the last phase published
     auto words = [&](int w) { return a.ex + ((size_t)(tag & 1u) * kW + w) * a.nsim; };
@@ -326,10 +339,10 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
         s0 = T(0);
         s1 = T(0);
         s2 = T(0);
-        const Group<T>* vp = reinterpret_cast<const Group<T>*>(sval + eo[r]);
-        const uint2* pp = reinterpret_cast<const uint2*>(spat + pe[r]);
-        const Pair<T>* xy = XY(b) + lp[r];
-        const T* z = Z(b) + lp[r];
+        const Group<T>* vp = reinterpret_cast<const Group<T>*>(sval + eo(r));
+        const uint2* pp = reinterpret_cast<const uint2*>(spat + pe(r));
+        const Pair<T>* xy = XY(b) + lp(r);
+        const T* z = Z(b) + lp(r);
         auto batch = [&](auto nc, const unsigned* o, const T* v) {
             constexpr int n = decltype(nc)::value;
             Pair<T> p[n];
@@ -349,7 +362,7 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
         };
         int k = 0;
         if constexpr (kG == 4 && R == 1) {
-            for (; k + 8 <= el[r]; k += 8) {
+            for (; k + 8 <= el(r); k += 8) {
                 const uint4 o4 = *reinterpret_cast<const uint4*>(pp + (k >> 2));
                 const unsigned o[4] = {o4.x, o4.y, o4.z, o4.w};
                 const Group<T> va = vp[(k >> 2) * 32], vb = vp[(k >> 2) * 32 + 32];
@@ -363,7 +376,7 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
             }
         }
 #pragma unroll(kUnroll)
-        for (; k < el[r]; k += 4) {
+        for (; k < el(r); k += 4) {
             const uint2 o2 = pp[k >> 2];
             const unsigned o[2] = {o2.x, o2.y};
             T v[4];
@@ -391,7 +404,7 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
     };
 #pragma unroll
     for (int r = 0; r < R; ++r)
-        if (gr[r] >= 0) load_pos(gr[r], lp[r]);
+        if (live(r)) load_pos(row(r), lp(r));
     for (int h = threadIdx.x; h < ti.nhalo; h += blockDim.x) {
         const TileHalo q = a.halo[ti.halo0 + h];
         load_pos(q.row, q.pos);
@@ -408,10 +421,10 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
         // correction form: the residual's matrix part of owned row r, in column
         // order (the entries below the row's own block, those in it, those above)
         auto matrix_part = [&](int r, Acc& r0, Acc& r1, Acc& r2) {
-            const T* vp = sval + eo[r];
-            const int16_t* pp = spat + pe[r];
-            const Pair<T>*hp = XY(0) + lp[r], *lpp = XY(1) + lp[r];
-            const T *hz = Z(0) + lp[r], *lz = Z(1) + lp[r];
+            const T* vp = sval + eo(r);
+            const int16_t* pp = spat + pe(r);
+            const Pair<T>*hp = XY(0) + lp(r), *lpp = XY(1) + lp(r);
+            const T *hz = Z(0) + lp(r), *lz = Z(1) + lp(r);
             const T h0x = hp[0].x, h0y = hp[0].y, h0z = hz[0], l0x = lpp[0].x, l0y = lpp[0].y, l0z = lz[0];
             auto part = [&](int k0, int k1) {
 #pragma unroll 4
@@ -424,25 +437,24 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
                     r2.add(v, diff_ff(hz[j], lz[j], h0z, l0z));
                 }
             };
-            const int ka = (pub[r] >> 8) & 255, kb = (pub[r] >> 16) & 255;
+            const int parts = __ldg(&a.slots[slot(r)].pub), ka = (parts >> 8) & 255, kb = (parts >> 16) & 255;
             part(ka, kb);
             part(0, ka);
-            part(kb, el[r]);
+            part(kb, el(r));
         };
         // ---- local step: curvature vectors, springs and (correction form without
         // a third vector) the matrix part of the residual, all from shared memory ----
-        T aq[R][3], rh[R][3], cx[R][3], px[R][3];
+        T aq[R][3], rh[R][3], px[R][3];
         Acc acc[kCorr ? R : 1][3];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             aq[r][0] = aq[r][1] = aq[r][2] = T(0);
             rh[r][0] = rh[r][1] = rh[r][2] = T(0);
-            cx[r][0] = cx[r][1] = cx[r][2] = T(0);
             px[r][0] = px[r][1] = px[r][2] = T(0);
-            if (gr[r] < 0) continue;
-            const int i = gr[r];
+            if (!live(r)) continue;
+            const int i = row(r);
             const int s = r * nw + warp;
-            const int st = __ldg(a.stencil + ti.slice0 + s) + lane, nst = pub[r] >> 24;
+            const int st = __ldg(a.stencil + ti.slice0 + s) + lane, nst = __ldg(&a.slots[slot(r)].pub) >> 24;
             const T strain = a.Strain[i];
             T a0, a1, a2;
             if constexpr (kCorr) {
@@ -476,8 +488,8 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
                     r2.add(dc, (T)(xo.z - x.z));
                     }
                 }
-                const Pair<T>*hp = XY(0) + lp[r], *lpp = XY(1) + lp[r];
-                const T *hz = Z(0) + lp[r], *lz = Z(1) + lp[r];
+                const Pair<T>*hp = XY(0) + lp(r), *lpp = XY(1) + lp(r);
+                const T *hz = Z(0) + lp(r), *lz = Z(1) + lp(r);
                 const T h0x = hp[0].x, h0y = hp[0].y, h0z = hz[0], l0x = lpp[0].x, l0y = lpp[0].y, l0z = lz[0];
                 a0 = a1 = a2 = T(0);
 #pragma unroll 4
@@ -502,8 +514,8 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
                 acc[r][1] = r1;
                 acc[r][2] = r2;
             } else {
-                const Pair<T>* xp = XY(cur) + lp[r];
-                const T* xz = Z(cur) + lp[r];
+                const Pair<T>* xp = XY(cur) + lp(r);
+                const T* xz = Z(cur) + lp(r);
                 const T x0 = xp[0].x, x1 = xp[0].y, x2 = xz[0];
                 const T l0 = a.tLbo0[i];
                 a0 = x0 * l0;
@@ -529,9 +541,6 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
                 rh[r][0] = t0;
                 rh[r][1] = t1;
                 rh[r][2] = t2;
-                cx[r][0] = x0;
-                cx[r][1] = x1;
-                cx[r][2] = x2;
                 if (a.tape) a.tape[(size_t)lg * a.nsim + i] = V4<T>{x0, x1, x2, T(0)};
             }
             const T nrm = dsqrt(norm2(a0, a1, a2));
@@ -553,19 +562,19 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
         ++tag;
 #pragma unroll
         for (int r = 0; r < R; ++r)
-            if (gr[r] >= 0) {
-                if (pub[r] & 1) publish(0, gr[r], aq[r][0], aq[r][1], aq[r][2]);
-                put(qb, lp[r], aq[r][0], aq[r][1], aq[r][2]);
+            if (live(r)) {
+                if (pub(r)) publish(0, row(r), aq[r][0], aq[r][1], aq[r][2]);
+                put(qb, lp(r), aq[r][0], aq[r][1], aq[r][2]);
             }
         if (!arrive(qb)) return;
         // ---- bending, then the right-hand side (direct) or residual (correction) ----
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            if (gr[r] < 0) continue;
-            const int i = gr[r];
-            const int st = __ldg(a.stencil + ti.slice0 + r * nw + warp) + lane, nst = pub[r] >> 24;
-            const Pair<T>* qp = XY(qb) + lp[r];
-            const T* qz = Z(qb) + lp[r];
+            if (!live(r)) continue;
+            const int i = row(r);
+            const int st = __ldg(a.stencil + ti.slice0 + r * nw + warp) + lane, nst = __ldg(&a.slots[slot(r)].pub) >> 24;
+            const Pair<T>* qp = XY(qb) + lp(r);
+            const T* qz = Z(qb) + lp(r);
             const T b0 = a.tBend0[i];
             if constexpr (kCorr) {
                 Acc r0 = acc[r][0], r1 = acc[r][1], r2 = acc[r][2];
@@ -635,18 +644,22 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 T s0 = T(0), s1 = T(0), s2 = T(0);
-                if (!kCorr) row_sum(r, cur, s0, s1, s2);
-                y[r][0] = jacobi<kCorr>(om1, cx[r][0], w, s0, rh[r][0], id[r]);
-                y[r][1] = jacobi<kCorr>(om1, cx[r][1], w, s1, rh[r][1], id[r]);
-                y[r][2] = jacobi<kCorr>(om1, cx[r][2], w, s2, rh[r][2], id[r]);
-                if (pub[r] & 1) publish(0, gr[r], y[r][0], y[r][1], y[r][2]);
+                T c0 = T(0), c1 = T(0), c2 = T(0);
+                if (!kCorr) {
+                    row_sum(r, cur, s0, s1, s2);
+                    own(cur, r, c0, c1, c2);
+                }
+                y[r][0] = jacobi<kCorr>(om1, c0, w, s0, rh[r][0], id[r]);
+                y[r][1] = jacobi<kCorr>(om1, c1, w, s1, rh[r][1], id[r]);
+                y[r][2] = jacobi<kCorr>(om1, c2, w, s2, rh[r][2], id[r]);
+                if (pub(r)) publish(0, row(r), y[r][0], y[r][1], y[r][2]);
             }
             // the curvature vectors (direct form), or the positions, have been read
             if (!kCorr || a.third) __syncthreads();
             cur = kCorr ? 1 : cur ^ 1;
 #pragma unroll
             for (int r = 0; r < R; ++r)
-                if (gr[r] >= 0) put(cur, lp[r], y[r][0], y[r][1], y[r][2]);
+                if (live(r)) put(cur, lp(r), y[r][0], y[r][1], y[r][2]);
         }
         if (!arrive(cur)) return;
         for (int it = 0; it < a.cheby; ++it) {
@@ -658,27 +671,31 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
             for (int r = 0; r < R; ++r) {
                 T s0, s1, s2, n[3];
                 row_sum(r, cur, s0, s1, s2);
-                const Pair<T> yxy = XY(cur)[lp[r]];
-                const T yz = Z(cur)[lp[r]];
-                n[0] = jacobi<kCorr>(om1, yxy.x, w, s0, rh[r][0], id[r]);
-                n[1] = jacobi<kCorr>(om1, yxy.y, w, s1, rh[r][1], id[r]);
-                n[2] = jacobi<kCorr>(om1, yz, w, s2, rh[r][2], id[r]);
+                T c0, c1, c2;
+                own(cur, r, c0, c1, c2);
+                n[0] = jacobi<kCorr>(om1, c0, w, s0, rh[r][0], id[r]);
+                n[1] = jacobi<kCorr>(om1, c1, w, s1, rh[r][1], id[r]);
+                n[2] = jacobi<kCorr>(om1, c2, w, s2, rh[r][2], id[r]);
                 if (it > 0) {
                     n[0] = fma_(om, add_(n[0], -px[r][0]), px[r][0]);
                     n[1] = fma_(om, add_(n[1], -px[r][1]), px[r][1]);
                     n[2] = fma_(om, add_(n[2], -px[r][2]), px[r][2]);
                 }
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    px[r][c] = cx[r][c];
-                    cx[r][c] = n[c];
+                // the next step's step before last: the other vector still holds this
+                // row's current x (the correction starts from zero)
+                if (kCorr && last) {
+                    px[r][0] = n[0];
+                    px[r][1] = n[1];
+                    px[r][2] = n[2];
+                } else if (!kCorr || it > 0) {
+                    own(cur ^ 1, r, px[r][0], px[r][1], px[r][2]);
                 }
-                if (gr[r] < 0) continue;
+                if (!live(r)) continue;
                 if (!(kCorr && last)) {
-                    if (pub[r] & 1) publish(0, gr[r], n[0], n[1], n[2]);
-                    put(cur ^ 1, lp[r], n[0], n[1], n[2]);
+                    if (pub(r)) publish(0, row(r), n[0], n[1], n[2]);
+                    put(cur ^ 1, lp(r), n[0], n[1], n[2]);
                 }
-                if (!kCorr && last && (kTets || lg == a.lg - 1)) a.P[gr[r]] = V4<S>{n[0], n[1], n[2], S(0)};
+                if (!kCorr && last && (kTets || lg == a.lg - 1)) a.P[row(r)] = V4<S>{n[0], n[1], n[2], S(0)};
             }
             if (last) break;
             cur ^= 1;
@@ -689,12 +706,14 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
             for (int r = 0; r < R; ++r) {
                 T s0, s1, s2;
                 row_sum(r, cur, s0, s1, s2);
-                const T y0 = jacobi<kCorr>(om1, cx[r][0], w, s0, rh[r][0], id[r]);
-                const T y1 = jacobi<kCorr>(om1, cx[r][1], w, s1, rh[r][1], id[r]);
-                const T y2 = jacobi<kCorr>(om1, cx[r][2], w, s2, rh[r][2], id[r]);
-                if (gr[r] < 0) continue;
-                if (pub[r] & 1) publish(0, gr[r], y0, y1, y2);
-                put(cur ^ 1, lp[r], y0, y1, y2);
+                T c0, c1, c2;
+                own(cur, r, c0, c1, c2);
+                const T y0 = jacobi<kCorr>(om1, c0, w, s0, rh[r][0], id[r]);
+                const T y1 = jacobi<kCorr>(om1, c1, w, s1, rh[r][1], id[r]);
+                const T y2 = jacobi<kCorr>(om1, c2, w, s2, rh[r][2], id[r]);
+                if (!live(r)) continue;
+                if (pub(r)) publish(0, row(r), y0, y1, y2);
+                put(cur ^ 1, lp(r), y0, y1, y2);
             }
             cur ^= 1;
             if (!arrive(cur)) return;
@@ -704,24 +723,24 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
             __syncthreads();  // both vectors have been read
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                if (gr[r] < 0) continue;
-                const V4<S> x = ldg_state(a.P, gr[r]);
-                const S q0 = x.x + (S)cx[r][0], q1 = x.y + (S)cx[r][1], q2 = x.z + (S)cx[r][2];
-                a.P[gr[r]] = V4<S>{q0, q1, q2, S(0)};
+                if (!live(r)) continue;
+                const V4<S> x = ldg_state(a.P, row(r));
+                const S q0 = x.x + (S)px[r][0], q1 = x.y + (S)px[r][1], q2 = x.z + (S)px[r][2];
+                a.P[row(r)] = V4<S>{q0, q1, q2, S(0)};
                 float hx, lx, hy, ly, hz, lz;
                 split_ff(q0, hx, lx);
                 split_ff(q1, hy, ly);
                 split_ff(q2, hz, lz);
                 if (kTets || lg == a.lg - 1) {
-                    a.Ph[gr[r]] = V4<T>{hx, hy, hz, T(0)};
-                    a.Pl[gr[r]] = V4<T>{lx, ly, lz, T(0)};
+                    a.Ph[row(r)] = V4<T>{hx, hy, hz, T(0)};
+                    a.Pl[row(r)] = V4<T>{lx, ly, lz, T(0)};
                 }
-                if (pub[r] & 1) {
-                    publish(0, gr[r], hx, hy, hz);
-                    publish(1, gr[r], lx, ly, lz);
+                if (pub(r)) {
+                    publish(0, row(r), hx, hy, hz);
+                    publish(1, row(r), lx, ly, lz);
                 }
-                put(0, lp[r], hx, hy, hz);
-                put(1, lp[r], lx, ly, lz);
+                put(0, lp(r), hx, hy, hz);
+                put(1, lp(r), lx, ly, lz);
             }
             if (lg == a.lg - 1) break;
             if (!arrive(0, 1)) return;

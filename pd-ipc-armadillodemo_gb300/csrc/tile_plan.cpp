@@ -156,7 +156,7 @@ size_t tile_smem_bytes(const TileInfo& t, int pat_stride, int value_bytes, int v
 void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block, TilePlan& P) {
     P = TilePlan();
     const int ns = H.nsim;
-    if (ns == 0) return;
+    if (ns == 0 || ns >= 1 << 30) return;
     std::vector<Model> models;
     for (int i = 0; i < ns;) {
         int e = i + 1;
@@ -417,6 +417,7 @@ void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block
         }
         T.npat = npat;
         T.nent = (int)P.val.size() - T.ent0;
+        if (T.nent >= 1 << 20 || npat * P.pat_stride > 65535) return;  // packed in the kernel
         T.halo0 = (int)P.halo.size();
         T.nhalo = (int)halo[t].size();
         std::sort(halo[t].begin(), halo[t].end());
