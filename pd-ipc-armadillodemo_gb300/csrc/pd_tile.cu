@@ -772,8 +772,11 @@ template <typename T, typename S>
 int tile_residents(int R, bool tets, int threads, size_t smem, int sms) {
     const void* f = tile_kernel<T, S, !std::is_same<T, S>::value>(R, tets);
     if (!f || threads > kTileMaxWarps * 32) return 0;
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max<size_t>(smem, 1)) !=
-        cudaSuccess)
+    // the kernel's limit is raised only: other contexts may hold larger tiles
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) return 0;
+    if ((size_t)fa.maxDynamicSharedSizeBytes < smem &&
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return 0;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem) != cudaSuccess) return 0;

@@ -1581,6 +1581,7 @@ private:
         };
         const int group_cap = prm_.pd_group_ctas > 0 ? prm_.pd_group_ctas : INT_MAX;
         std::vector<Cand> cands;
+        int order_block = -1;  // the default configuration's rows per CTA on the band path (whatever the launches)
         const bool dflt_l1 = prm_.persistent != 2, dflt_ls = prm_.persistent != 3;
         for (int pass = 0; pass < 2; ++pass) {
             const bool smem_mat = pass == 0 && fits16;
@@ -1622,11 +1623,17 @@ private:
                     const void* f =
                         persistent_kernel(kCorrection, smem_mat, c.ch.band, c.band_param, c.ch.l1_gather, R, H.ntet > 0);
                     if (!f) continue;
-                    PD_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)std::max<size_t>(c.sm, 1)));
+                    cudaFuncAttributes fa;  // the kernel's limit is raised only: other contexts may need more
+                    PD_CK(cudaFuncGetAttributes(&fa, f));
+                    if ((size_t)fa.maxDynamicSharedSizeBytes < c.sm)
+                        PD_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.sm));
                     int per_sm = 0;
                     PD_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, c.threads, c.sm));
-                    if (per_sm < 1 || !form_groups(c.spc, c.ctas, std::min(per_sm * nsm, group_cap), c.groups)) continue;
+                    if (per_sm < 1) continue;
+                    if (order_block < 0 && c.ch.l1_gather == dflt_l1 && c.ch.local_sync == dflt_ls &&
+                        form_groups(c.spc, c.ctas, per_sm * nsm, c.groups))
+                        order_block = c.ch.band ? c.spc * kSlice : 0;
+                    if (!form_groups(c.spc, c.ctas, std::min(per_sm * nsm, group_cap), c.groups)) continue;
                     cands.push_back(std::move(c));
                 }
             }
@@ -1648,7 +1655,7 @@ private:
         if (!force && prm_.persistent == 1) {
             // compact tiles where a partition fits; a row sums in the order of
             // the configuration they stand in for, so the results keep its bits
-            pdipc_status r = plan_tiles(H, pick && pick->ch.band ? pick->spc * kSlice : 0, err);
+            pdipc_status r = plan_tiles(H, std::max(order_block, 0), err);
             if (r != PDIPC_OK || tile_on_) return r;
         }
         if (!pick) return PDIPC_OK;
