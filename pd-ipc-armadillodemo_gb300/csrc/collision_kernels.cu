@@ -19,6 +19,7 @@
 // heap tree over the same boxes.
 #include <cfloat>
 #include <mutex>
+#include <type_traits>
 
 #include "geometry.cuh"
 #include "kernels.cuh"
@@ -568,41 +569,53 @@ __device__ __forceinline__ void toi_rel(const int* ids, const V4<T>* __restrict_
     }
 }
 
+// Stage 1 of a candidate on FP32 coordinates that are the exact ones rounded:
+// false only when the exact test's time of impact is 1 for certain (the
+// swept-box filter with the distance widened past the largest effect of the
+// rounding, |low| <= 2^-24 |x| and the roundings here: < 2^-18 of the largest
+// coordinate; then the CCD's box-gap exit).  A NaN or infinite coordinate goes on
+// to the exact test.
+template <typename T, bool kPT>
+__device__ __forceinline__ bool toi_maybe(const int* ids, const V4<T>* __restrict__ X0h, const V4<T>* __restrict__ X1h,
+                                          T slack) {
+    T xh[4][3], dh[4][3], m = T(0);
+    const V4<T> o = ld4(X0h, ids[0]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const V4<T> ah = ld4(X0h, ids[j]), bh = ld4(X1h, ids[j]);
+        xh[j][0] = ah.x - o.x;
+        xh[j][1] = ah.y - o.y;
+        xh[j][2] = ah.z - o.z;
+        dh[j][0] = bh.x - ah.x;
+        dh[j][1] = bh.y - ah.y;
+        dh[j][2] = bh.z - ah.z;
+        m = dmax(m, dmax(dmax(fabsf(ah.x), fabsf(ah.y)), dmax(fabsf(ah.z), fabsf(bh.x))));
+        m = dmax(m, dmax(fabsf(bh.y), fabsf(bh.z)));
+    }
+    const T wide = slack + m * T(1.0 / 65536.0);
+    if (!(kPT ? geo::pt_ccd_broad<T>(xh, dh, wide) : geo::ee_ccd_broad<T>(xh, dh, wide))) return false;
+    // the CCD's box-gap exit from the rounded coordinates too: they are within
+    // 2^-22 m of the exact relative coordinates and motion per component
+    // (m bounds |x|), so the margins below keep it conservative; most pairs
+    // settle here without loading anything more
+    const T eps = m * T(1.0 / 1048576.0);
+    return !geo::ccd_trivial_approx<T, kPT>(xh, dh, T(4) * eps, T(8) * eps);
+}
+
+template <bool kPT>
+__device__ __forceinline__ bool shares_vertex(const int4 c) {
+    return kPT ? (c.x == c.y || c.x == c.z || c.x == c.w) : (c.x == c.z || c.x == c.w || c.y == c.z || c.y == c.w);
+}
+
 // Mixed mode, stage 1 of a candidate: false when its time of impact is 1
-// without any CCD iteration (shared vertex; the swept-box filter, first on the
-// high parts alone with the distance widened past the largest effect of the
-// dropped low parts (|low| <= 2^-24 |x|, plus the roundings: < 2^-18 of the
-// largest coordinate), then exactly; no motion, or the CCD's box-gap exit).
+// without any CCD iteration (shared vertex; the filters above on the high
+// parts, then exactly; no motion, or the CCD's box-gap exit).
 template <typename T, bool kPT>
 __device__ __forceinline__ bool toi_needs_ccd(const int4 c, const V4<T>* __restrict__ X0h, const V4<T>* __restrict__ X0l,
                                               const V4<T>* __restrict__ X1h, const V4<T>* __restrict__ X1l, T slack) {
-    if (kPT ? (c.x == c.y || c.x == c.z || c.x == c.w) : (c.x == c.z || c.x == c.w || c.y == c.z || c.y == c.w))
-        return false;
+    if (shares_vertex<kPT>(c)) return false;
     const int ids[4] = {c.x, c.y, c.z, c.w};
-    {
-        T xh[4][3], dh[4][3], m = T(0);
-        const V4<T> o = ld4(X0h, ids[0]);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const V4<T> ah = ld4(X0h, ids[j]), bh = ld4(X1h, ids[j]);
-            xh[j][0] = ah.x - o.x;
-            xh[j][1] = ah.y - o.y;
-            xh[j][2] = ah.z - o.z;
-            dh[j][0] = bh.x - ah.x;
-            dh[j][1] = bh.y - ah.y;
-            dh[j][2] = bh.z - ah.z;
-            m = dmax(m, dmax(dmax(fabsf(ah.x), fabsf(ah.y)), dmax(fabsf(ah.z), fabsf(bh.x))));
-            m = dmax(m, dmax(fabsf(bh.y), fabsf(bh.z)));
-        }
-        const T wide = slack + m * T(1.0 / 65536.0);
-        if (!(kPT ? geo::pt_ccd_broad<T>(xh, dh, wide) : geo::ee_ccd_broad<T>(xh, dh, wide))) return false;
-        // the CCD's box-gap exit from the high parts too: they are within
-        // 2^-22 m of the exact relative coordinates and motion per component
-        // (m bounds |x|), so the margins below keep it conservative; most pairs
-        // settle here without loading the low parts
-        const T eps = m * T(1.0 / 1048576.0);
-        if (geo::ccd_trivial_approx<T, kPT>(xh, dh, T(4) * eps, T(8) * eps)) return false;
-    }
+    if (!toi_maybe<T, kPT>(ids, X0h, X1h, slack)) return false;
     T x[4][3], dx[4][3];
     toi_rel<T>(ids, X0h, X0l, X1h, X1l, x, dx);
     if (!(kPT ? geo::pt_ccd_broad<T>(x, dx, slack) : geo::ee_ccd_broad<T>(x, dx, slack))) return false;
@@ -621,6 +634,89 @@ __device__ __forceinline__ TC toi_ccd(const int4 c, const V4<TC>* __restrict__ X
     toi_rel<T>(ids, X0h, X0l, X1h, X1l, x, dx);
     const T tf = kPT ? geo::ccd_pt<T>(x, dx, (T)eta, max_iter) : geo::ccd_ee<T>(x, dx, (T)eta, max_iter);
     return tf < T(1) ? toi_refine<TC, kPT>(X0, X1, ids, eta, max_iter) : TC(1);
+}
+
+// The whole test of one candidate in the state's own arithmetic (FP32 and FP64 modes).
+template <typename TC, bool kPT>
+__device__ __forceinline__ TC toi_exact(const int4 c, const V4<TC>* __restrict__ X0, const V4<TC>* __restrict__ X1,
+                                        TC slack, TC eta, int max_iter) {
+    const int ids[4] = {c.x, c.y, c.z, c.w};
+    TC x[4][3], dx[4][3];
+    gather4<TC, TC>(X0, ids, x);
+    gather4<TC, TC>(X1, ids, dx);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) dx[j][k] -= x[j][k];
+    if (kPT) return geo::pt_ccd_broad<TC>(x, dx, slack) ? geo::ccd_pt<TC>(x, dx, eta, max_iter) : TC(1);
+    return geo::ee_ccd_broad<TC>(x, dx, slack) ? geo::ccd_ee<TC>(x, dx, eta, max_iter) : TC(1);
+}
+
+// positions rounded to FP32 (the FP64 mode's filters)
+__global__ void k_round(int n, const V4<double>* __restrict__ A, V4<float>* __restrict__ a,
+                        const V4<double>* __restrict__ B, V4<float>* __restrict__ b,
+                        const OuterGate* __restrict__ gate) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n || outer_stopped(gate)) return;
+    const V4<double> x = A[i];
+    a[i] = V4<float>{(float)x.x, (float)x.y, (float)x.z, 0.f};
+    if (B) {
+        const V4<double> y = B[i];
+        b[i] = V4<float>{(float)y.x, (float)y.y, (float)y.z, 0.f};
+    }
+}
+
+// The FP64 mode's time of impact.  FP64 arithmetic is what bounds it (the whole
+// test in FP64 for every candidate: 2.45 ms for the 5.4 M candidates of a 257x257
+// cloth over its obstacle), and almost every candidate's time of impact is 1:
+// FP32 filters on rounded positions settle those, warps queue the rest and run
+// the FP64 test on 32 at a time.  A filter only drops candidates whose FP64
+// test gives 1, so the minimum and every per-candidate time keep their bits.
+template <bool kPT>
+__global__ void __launch_bounds__(kBlock, 4) k_toi_f64(int64_t n, const int4* __restrict__ cand,
+                                                       const V4<double>* __restrict__ X0,
+                                                       const V4<double>* __restrict__ X1,
+                                                       const V4<float>* __restrict__ X0h,
+                                                       const V4<float>* __restrict__ X1h, double slack, double eta,
+                                                       int max_iter, double* __restrict__ per,
+                                                       double* __restrict__ toi_min,
+                                                       const OuterGate* __restrict__ gate) {
+    if (outer_stopped(gate)) return;
+    __shared__ int64_t queue[kBlock / 32][64];
+    double local = 1.0;
+    const float wide = __double2float_ru(slack);
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int qn = 0;
+    auto test = [&](int64_t t) {
+        const double toi = toi_exact<double, kPT>(cand[t], X0, X1, slack, eta, max_iter);
+        if (per) per[t] = toi;
+        if (toi < local) local = toi;
+    };
+    const int64_t step = (int64_t)gridDim.x * (kBlock / 32) * 32;
+    for (int64_t base = ((int64_t)blockIdx.x * (kBlock / 32) + w) * 32; base < n; base += step) {
+        const int64_t t = base + lane;
+        bool need = false;
+        if (t < n) {
+            const int4 c = cand[t];
+            const int ids[4] = {c.x, c.y, c.z, c.w};
+            need = !shares_vertex<kPT>(c) && toi_maybe<float, kPT>(ids, X0h, X1h, wide);
+            if (!need && per) per[t] = 1.0;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, need);
+        if (need) queue[w][qn + __popc(m & ((1u << lane) - 1u))] = t;
+        qn += __popc(m);
+        __syncwarp();
+        if (qn >= 32) {
+            const int64_t tq = queue[w][lane];
+            __syncwarp();
+            if (lane < qn - 32) queue[w][lane] = queue[w][lane + 32];
+            __syncwarp();
+            qn -= 32;
+            test(tq);
+        }
+    }
+    if (lane < qn) test(queue[w][lane]);
+    block_min_to(local, toi_min);
 }
 
 // getImpactOfTimeKernel (cu:2610-2704): skip pairs sharing a vertex, swept-AABB
@@ -674,24 +770,7 @@ __global__ void __launch_bounds__(kBlock, kCandBlocks<T>) k_toi(int64_t n, const
     } else {
         for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
             const int4 c = cand[t];
-            const int ids[4] = {c.x, c.y, c.z, c.w};
-            TC toi = TC(1);
-            const bool shared = kPT ? (c.x == c.y || c.x == c.z || c.x == c.w)
-                                    : (c.x == c.z || c.x == c.w || c.y == c.z || c.y == c.w);
-            if (!shared) {
-                TC x[4][3], dx[4][3];
-                gather4<TC, TC>(X0, ids, x);
-                gather4<TC, TC>(X1, ids, dx);
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) dx[j][k] -= x[j][k];
-                if (kPT) {
-                    if (geo::pt_ccd_broad<TC>(x, dx, slack)) toi = geo::ccd_pt<TC>(x, dx, eta, max_iter);
-                } else {
-                    if (geo::ee_ccd_broad<TC>(x, dx, slack)) toi = geo::ccd_ee<TC>(x, dx, eta, max_iter);
-                }
-            }
+            const TC toi = shares_vertex<kPT>(c) ? TC(1) : toi_exact<TC, kPT>(c, X0, X1, slack, eta, max_iter);
             if (per) per[t] = toi;
             if (toi < local) local = toi;
         }
@@ -801,6 +880,44 @@ struct ContactConsts {
     TC dh, dh2, kappa, dt;
 };
 
+// A contact candidate on FP32 coordinates that are the exact ones rounded: false
+// only when the pair is farther apart than dhat for certain (box filter widened
+// as in toi_maybe; the boxes' Euclidean gap bounds the distance from below, and a
+// pair beyond sqrt(2) dhat after the widening fails the exact test).
+template <typename T, bool kPT>
+__device__ __forceinline__ bool contact_maybe(const int* ids, const V4<T>* __restrict__ Xh, T dh, T dh2) {
+    T qh[4][3], m = T(0);
+    const V4<T> o = ld4(Xh, ids[0]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const V4<T> ah = ld4(Xh, ids[j]);
+        qh[j][0] = ah.x - o.x;
+        qh[j][1] = ah.y - o.y;
+        qh[j][2] = ah.z - o.z;
+        m = dmax(m, dmax(fabsf(ah.x), dmax(fabsf(ah.y), fabsf(ah.z))));
+    }
+    const T wide = dh + m * T(1.0 / 65536.0);
+    bool farh = false;
+    if (kPT) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const T tmin = geo::mn3(qh[1][k], qh[2][k], qh[3][k]);
+            const T tmax = geo::mx3(qh[1][k], qh[2][k], qh[3][k]);
+            if ((qh[0][k] - tmax) > wide || (tmin - qh[0][k]) > wide) farh = true;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const T mina = dmin(qh[0][k], qh[1][k]), maxa = dmax(qh[0][k], qh[1][k]);
+            const T minb = dmin(qh[2][k], qh[3][k]), maxb = dmax(qh[2][k], qh[3][k]);
+            if ((mina - maxb) > wide || (minb - maxa) > wide) farh = true;
+        }
+    }
+    if (farh) return false;
+    const T g = dsqrt(kPT ? geo::box_gap2<T, 1, 3>(qh, qh + 1) : geo::box_gap2<T, 2, 2>(qh, qh + 2)) - T(2) * (wide - dh);
+    return !(g > T(0) && g * g > T(2) * dh2);
+}
+
 // setCollisionConstraintsKernel (cu:2756-2892): a pair closer than dhat adds
 // w = kappa b(d^2) + min(m_p, m_q)/dt^2 to the diagonal of its 4 vertices and
 // w * target to their right-hand side; targets push the pair apart to dhat
@@ -825,40 +942,8 @@ __device__ __forceinline__ unsigned contact_candidate(const int4 c, const V4<TC>
         return 0u;
     TC p[4][3];
     if constexpr (kRel) {
-        if (kStage != 2) {  // the box filter on the high parts alone, widened as in k_toi
-            T qh[4][3], m = T(0);
-            const V4<T> o = ld4(Xh, ids[0]);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const V4<T> ah = ld4(Xh, ids[j]);
-                qh[j][0] = ah.x - o.x;
-                qh[j][1] = ah.y - o.y;
-                qh[j][2] = ah.z - o.z;
-                m = dmax(m, dmax(fabsf(ah.x), dmax(fabsf(ah.y), fabsf(ah.z))));
-            }
-            const T wide = (T)cc.dh + m * T(1.0 / 65536.0);
-            bool farh = false;
-            if (kPT) {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const T tmin = geo::mn3(qh[1][k], qh[2][k], qh[3][k]);
-                    const T tmax = geo::mx3(qh[1][k], qh[2][k], qh[3][k]);
-                    if ((qh[0][k] - tmax) > wide || (tmin - qh[0][k]) > wide) farh = true;
-                }
-            } else {
-#pragma unroll
-                for (int k = 0; k < 3; ++k) {
-                    const T mina = dmin(qh[0][k], qh[1][k]), maxa = dmax(qh[0][k], qh[1][k]);
-                    const T minb = dmin(qh[2][k], qh[3][k]), maxb = dmax(qh[2][k], qh[3][k]);
-                    if ((mina - maxb) > wide || (minb - maxa) > wide) farh = true;
-                }
-            }
-            if (farh) return 0u;
-            // the boxes' Euclidean gap also bounds the distance from below: a
-            // pair beyond sqrt(2) dhat (after the widening) fails the filter below
-            const T g = dsqrt(kPT ? geo::box_gap2<T, 1, 3>(qh, qh + 1) : geo::box_gap2<T, 2, 2>(qh, qh + 2)) -
-                        T(2) * (wide - (T)cc.dh);
-            if (g > T(0) && g * g > T(2) * (T)cc.dh2) return 0u;
+        if (kStage != 2) {  // the filters on the high parts alone
+            if (!contact_maybe<T, kPT>(ids, Xh, (T)cc.dh, (T)cc.dh2)) return 0u;
             if (kStage == 1) return 1u;
         }
         T q[4][3];
@@ -1006,6 +1091,54 @@ __global__ void __launch_bounds__(kBlock, kCandBlocks<T>) k_contact(int64_t n, c
     if ((threadIdx.x & 31) == 0 && my) atomicAdd(active, (unsigned long long)my);
 }
 
+// The FP64 mode's contact pass: the FP32 filters on rounded positions first, as
+// in k_toi_f64, then the FP64 test on full warps of survivors (1.22 ms for the
+// 257x257 cloth's candidates with the whole test in FP64).
+template <bool kPT>
+__global__ void __launch_bounds__(kBlock, 4) k_contact_f64(int64_t n, const int4* __restrict__ cand,
+                                                           const V4<double>* __restrict__ X,
+                                                           const V4<float>* __restrict__ Xh,
+                                                           const double* __restrict__ mass,
+                                                           ContactConsts<double> cc, double* __restrict__ diag,
+                                                           V4<double>* __restrict__ rhs,
+                                                           unsigned long long* __restrict__ active,
+                                                           const OuterGate* __restrict__ gate) {
+    if (outer_stopped(gate)) return;
+    __shared__ int64_t queue[kBlock / 32][64];
+    const float dh = __double2float_ru(cc.dh), dh2 = __double2float_ru(cc.dh2);
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    unsigned int my = 0;
+    int qn = 0;
+    auto test = [&](int64_t t) {
+        my += contact_candidate<double, double, kPT, false, 0>(cand[t], X, nullptr, nullptr, mass, cc, diag, rhs);
+    };
+    const int64_t step = (int64_t)gridDim.x * (kBlock / 32) * 32;
+    for (int64_t base = ((int64_t)blockIdx.x * (kBlock / 32) + w) * 32; base < n; base += step) {
+        const int64_t t = base + lane;
+        bool need = false;
+        if (t < n) {
+            const int4 c = cand[t];
+            const int ids[4] = {c.x, c.y, c.z, c.w};
+            need = !shares_vertex<kPT>(c) && contact_maybe<float, kPT>(ids, Xh, dh, dh2);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, need);
+        if (need) queue[w][qn + __popc(m & ((1u << lane) - 1u))] = t;
+        qn += __popc(m);
+        __syncwarp();
+        if (qn >= 32) {
+            const int64_t tq = queue[w][lane];
+            __syncwarp();
+            if (lane < qn - 32) queue[w][lane] = queue[w][lane + 32];
+            __syncwarp();
+            qn -= 32;
+            test(tq);
+        }
+    }
+    if (lane < qn) test(queue[w][lane]);
+    my = warp_sum(my);
+    if (lane == 0 && my) atomicAdd(active, (unsigned long long)my);
+}
+
 }  // namespace
 
 template <typename T, typename TC>
@@ -1063,7 +1196,19 @@ template <typename T, typename TC>
 void launch_toi(const Dev<T, TC>& d, Pos<T, TC> X0, Pos<T, TC> X1, const SolverConsts& c, TC* per_pt,
                 TC* per_ee, cudaStream_t s) {
     constexpr bool kRel = sizeof(T) == 4 && sizeof(TC) == 8;
-    if (c.ccd_mode != 2) {  // the reference's additive CCD
+    if constexpr (std::is_same<T, double>::value) {
+        if (c.ccd_mode != 2 && d.nPT + d.nEE > 0) {
+            k_round<<<blocks_for(d.ntot), kBlock, 0, s>>>(d.ntot, X0.x, d.F0, X1.x, d.F1, d.Gate);
+            if (d.nPT > 0)
+                k_toi_f64<true><<<grid_cap(d.nPT, kBlock, c.cand_grid), kBlock, 0, s>>>(
+                    d.nPT, d.PT, X0.x, X1.x, d.F0, d.F1, c.ccd_slack, c.ccd_eta, c.ccd_max_iter, per_pt, d.ToiMin,
+                    d.Gate);
+            if (d.nEE > 0)
+                k_toi_f64<false><<<grid_cap(d.nEE, kBlock, c.cand_grid), kBlock, 0, s>>>(
+                    d.nEE, d.EE, X0.x, X1.x, d.F0, d.F1, c.ccd_slack, c.ccd_eta, c.ccd_max_iter, per_ee, d.ToiMin,
+                    d.Gate);
+        }
+    } else if (c.ccd_mode != 2) {  // the reference's additive CCD
         if (d.nPT > 0)
             k_toi<T, TC, true, kRel><<<grid_cap(d.nPT, kBlock, c.cand_grid), kBlock, 0, s>>>(
                 d.nPT, d.PT, X0.x, X1.x, X0.hi, X0.lo, X1.hi, X1.lo, (TC)c.ccd_slack, (TC)c.ccd_eta,
@@ -1115,6 +1260,18 @@ void launch_contact(const Dev<T, TC>& d, Pos<T, TC> X, const SolverConsts& c, cu
     cc.kappa = (TC)(T)c.kappa;
     cc.dt = (TC)(T)c.dt;
     constexpr bool kRel = sizeof(T) == 4 && sizeof(TC) == 8;
+    if constexpr (std::is_same<T, double>::value) {
+        if (d.nPT + d.nEE > 0)
+            k_round<<<blocks_for(d.ntot), kBlock, 0, s>>>(d.ntot, X.x, d.F0, (const V4<double>*)nullptr,
+                                                          (V4<float>*)nullptr, d.Gate);
+        if (d.nPT > 0)
+            k_contact_f64<true><<<grid_cap(d.nPT, kBlock, c.cand_grid), kBlock, 0, s>>>(
+                d.nPT, d.PT, X.x, d.F0, d.CollMass, cc, d.CollDiag, d.CollRhs, d.ActiveCount, d.Gate);
+        if (d.nEE > 0)
+            k_contact_f64<false><<<grid_cap(d.nEE, kBlock, c.cand_grid), kBlock, 0, s>>>(
+                d.nEE, d.EE, X.x, d.F0, d.CollMass, cc, d.CollDiag, d.CollRhs, d.ActiveCount, d.Gate);
+        return;
+    } else {
     if (d.nPT > 0)
         k_contact<T, TC, true, kRel><<<grid_cap(d.nPT, kBlock, c.cand_grid), kBlock, 0, s>>>(d.nPT, d.PT, X.x, X.hi, X.lo, d.CollMass,
                                                                          cc, d.CollDiag, d.CollRhs, d.ActiveCount,
@@ -1123,6 +1280,7 @@ void launch_contact(const Dev<T, TC>& d, Pos<T, TC> X, const SolverConsts& c, cu
         k_contact<T, TC, false, kRel><<<grid_cap(d.nEE, kBlock, c.cand_grid), kBlock, 0, s>>>(d.nEE, d.EE, X.x, X.hi, X.lo,
                                                                           d.CollMass, cc, d.CollDiag, d.CollRhs,
                                                                           d.ActiveCount, d.Gate);
+    }
 }
 
 // ---------------- no-allocation scratch of the per-candidate toi pass ----------------

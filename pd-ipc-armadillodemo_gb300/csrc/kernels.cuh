@@ -34,6 +34,9 @@ struct Dev {
     V4<T>* Poh = nullptr;     // [ntot]
     V4<T>* Pol = nullptr;     // [ntot]
     V4<T>* Dh = nullptr;      // (float) Dir [ntot]
+    // FP64 mode only: positions rounded to FP32, rewritten before every use
+    V4<float>* F0 = nullptr;  // [ntot]
+    V4<float>* F1 = nullptr;  // [ntot]
 
     // solver work
     // Y, B, C: [64 ceil(nsim / 64)]; row order on the per-sweep path, slot

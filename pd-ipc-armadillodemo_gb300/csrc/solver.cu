@@ -151,6 +151,10 @@ public:
             launch_split(d, d.P, d.Ph, d.Pl, nt, s_);
             launch_split(d, d.Pold, d.Poh, d.Pol, nt, s_);
         }
+        if (std::is_same<T, double>::value) {
+            PD_CK(zeros(d.F0, nt));
+            PD_CK(zeros(d.F1, nt));
+        }
         PD_CK(zeros(d.X0, ns));
         PD_CK(zeros(d.Vel, ns));
         PD_CK(zeros(d.Dir, nt));
@@ -2344,7 +2348,9 @@ private:
         PD_CK(cudaEventRecordWithFlags(ev[kEvGate], s_, rf));
         launch_copy_old(d, s_);
         // toi x2 (+ cubic), finalize, clamp, contact clear, contact x2, gate, copy into Pold
-        n = (1 + (c_.ccd_mode != 0)) * ((d.nPT > 0) + (d.nEE > 0)) + (d.nPT > 0) + (d.nEE > 0) + 5 +
+        const int lists = (d.nPT > 0) + (d.nEE > 0);
+        n = (1 + (c_.ccd_mode != 0)) * lists + lists + 5 +
+            (std::is_same<T, double>::value && lists ? 1 + (c_.ccd_mode != 2) : 0) +  // FP64: rounded positions
             (inst ? 1 + (d.nPT > 0) + (d.nEE > 0) : 0);
         return PDIPC_OK;
     }
