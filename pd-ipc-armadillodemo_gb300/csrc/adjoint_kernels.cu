@@ -79,64 +79,77 @@ __global__ void k_adj_tables(int nsim, int nslice, const int* __restrict__ lPtr,
     }
 }
 
+// cw[t][j] = (relax D_j^-1) scale_t: the factor of column j in the adjoint of the
+// sweeps whose output adjoint is scaled by scale_t (t = 0: 1; t >= 1: the
+// Chebyshev steps' factors).  Once per step: D does not change in it.
+template <typename T>
+__global__ void k_adj_weights(int nsim, int nt, T relax, const AdjScales<T> sc, const T* __restrict__ InvD,
+                              T* __restrict__ cw) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nsim) return;
+    const T a = relax * InvD[i];
+    for (int t = 0; t < nt; ++t) cw[(size_t)t * nsim + i] = a * sc.s[t];
+}
+
 // Adjoint of one sweep S at input z, output adjoint u = scale * in:
 //   out (= or +=) J^T u;  rho += u;  kbar_i += u_i . dS_i/dk_i;
 // other (if set) += (1 - scale) in: the Chebyshev step's term on X_{t-1}.
+// One component of a row per thread, a block's three warps the x, y and z of the
+// same 32 rows (as k_sweep3: with a row per thread an FP64 sweep of few rows is
+// one long chain per scheduler; a 128x128 rollout of two steps and its
+// gradients 70.4 ms, split 56.3).
+constexpr int kRows3 = 32;
 template <typename T>
-__global__ void __launch_bounds__(kBlock) k_adj_sweep(
-    int nsim, T relax, T scale, const V4<T>* __restrict__ in, V4<T>* __restrict__ other,
+__global__ void __launch_bounds__(3 * kRows3) k_adj_sweep(
+    int nsim, T relax, T scale, const T* __restrict__ cw, const V4<T>* __restrict__ in, V4<T>* __restrict__ other,
     const V4<T>* __restrict__ z, V4<T>* __restrict__ out, int accumulate, V4<T>* __restrict__ rho,
     T* __restrict__ kbar, const V4<T>* __restrict__ Rhs, const T* __restrict__ InvD, const int* __restrict__ sOff,
     const int* __restrict__ sLen, const int* __restrict__ sCol, const T* __restrict__ sVal,
     const T* __restrict__ NTval, const int* __restrict__ lPtr, const int* __restrict__ lNbr) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nsim) return;
-    const V4<T> a = in[i];
-    const V4<T> u{scale * a.x, scale * a.y, scale * a.z, T(0)};
-    const T idi = InvD[i];
-    const int sl = i >> 5, base = sOff[sl] + (i & 31), len = sLen[sl];
-    T j0 = T(0), j1 = T(0), j2 = T(0);  // sum_j N_ji w D_j^-1 u_j
-    T n0 = T(0), n1 = T(0), n2 = T(0);  // (N z)_i
-    for (int k = 0; k < len; ++k) {
-        const int at = base + 32 * k;
-        const int j = sCol[at];
-        const T c = NTval[at] * (relax * InvD[j] * scale);
-        const V4<T> aj = in[j];
-        j0 += c * aj.x;
-        j1 += c * aj.y;
-        j2 += c * aj.z;
-        const T v = sVal[at];
-        const V4<T> zj = z[j];
-        n0 += v * zj.x;
-        n1 += v * zj.y;
-        n2 += v * zj.z;
+    __shared__ T us[3][kRows3], gs[3][kRows3];
+    const int l = threadIdx.x % kRows3, c = threadIdx.x / kRows3, i = blockIdx.x * kRows3 + l;
+    const bool live = i < nsim;
+    auto comp = [&](const V4<T>* v, int j) -> const T* { return reinterpret_cast<const T*>(v + j) + c; };
+    T idi = T(0);
+    if (live) {
+        const T a = *comp(in, i);
+        const T u = scale * a;
+        idi = __ldg(InvD + i);
+        const int sl = i >> 5, base = __ldg(sOff + sl) + (i & 31), len = __ldg(sLen + sl);
+        T js = T(0);  // sum_j N_ji w D_j^-1 u_j
+        T ns = T(0);  // (N z)_i
+#pragma unroll 4
+        for (int k = 0; k < len; ++k) {
+            const int at = base + 32 * k;
+            const int j = __ldg(sCol + at);
+            const T f = __ldg(NTval + at) * __ldg(cw + j);
+            js += f * __ldg(comp(in, j));
+            ns += __ldg(sVal + at) * __ldg(comp(z, j));
+        }
+        const int b = __ldg(lPtr + i), e = __ldg(lPtr + i + 1);
+        T ss = T(0);  // sum of the spring neighbours' z
+#pragma unroll 4
+        for (int s = b + 1; s < e; ++s) ss += __ldg(comp(z, __ldg(lNbr + s)));
+        const T dg = T(e - b - 1) * idi;
+        us[c][l] = u;
+        gs[c][l] = ss - dg * (ns + *comp(Rhs, i));
+        T* r = const_cast<T*>(comp(rho, i));
+        *r += u;
+        if (other) {
+            T* o = const_cast<T*>(comp(other, i));
+            *o += (T(1) - scale) * a;
+        }
+        const T om = T(1) - relax;
+        T y = om * u + js;
+        T* w = const_cast<T*>(comp(out, i));
+        if (accumulate) y = *w + y;
+        *w = y;
     }
-    const int b = lPtr[i], e = lPtr[i + 1];
-    T s0 = T(0), s1 = T(0), s2 = T(0);  // sum of the spring neighbours' z
-    for (int s = b + 1; s < e; ++s) {
-        const V4<T> zj = z[lNbr[s]];
-        s0 += zj.x;
-        s1 += zj.y;
-        s2 += zj.z;
+    __syncthreads();
+    if (live && c == 0) {
+        const V4<T> u{us[0][l], us[1][l], us[2][l], T(0)}, g{gs[0][l], gs[1][l], gs[2][l], T(0)};
+        kbar[i] += relax * idi * dot3(u, g);
     }
-    const V4<T> r = Rhs[i];
-    const T dg = T(e - b - 1) * idi;
-    const V4<T> g{s0 - dg * (n0 + r.x), s1 - dg * (n1 + r.y), s2 - dg * (n2 + r.z), T(0)};
-    kbar[i] += relax * idi * dot3(u, g);
-    V4<T> p = rho[i];
-    rho[i] = V4<T>{p.x + u.x, p.y + u.y, p.z + u.z, T(0)};
-    if (other) {
-        const T f = T(1) - scale;
-        const V4<T> o = other[i];
-        other[i] = V4<T>{o.x + f * a.x, o.y + f * a.y, o.z + f * a.z, T(0)};
-    }
-    const T om = T(1) - relax;
-    V4<T> y{om * u.x + j0, om * u.y + j1, om * u.z + j2, T(0)};
-    if (accumulate) {
-        const V4<T> q = out[i];
-        y = V4<T>{q.x + y.x, q.y + y.y, q.z + y.z, T(0)};
-    }
-    out[i] = y;
 }
 
 // adjoint of the right-hand side: rb = w D^-1 rho; rhs0's adjoint collects it
@@ -462,11 +475,16 @@ void launch_adj_tables(const Dev<T, TC>& d, T* lLboT, T* NTval, cudaStream_t s) 
                                                      d.sCol, d.sVal, lLboT, NTval);
 }
 template <typename T, typename TC>
-void launch_adj_sweep(const Dev<T, TC>& d, const T* NTval, T relax, T scale, const V4<T>* in, V4<T>* other,
-                      const V4<T>* z, V4<T>* out, bool accumulate, V4<T>* rho, T* kbar, cudaStream_t s) {
-    k_adj_sweep<T><<<blocks_for(d.nsim), kBlock, 0, s>>>(d.nsim, relax, scale, in, other, z, out, accumulate ? 1 : 0,
-                                                         rho, kbar, d.Rhs, d.InvD, d.sOff, d.sLen, d.sCol, d.sVal,
-                                                         NTval, d.lPtr, d.lNbr);
+void launch_adj_weights(const Dev<T, TC>& d, T relax, const AdjScales<T>& sc, int nt, T* cw, cudaStream_t s) {
+    k_adj_weights<T><<<blocks_for(d.nsim), kBlock, 0, s>>>(d.nsim, nt, relax, sc, d.InvD, cw);
+}
+template <typename T, typename TC>
+void launch_adj_sweep(const Dev<T, TC>& d, const T* NTval, const T* cw, T relax, T scale, const V4<T>* in,
+                      V4<T>* other, const V4<T>* z, V4<T>* out, bool accumulate, V4<T>* rho, T* kbar,
+                      cudaStream_t s) {
+    k_adj_sweep<T><<<blocks_for(d.nsim, kRows3), 3 * kRows3, 0, s>>>(
+        d.nsim, relax, scale, cw, in, other, z, out, accumulate ? 1 : 0, rho, kbar, d.Rhs, d.InvD, d.sOff, d.sLen,
+        d.sCol, d.sVal, NTval, d.lPtr, d.lNbr);
 }
 template <typename T, typename TC>
 void launch_adj_local(const Dev<T, TC>& d, const T* lLboT, T relax, const V4<T>* x, const V4<T>* rho, V4<T>* rb,
@@ -491,8 +509,10 @@ void launch_adj_step_end(const Dev<T, TC>& d, T dt, V4<T>* pb, V4<T>* vb, const 
 }
 
 template void launch_adj_tables<double, double>(const Dev<double, double>&, double*, double*, cudaStream_t);
-template void launch_adj_sweep<double, double>(const Dev<double, double>&, const double*, double, double,
-                                               const V4<double>*, V4<double>*, const V4<double>*, V4<double>*,
+template void launch_adj_weights<double, double>(const Dev<double, double>&, double, const AdjScales<double>&, int,
+                                                 double*, cudaStream_t);
+template void launch_adj_sweep<double, double>(const Dev<double, double>&, const double*, const double*, double,
+                                               double, const V4<double>*, V4<double>*, const V4<double>*, V4<double>*,
                                                bool, V4<double>*, double*, cudaStream_t);
 template void launch_adj_local<double, double>(const Dev<double, double>&, const double*, double,
                                                const V4<double>*, const V4<double>*, V4<double>*, V4<double>*,

@@ -333,11 +333,21 @@ void launch_pen_uniform(const Dev<T, TC>& d, V4<TC>* F, const int* times, TC dam
 // values in the SELL layout of sVal
 template <typename T, typename TC>
 void launch_adj_tables(const Dev<T, TC>& d, T* lLboT, T* NTval, cudaStream_t s);
-// one sweep's adjoint at input z with output adjoint scale * in:
+// the factors relax D_j^-1 scale of the sweeps' adjoints, for each scale
+constexpr int kMaxAdjScales = 64;
+template <typename T>
+struct AdjScales {
+    T s[kMaxAdjScales];
+};
+template <typename T, typename TC>
+void launch_adj_weights(const Dev<T, TC>& d, T relax, const AdjScales<T>& sc, int nt, T* cw, cudaStream_t s);
+// one sweep's adjoint at input z with output adjoint scale * in (cw: its
+// factors of launch_adj_weights):
 // out (= or +=) J^T u, rho += u, kbar += dS/dk . u, other += (1 - scale) in
 template <typename T, typename TC>
-void launch_adj_sweep(const Dev<T, TC>& d, const T* NTval, T relax, T scale, const V4<T>* in, V4<T>* other,
-                      const V4<T>* z, V4<T>* out, bool accumulate, V4<T>* rho, T* kbar, cudaStream_t s);
+void launch_adj_sweep(const Dev<T, TC>& d, const T* NTval, const T* cw, T relax, T scale, const V4<T>* in,
+                      V4<T>* other, const V4<T>* z, V4<T>* out, bool accumulate, V4<T>* rho, T* kbar,
+                      cudaStream_t s);
 // the local step's adjoint at x from rho (sum of the sweeps' output adjoints):
 // rb, qb scratch; r0b += w D^-1 rho; xb += d(rhs)/dx^T rb; kbar += d(rhs)/dk . rb;
 // with strain-limit elements (tets, cloth triangles) their SVD-derivative

@@ -292,6 +292,55 @@ __global__ void __launch_bounds__(kBlock) k_sweep(int nsim, T relax, T omega, co
     out[i] = V4<T>{y0, y1, y2, T(0)};
 }
 
+// The FP64 sweep, one component of a row per thread: a block's three warps take
+// the x, y and z of the same 32 rows.  A warp's FP64 instruction occupies its
+// scheduler's FP64 unit for 64 cycles, so a row of 24 entries costs a thread
+// that does all three components 2.5 us however few rows there are; split, a
+// third of that, and three times the warps hide the gathers.  Same operations
+// per component as k_sweep: the results keep its bits.  Measured (GB300, one
+// sweep with its launch): 64x64 10.3 -> 6.2 us, 128x128 10.3 -> 8.2, 257x257 15.5 ->
+// 14.4, 512x512 43.1 -> 45.0: past kSplitRows the FP64 units are full either way and
+// k_sweep, which loads offsets and values once per row, is the faster one.
+constexpr int kRows3 = 32, kSplitRows = 1 << 17;
+template <bool kCheby>
+__global__ void __launch_bounds__(3 * kRows3) k_sweep3(int nsim, double relax, double omega,
+                                                       const V4<double>* __restrict__ src,
+                                                       const V4<double>* __restrict__ prev, V4<double>* __restrict__ out,
+                                                       const V4<double>* __restrict__ Rhs,
+                                                       const double* __restrict__ InvD, const Sell<double> M,
+                                                       const RowSkip skip) {
+    const int c = threadIdx.x / kRows3, i = blockIdx.x * kRows3 + threadIdx.x % kRows3;
+    if (i >= nsim || skip(i)) return;
+    const double* __restrict__ x = reinterpret_cast<const double*>(src) + c;
+    const int base = __ldg(M.off + (i >> 5)) + (i & 31), len = __ldg(M.len + (i >> 5));
+    const int16_t* po = M.rowPat ? M.patOff + (size_t)__ldg(M.rowPat + i) * M.patW : nullptr;
+    double s = 0.0;
+    // batches of eight entries in flight: a row's loads are two dependent L2
+    // accesses (column, then gather), and a batch pays them once
+    constexpr int kB = 8;
+    for (int k0 = 0; k0 < len; k0 += kB) {
+        double v[kB], xj[kB];
+#pragma unroll
+        for (int q = 0; q < kB; ++q) {
+            const int k = min(k0 + q, len - 1);
+            const int j = po ? i + (int)__ldg(po + k) : __ldg(M.col + base + 32 * k);
+            v[q] = __ldg(M.val + base + 32 * k);
+            xj[q] = __ldg(x + 4 * (size_t)j);
+        }
+#pragma unroll
+        for (int q = 0; q < kB; ++q)
+            if (k0 + q < len) s = __fma_rn(v[q], xj[q], s);
+    }
+    const size_t at = 4 * (size_t)i;
+    const double t = __dmul_rn(__dadd_rn(s, __ldg(reinterpret_cast<const double*>(Rhs) + at + c)), __ldg(InvD + i));
+    double y = __fma_rn(1.0 - relax, __ldg(x + at), __dmul_rn(relax, t));
+    if (kCheby) {  // prev may be the vector this row overwrites: the row's own value only
+        const double p = reinterpret_cast<const double*>(prev)[at + c];
+        y = __fma_rn(omega, __dadd_rn(y, -p), p);
+    }
+    reinterpret_cast<double*>(out)[at + c] = y;
+}
+
 // Correction form, one vertex per thread.  With x the current positions,
 //   r0 = b - A x
 //      = Dinert (y - x) + k_pin (X_rest - x) + sum_c w_c (target_c - x_c) + Dcoll (x_c - x)
@@ -709,6 +758,18 @@ void launch_local_rhs_sweep(const Dev<T, TC>& d, T relax, cudaStream_t s) {
 template <typename T, typename TC>
 void launch_sweep(const Dev<T, TC>& d, const V4<T>* src, const V4<T>* prev, V4<T>* out, T relax, T omega,
                   cudaStream_t s) {
+    if constexpr (std::is_same<T, double>::value) {
+        if (d.nsim <= kSplitRows) {
+            const int nb = blocks_for(d.nsim, kRows3);
+            if (prev)
+                k_sweep3<true><<<nb, 3 * kRows3, 0, s>>>(d.nsim, relax, omega, src, prev, out, d.Rhs, d.InvD,
+                                                         sell_of(d), skip_of(d));
+            else
+                k_sweep3<false><<<nb, 3 * kRows3, 0, s>>>(d.nsim, relax, omega, src, prev, out, d.Rhs, d.InvD,
+                                                          sell_of(d), skip_of(d));
+            return;
+        }
+    }
     if (prev)
         k_sweep<T, true><<<blocks_for(d.nsim), kBlock, 0, s>>>(d.nsim, relax, omega, src, prev, out, d.Rhs, d.InvD,
                                                               sell_of(d), skip_of(d));

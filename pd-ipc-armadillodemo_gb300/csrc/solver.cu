@@ -1132,6 +1132,7 @@ private:
         PD_CK(alloc(adj_ntval_, (size_t)sell_padded_));
         PD_CK(alloc(adj_final_, 2 * (size_t)ns));
         PD_CK(alloc(adj_kb_, (size_t)ns));
+        PD_CK(alloc(adj_cw_, (size_t)cb * ns));
         if (d_.ntet > 0) PD_CK(alloc(adj_eb_, 4 * (size_t)d_.ntet));
         for (V4<TC>** b : {&adj_pb_, &adj_vb_, &adj_r0b_, &adj_rb_, &adj_qb_, &adj_u_, &adj_rho_})
             PD_CK(alloc(*b, (size_t)ns));
@@ -1167,6 +1168,14 @@ private:
                 }
             }
             if (tile_on_) launch_diag(d, s_);  // the tiled solve keeps its diagonal in registers
+            {   // the sweeps' column factors: scale 1, then the Chebyshev steps'
+                AdjScales<T> sc;
+                for (int t0 = 0; t0 < cb; t0 += kMaxAdjScales) {
+                    const int nt = std::min(kMaxAdjScales, cb - t0);
+                    for (int t = 0; t < nt; ++t) sc.s[t] = t0 + t ? oms[t0 + t - 1] : T(1);
+                    launch_adj_weights(d, w, sc, nt, adj_cw_ + (size_t)t0 * ns, s_);
+                }
+            }
             launch_adj_step_begin(d, invt, adj_pb_, adj_vb_, adj_r0b_, s_);
             const size_t vb = sizeof(V4<TC>) * ns;
             for (int l = adj_tape_n_ - 1; l >= 0; --l) {
@@ -1188,14 +1197,14 @@ private:
                 PD_CK(cudaMemsetAsync(adj_rho_, 0, vb, s_));
                 std::swap(adj_xb_[cb], adj_pb_);
                 for (int it = cb - 1; it >= 1; --it) {
-                    launch_adj_sweep(d, adj_ntval_, w, oms[it - 1], adj_xb_[it + 1], adj_xb_[it - 1], adj_ys_[it],
+                    launch_adj_sweep(d, adj_ntval_, adj_cw_ + (size_t)it * ns, w, oms[it - 1], adj_xb_[it + 1], adj_xb_[it - 1], adj_ys_[it],
                                      adj_u_, false, adj_rho_, adj_kb_, s_);
-                    launch_adj_sweep(d, adj_ntval_, w, T(1), adj_u_, (V4<T>*)nullptr, adj_xs_[it], adj_xb_[it], true,
+                    launch_adj_sweep(d, adj_ntval_, adj_cw_, w, T(1), adj_u_, (V4<T>*)nullptr, adj_xs_[it], adj_xb_[it], true,
                                      adj_rho_, adj_kb_, s_);
                 }
-                launch_adj_sweep(d, adj_ntval_, w, T(1), adj_xb_[1], (V4<T>*)nullptr, adj_ys_[0], adj_u_, false,
+                launch_adj_sweep(d, adj_ntval_, adj_cw_, w, T(1), adj_xb_[1], (V4<T>*)nullptr, adj_ys_[0], adj_u_, false,
                                  adj_rho_, adj_kb_, s_);
-                launch_adj_sweep(d, adj_ntval_, w, T(1), adj_u_, (V4<T>*)nullptr, adj_xs_[0], adj_xb_[0], true,
+                launch_adj_sweep(d, adj_ntval_, adj_cw_, w, T(1), adj_u_, (V4<T>*)nullptr, adj_xs_[0], adj_xb_[0], true,
                                  adj_rho_, adj_kb_, s_);
                 launch_adj_local(d, adj_lboT_, w, x, adj_rho_, adj_rb_, adj_qb_, adj_r0b_, adj_xb_[0], adj_kb_,
                                  adj_eb_, s_);
@@ -2538,6 +2547,7 @@ private:
     T* adj_lboT_ = nullptr;
     T* adj_ntval_ = nullptr;
     T* adj_kb_ = nullptr;
+    T* adj_cw_ = nullptr;
     V4<TC>* adj_eb_ = nullptr;  // strain-limit elements' adjoints (4 per element)
     V4<TC>* adj_final_ = nullptr;
     V4<TC>*adj_pb_ = nullptr, *adj_vb_ = nullptr, *adj_r0b_ = nullptr, *adj_rb_ = nullptr, *adj_qb_ = nullptr,
