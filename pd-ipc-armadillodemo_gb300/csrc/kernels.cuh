@@ -274,6 +274,11 @@ void launch_inst_gate(const Dev<T, TC>& d, double tol, bool test, cudaStream_t s
 // positions X, after a host write of X
 template <typename T, typename TC>
 void launch_split(const Dev<T, TC>& d, const V4<TC>* X, V4<T>* hi, V4<T>* lo, int n, cudaStream_t s);
+// a state vector from and to the host's layout, three doubles a vertex
+template <typename TC>
+void launch_unpack(V4<TC>* dst, const double* raw, int n, cudaStream_t s);
+template <typename TC>
+void launch_pack(double* raw, const V4<TC>* src, int n, cudaStream_t s);
 int direction_blocks(int nsim);
 
 // ---------------- collision kernels (collision_kernels.cu) ----------------

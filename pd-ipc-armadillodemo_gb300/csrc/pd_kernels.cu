@@ -582,6 +582,25 @@ __global__ void k_split(int n, const V4<double>* __restrict__ X, V4<float>* __re
     }
 }
 
+// one vertex per thread; a warp's 24-byte vertices are six whole 128-byte lines
+template <typename S>
+__global__ void k_unpack(int n, const double* __restrict__ raw, V4<S>* __restrict__ X) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double* q = raw + 3 * (size_t)i;
+    X[i] = V4<S>{(S)q[0], (S)q[1], (S)q[2], S(0)};
+}
+template <typename S>
+__global__ void k_pack(int n, const V4<S>* __restrict__ X, double* __restrict__ raw) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const V4<S> x = X[i];
+    double* q = raw + 3 * (size_t)i;
+    q[0] = (double)x.x;
+    q[1] = (double)x.y;
+    q[2] = (double)x.z;
+}
+
 template <typename T, typename S>
 __global__ void k_copy_old(int nsim, const V4<S>* __restrict__ P, V4<S>* __restrict__ Pold,
                            const V4<T>* __restrict__ Ph, const V4<T>* __restrict__ Pl, V4<T>* __restrict__ Poh,
@@ -794,6 +813,14 @@ void launch_split(const Dev<T, TC>& d, const V4<TC>* X, V4<T>* hi, V4<T>* lo, in
         if (n > 0) k_split<<<blocks_for(n), kBlock, 0, s>>>(n, X, hi, lo);
     }
 }
+template <typename TC>
+void launch_unpack(V4<TC>* dst, const double* raw, int n, cudaStream_t s) {
+    if (n > 0) k_unpack<TC><<<blocks_for(n), kBlock, 0, s>>>(n, raw, dst);
+}
+template <typename TC>
+void launch_pack(double* raw, const V4<TC>* src, int n, cudaStream_t s) {
+    if (n > 0) k_pack<TC><<<blocks_for(n), kBlock, 0, s>>>(n, src, raw);
+}
 template <typename T, typename TC>
 void launch_copy_old(const Dev<T, TC>& d, cudaStream_t s) {
     k_copy_old<T, TC><<<blocks_for(d.nsim), kBlock, 0, s>>>(d.nsim, d.P, d.Pold, d.Ph, d.Pl, d.Poh, d.Pol, d.Gate);
@@ -835,6 +862,11 @@ void launch_velocity(const Dev<T, TC>& d, TC invt, cudaStream_t s) {
     template void launch_inst_gate<T, TC>(const Dev<T, TC>&, double, bool, cudaStream_t);                    \
     template void launch_split<T, TC>(const Dev<T, TC>&, const V4<TC>*, V4<T>*, V4<T>*, int, cudaStream_t);  \
     template void launch_velocity<T, TC>(const Dev<T, TC>&, TC, cudaStream_t);
+
+template void launch_unpack<float>(V4<float>*, const double*, int, cudaStream_t);
+template void launch_unpack<double>(V4<double>*, const double*, int, cudaStream_t);
+template void launch_pack<float>(double*, const V4<float>*, int, cudaStream_t);
+template void launch_pack<double>(double*, const V4<double>*, int, cudaStream_t);
 
 PDIPC_INST_PD(float, float)
 PDIPC_INST_PD(double, double)

@@ -21,6 +21,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <type_traits>
 
 #include "kernels.cuh"
@@ -394,7 +395,8 @@ public:
         }
         PD_CK(cudaMallocHost(&pin_, sizeof(Pinned)));
         std::memset(pin_, 0, sizeof(Pinned));
-        PD_CK(cudaMallocHost(&stage_, sizeof(V4<TC>) * (size_t)std::max(nt, 1)));
+        PD_CK(alloc(raw_, 3 * (size_t)std::max(nt, 1)));
+        PD_CK(cudaMallocHost(&stage_, sizeof(double) * 3 * (size_t)std::max(nt + ns, 1)));
 
         // ---- persistent PD solve plan (needs every buffer above) ----
         pdipc_status pr = plan_persistent(H, err);
@@ -711,30 +713,55 @@ public:
     }
 
     pdipc_status get_positions(double* out, std::string& err) override {
-        PD_CK(cudaMemcpyAsync(stage_, d_.P, sizeof(V4<TC>) * d_.ntot, cudaMemcpyDeviceToHost, s_));
-        PD_CK(cudaStreamSynchronize(s_));
-        for (int i = 0; i < d_.ntot; ++i) {
-            out[3 * (size_t)i] = (double)stage_[i].x;
-            out[3 * (size_t)i + 1] = (double)stage_[i].y;
-            out[3 * (size_t)i + 2] = (double)stage_[i].z;
-        }
-        return PDIPC_OK;
+        return download_vec(d_.P, out, d_.ntot, err);
     }
     pdipc_status get_velocities(double* out, std::string& err) override {
-        PD_CK(cudaMemcpyAsync(stage_, d_.Vel, sizeof(V4<TC>) * d_.nsim, cudaMemcpyDeviceToHost, s_));
-        PD_CK(cudaStreamSynchronize(s_));
-        for (int i = 0; i < d_.nsim; ++i) {
-            out[3 * (size_t)i] = (double)stage_[i].x;
-            out[3 * (size_t)i + 1] = (double)stage_[i].y;
-            out[3 * (size_t)i + 2] = (double)stage_[i].z;
-        }
+        return download_vec(d_.Vel, out, d_.nsim, err);
+    }
+    // Host vectors are three doubles a vertex, device ones aligned 4-vectors of
+    // the state scalar: copies move the host's own layout and a kernel repacks it.
+    // Up: through a pinned buffer, filled by a few threads when it is large (a
+    // packing loop took 600 us for 7.3 MB; the copy engine reads pageable memory
+    // it has seen at link speed, 60 us, but needs 1-3 ms for a fresh array).
+    // Down: straight to the caller's memory, whose pages are mapped first (100 us;
+    // the copy engine faulting fresh pages in took 1-1.5 ms).  enqueue_vec leaves
+    // the copy in flight from the buffer's part at `at`.
+    pdipc_status enqueue_vec(V4<TC>* dst, const double* src, int n, int at, std::string& err) {
+        double* part = stage_ + 3 * (size_t)at;
+        copy_host(part, src, sizeof(double) * 3 * (size_t)n);
+        PD_CK(cudaMemcpyAsync(raw_, part, sizeof(double) * 3 * (size_t)n, cudaMemcpyHostToDevice, s_));
+        launch_unpack(dst, raw_, n, s_);
         return PDIPC_OK;
     }
     pdipc_status upload_vec(V4<TC>* dst, const double* src, int n, std::string& err) {
+        pdipc_status r = enqueue_vec(dst, src, n, 0, err);
+        if (r != PDIPC_OK) return r;
         PD_CK(cudaStreamSynchronize(s_));
-        for (int i = 0; i < n; ++i)
-            stage_[i] = V4<TC>{(TC)src[3 * (size_t)i], (TC)src[3 * (size_t)i + 1], (TC)src[3 * (size_t)i + 2], TC(0)};
-        PD_CK(cudaMemcpyAsync(dst, stage_, sizeof(V4<TC>) * n, cudaMemcpyHostToDevice, s_));
+        return PDIPC_OK;
+    }
+    static void copy_host(double* dst, const double* src, size_t bytes) {
+        constexpr size_t kPart = (size_t)1 << 20;  // below, a thread costs more than it saves
+        const size_t parts = std::min<size_t>(6, bytes / kPart + 1);
+        const size_t len = (bytes / parts + 63) / 64 * 64;
+        auto part = [=](size_t k) {
+            const size_t b = std::min(bytes, k * len), e = std::min(bytes, b + len);
+            std::memcpy(reinterpret_cast<char*>(dst) + b, reinterpret_cast<const char*>(src) + b, e - b);
+        };
+        std::vector<std::thread> th;
+        size_t started = 1;
+        try {
+            for (; started < parts; ++started) th.emplace_back(part, started);
+        } catch (...) {  // no thread to be had: this one copies the rest
+        }
+        part(0);
+        for (size_t k = started; k < parts; ++k) part(k);
+        for (std::thread& t : th) t.join();
+    }
+    pdipc_status download_vec(const V4<TC>* src, double* dst, int n, std::string& err) {
+        launch_pack(raw_, src, n, s_);
+        volatile char* page = reinterpret_cast<volatile char*>(dst);
+        for (size_t b = 0; b < sizeof(double) * 3 * (size_t)n; b += 4096) page[b] = 0;
+        PD_CK(cudaMemcpyAsync(dst, raw_, sizeof(double) * 3 * (size_t)n, cudaMemcpyDeviceToHost, s_));
         PD_CK(cudaStreamSynchronize(s_));
         return PDIPC_OK;
     }
@@ -744,10 +771,12 @@ public:
     }
     // positions (and velocities) to the device without touching a recording
     pdipc_status put_state(const double* X, const double* V, std::string& err) {
-        pdipc_status r = upload_vec(d_.P, X, d_.ntot, err);
+        pdipc_status r = enqueue_vec(d_.P, X, d_.ntot, 0, err);
+        if (r == PDIPC_OK) launch_split(d_, d_.P, d_.Ph, d_.Pl, d_.ntot, s_);
+        if (r == PDIPC_OK && V) r = enqueue_vec(d_.Vel, V, d_.nsim, d_.ntot, err);
+        const cudaError_t e = cudaStreamSynchronize(s_);  // the buffer is free again, on errors too
         if (r != PDIPC_OK) return r;
-        launch_split(d_, d_.P, d_.Ph, d_.Pl, d_.ntot, s_);
-        if (V) return upload_vec(d_.Vel, V, d_.nsim, err);
+        PD_CK(e);
         return PDIPC_OK;
     }
     pdipc_status reset(std::string& err) override {
@@ -933,16 +962,6 @@ public:
             PD_CK(zeros(pen_f_, d_.ntot));
             PD_CK(zeros(pen_v_, d_.nsim));
             PD_CK(zeros(pen_t_, d_.ntot));
-        }
-        return PDIPC_OK;
-    }
-    pdipc_status download_vec(const V4<TC>* src, double* dst, int n, std::string& err) {
-        PD_CK(cudaMemcpyAsync(stage_, src, sizeof(V4<TC>) * n, cudaMemcpyDeviceToHost, s_));
-        PD_CK(cudaStreamSynchronize(s_));
-        for (int i = 0; i < n; ++i) {
-            dst[3 * (size_t)i] = (double)stage_[i].x;
-            dst[3 * (size_t)i + 1] = (double)stage_[i].y;
-            dst[3 * (size_t)i + 2] = (double)stage_[i].z;
         }
         return PDIPC_OK;
     }
@@ -1300,20 +1319,9 @@ private:
             err = e2;
             return rl;
         }
-        PD_CK(cudaMemcpyAsync(stage_, adj_pb_, sizeof(V4<TC>) * ns, cudaMemcpyDeviceToHost, s_));
-        PD_CK(cudaStreamSynchronize(s_));
-        for (int i = 0; i < ns; ++i) {
-            gx0[3 * (size_t)i] = (double)stage_[i].x;
-            gx0[3 * (size_t)i + 1] = (double)stage_[i].y;
-            gx0[3 * (size_t)i + 2] = (double)stage_[i].z;
-        }
-        PD_CK(cudaMemcpyAsync(stage_, adj_vb_, sizeof(V4<TC>) * ns, cudaMemcpyDeviceToHost, s_));
-        PD_CK(cudaStreamSynchronize(s_));
-        for (int i = 0; i < ns; ++i) {
-            gv0[3 * (size_t)i] = (double)stage_[i].x;
-            gv0[3 * (size_t)i + 1] = (double)stage_[i].y;
-            gv0[3 * (size_t)i + 2] = (double)stage_[i].z;
-        }
+        r = download_vec(adj_pb_, gx0, ns, err);
+        if (r == PDIPC_OK) r = download_vec(adj_vb_, gv0, ns, err);
+        if (r != PDIPC_OK) return r;
         if (gk) {
             PD_CK(cudaMemcpyAsync(gk, adj_kb_, sizeof(T) * ns, cudaMemcpyDeviceToHost, s_));
             PD_CK(cudaStreamSynchronize(s_));
@@ -1388,8 +1396,8 @@ private:
         ptrs_.clear();
         if (pin_) cudaFreeHost(pin_);
         if (stage_) cudaFreeHost(stage_);
-        pin_ = nullptr;
         stage_ = nullptr;
+        pin_ = nullptr;
         if (ev0_) cudaEventDestroy(ev0_);
         if (ev1_) cudaEventDestroy(ev1_);
         for (auto& ring : evo_)
@@ -2579,7 +2587,8 @@ private:
     int* pCtaTetPtr_ = nullptr;   // per-CTA range of the tets it projects
     int* pCtaTetIdx_ = nullptr;
     unsigned epoch_ = 1;
-    V4<TC>* stage_ = nullptr;  // pinned host staging of one state vector
+    double* stage_ = nullptr;  // pinned: positions of every vertex, then velocities, in the host's layout
+    double* raw_ = nullptr;  // one state vector in the host's layout (three doubles a vertex)
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t graph_exec_ = nullptr;
     int graph_nodes_ = 0;
