@@ -882,8 +882,9 @@ struct ContactConsts {
 
 // A contact candidate on FP32 coordinates that are the exact ones rounded: false
 // only when the pair is farther apart than dhat for certain (box filter widened
-// as in toi_maybe; the boxes' Euclidean gap bounds the distance from below, and a
-// pair beyond sqrt(2) dhat after the widening fails the exact test).
+// as in toi_maybe; the boxes' Euclidean gap and the separation along the diagonals
+// bound the distance from below, and a pair beyond sqrt(2) dhat after the widening
+// fails the exact test).
 template <typename T, bool kPT>
 __device__ __forceinline__ bool contact_maybe(const int* ids, const V4<T>* __restrict__ Xh, T dh, T dh2) {
     T qh[4][3], m = T(0);
@@ -914,7 +915,9 @@ __device__ __forceinline__ bool contact_maybe(const int* ids, const V4<T>* __res
         }
     }
     if (farh) return false;
-    const T g = dsqrt(kPT ? geo::box_gap2<T, 1, 3>(qh, qh + 1) : geo::box_gap2<T, 2, 2>(qh, qh + 2)) - T(2) * (wide - dh);
+    T g = dsqrt(kPT ? geo::box_gap2<T, 1, 3>(qh, qh + 1) : geo::box_gap2<T, 2, 2>(qh, qh + 2)) - T(2) * (wide - dh);
+    if (g > T(0) && g * g > T(2) * dh2) return false;
+    g = (kPT ? geo::diagonal_gap<T, 1, 3>(qh, qh + 1) : geo::diagonal_gap<T, 2, 2>(qh, qh + 2)) - T(4) * (wide - dh);
     return !(g > T(0) && g * g > T(2) * dh2);
 }
 

@@ -178,6 +178,38 @@ __device__ __forceinline__ R box_gap2(const R (*a)[3], const R (*b)[3]) {
     return g2;
 }
 
+// Largest separation of points a[0..na) and b[0..nb) along the six diagonals of
+// the coordinate planes (unit vectors): another lower bound of the distance.  It
+// parts what boxes cannot, the diagonal of one mesh cell from the edges of the
+// next.
+template <typename R, int NA, int NB>
+__device__ __forceinline__ R diagonal_gap(const R (*a)[3], const R (*b)[3]) {
+    R g = R(0);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int l = (k + 1) % 3;
+#pragma unroll
+        for (int sg = 0; sg < 2; ++sg) {
+            auto at = [&](const R* p) { return sg ? p[k] - p[l] : p[k] + p[l]; };
+            R amin = at(a[0]), amax = amin, bmin = at(b[0]), bmax = bmin;
+#pragma unroll
+            for (int j = 1; j < NA; ++j) {
+                const R v = at(a[j]);
+                amin = dmin(amin, v);
+                amax = dmax(amax, v);
+            }
+#pragma unroll
+            for (int j = 1; j < NB; ++j) {
+                const R v = at(b[j]);
+                bmin = dmin(bmin, v);
+                bmax = dmax(bmax, v);
+            }
+            g = dmax(g, dmax(bmin - amax, amin - bmax));
+        }
+    }
+    return g * R(0.70710678);
+}
+
 // True when ccd_pt / ccd_ee below return 1 before computing any distance (no
 // relative motion, or the box-gap exit of their first step): the same
 // arithmetic as their opening lines, on copies.
@@ -206,8 +238,8 @@ __device__ __forceinline__ bool ccd_ee_trivial(const R (*x)[3], const R (*dx)[3]
 // The same exit decided from approximate coordinates: x and dx within eps of
 // the exact ones per component.  The motion bound is taken eps_m larger and the
 // box gap eps_g smaller (eps_m >= 8 eps, eps_g >= 4 eps cover the mean
-// subtraction, the norms and the box corners), so a true result implies the
-// exact test's.
+// subtraction, the norms and the box corners), so a true result implies that the
+// exact test returns 1.
 template <typename R, bool kPT>
 __device__ __forceinline__ bool ccd_trivial_approx(const R (*x)[3], const R (*dx)[3], R eps_g, R eps_m) {
     R mov[3], d[4][3];
@@ -223,7 +255,12 @@ __device__ __forceinline__ bool ccd_trivial_approx(const R (*x)[3], const R (*dx
         maxd = dsqrt(dmax(sqn(d[0]), sqn(d[1]))) + dsqrt(dmax(sqn(d[2]), sqn(d[3])));
     }
     maxd += eps_m;
-    const R gap = dsqrt(kPT ? box_gap2<R, 1, 3>(x, x + 1) : box_gap2<R, 2, 2>(x, x + 2)) - eps_g;
+    R gap = dsqrt(kPT ? box_gap2<R, 1, 3>(x, x + 1) : box_gap2<R, 2, 2>(x, x + 2)) - eps_g;
+    if (gap > R(0) && R(0.81) * gap * gap > R(4) * maxd * maxd) return true;
+    // the diagonals bound the distance, not the boxes' gap: where only they clear
+    // the bound, the test goes on to its first distance d, and returns 1 all the
+    // same since 0.9 d > 2 maxd
+    gap = (kPT ? diagonal_gap<R, 1, 3>(x, x + 1) : diagonal_gap<R, 2, 2>(x, x + 2)) - R(2) * eps_g;
     return gap > R(0) && R(0.81) * gap * gap > R(4) * maxd * maxd;
 }
 
