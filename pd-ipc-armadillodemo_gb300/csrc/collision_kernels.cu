@@ -933,22 +933,19 @@ __device__ __forceinline__ bool contact_maybe(const int* ids, const V4<T>* __res
 // the whole test and, for a pair closer than dhat, its diagonal and right-hand
 // side terms; 1 (mixed mode): only the shared-vertex test and the box filters on
 // the high parts of the mirrors (1: the pair survives them); 2 (mixed mode): the
-// rest, for a pair that survived stage 1.  Returns 1 for an active pair.
+// FP32 distance of a pair that survived stage 1 (1: within 1.1 dhat); 3 (mixed
+// mode): the FP64 distance and the terms of a pair that survived stage 2.  Stages
+// 0 and 3 return 1 for an active pair.
 template <typename T, typename TC, bool kPT, bool kRel, int kStage>
 __device__ __forceinline__ unsigned contact_candidate(const int4 c, const V4<TC>* __restrict__ X,
                                                       const V4<T>* __restrict__ Xh, const V4<T>* __restrict__ Xl,
                                                       const TC* __restrict__ mass, const ContactConsts<TC>& cc,
                                                       T* __restrict__ diag, V4<T>* __restrict__ rhs) {
     const int ids[4] = {c.x, c.y, c.z, c.w};
-    if (kStage != 2 &&
-        (kPT ? (c.x == c.y || c.x == c.z || c.x == c.w) : (c.x == c.z || c.x == c.w || c.y == c.z || c.y == c.w)))
-        return 0u;
+    if (kStage < 2 && shares_vertex<kPT>(c)) return 0u;
     TC p[4][3];
-    if constexpr (kRel) {
-        if (kStage != 2) {  // the filters on the high parts alone
-            if (!contact_maybe<T, kPT>(ids, Xh, (T)cc.dh, (T)cc.dh2)) return 0u;
-            if (kStage == 1) return 1u;
-        }
+    if constexpr (kStage == 1) return contact_maybe<T, kPT>(ids, Xh, (T)cc.dh, (T)cc.dh2);
+    if constexpr (kStage == 2) {
         T q[4][3];
         const V4<T> oh = ld4(Xh, ids[0]), ol = ld4(Xl, ids[0]);
 #pragma unroll
@@ -978,7 +975,9 @@ __device__ __forceinline__ unsigned contact_candidate(const int4 c, const V4<TC>
         T df[3], a_, b_, c_;
         const T d2f = kPT ? geo::vtx_tri<T>(q[0], q[1], q[2], q[3], &a_, &b_, &c_, df)
                           : geo::edge_edge_sq<T>(q[0], q[1], q[2], q[3], &a_, &b_, df);
-        if (!(d2f < (T)(1.21 * cc.dh2))) return 0u;
+        return d2f < (T)(1.21 * cc.dh2);
+    }
+    if constexpr (kRel) {
         const V4<TC> o = ld4(X, ids[0]);  // close pair: FP64 relative coordinates
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -1051,6 +1050,14 @@ __device__ __forceinline__ unsigned contact_candidate(const int4 c, const V4<TC>
     return 1u;
 }
 
+// Stage 3 out of line: its registers stay out of the filters' loop.
+template <typename T, typename TC, bool kPT>
+__device__ __noinline__ unsigned contact_exact(const int4 c, const V4<TC>* __restrict__ X, const TC* __restrict__ mass,
+                                               const ContactConsts<TC>& cc, T* __restrict__ diag,
+                                               V4<T>* __restrict__ rhs) {
+    return contact_candidate<T, TC, kPT, true, 3>(c, X, nullptr, nullptr, mass, cc, diag, rhs);
+}
+
 template <typename T, typename TC, bool kPT, bool kRel>
 __global__ void __launch_bounds__(kBlock, kCandBlocks<T>) k_contact(int64_t n, const int4* __restrict__ cand,
                                                     const V4<TC>* __restrict__ X, const V4<T>* __restrict__ Xh,
@@ -1063,29 +1070,51 @@ __global__ void __launch_bounds__(kBlock, kCandBlocks<T>) k_contact(int64_t n, c
     if constexpr (kRel) {
         // Most candidates fail the cheap stage-1 filter.  Each warp filters 32
         // consecutive candidates at a time and queues the survivors in shared
-        // memory; whenever 32 are queued the whole warp runs the rest of the
-        // test on them, so the distance work runs on full warps.
-        __shared__ int64_t queue[kBlock / 32][64];
+        // memory; whenever 32 are queued the whole warp runs the FP32 distance on
+        // them.  The few pairs that leaves are queued once more, because the FP64
+        // part is a few hundred FP64 instructions, which cost a warp the same for
+        // one lane as for 32; the block's last, partly filled queues are emptied
+        // together.  (Four layers of 256x256 on one another: 1.65 ms a pass with the
+        // FP64 part run as it came, 0.96 this way.)
+        constexpr int kW = kBlock / 32;
+        __shared__ int64_t queue[kW][64], close[kW][64];
+        __shared__ int left[kW];
         const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        int qn = 0;
-        const int64_t step = (int64_t)gridDim.x * (kBlock / 32) * 32;
-        for (int64_t base = ((int64_t)blockIdx.x * (kBlock / 32) + w) * 32; base < n; base += step) {
-            const int64_t t = base + lane;
-            const bool pass = t < n && contact_candidate<T, TC, kPT, kRel, 1>(cand[t], X, Xh, Xl, mass, cc, diag, rhs);
-            const unsigned m = __ballot_sync(0xffffffffu, pass);
-            if (pass) queue[w][qn + __popc(m & ((1u << lane) - 1u))] = t;
-            qn += __popc(m);
+        int qn = 0, cn = 0;
+        // append the lanes' candidates t (in), take 32 from the front once there are
+        auto push = [&](int64_t* q, int& nq, bool in, int64_t t) {
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            if (in) q[nq + __popc(m & ((1u << lane) - 1u))] = t;
+            nq += __popc(m);
             __syncwarp();
-            if (qn >= 32) {
-                const int64_t tq = queue[w][lane];
-                __syncwarp();
-                if (lane < qn - 32) queue[w][lane] = queue[w][lane + 32];
-                __syncwarp();
-                qn -= 32;
-                my += contact_candidate<T, TC, kPT, kRel, 2>(cand[tq], X, Xh, Xl, mass, cc, diag, rhs);
-            }
+        };
+        auto pop = [&](int64_t* q, int& nq) -> int64_t {
+            const int64_t t = q[lane];
+            __syncwarp();
+            if (lane < nq - 32) q[lane] = q[lane + 32];
+            __syncwarp();
+            nq -= 32;
+            return t;
+        };
+        auto exact = [&](int64_t t) { my += contact_exact<T, TC, kPT>(cand[t], X, mass, cc, diag, rhs); };
+        auto near = [&](bool in, int64_t t) {
+            in = in && contact_candidate<T, TC, kPT, kRel, 2>(cand[t], X, Xh, Xl, mass, cc, diag, rhs);
+            push(close[w], cn, in, t);
+            if (cn >= 32) exact(pop(close[w], cn));
+        };
+        const int64_t step = (int64_t)gridDim.x * kW * 32;
+        for (int64_t base = ((int64_t)blockIdx.x * kW + w) * 32; base < n; base += step) {
+            const int64_t t = base + lane;
+            push(queue[w], qn, t < n && contact_candidate<T, TC, kPT, kRel, 1>(cand[t], X, Xh, Xl, mass, cc, diag, rhs),
+                 t);
+            if (qn >= 32) near(true, pop(queue[w], qn));
         }
-        if (lane < qn) my += contact_candidate<T, TC, kPT, kRel, 2>(cand[queue[w][lane]], X, Xh, Xl, mass, cc, diag, rhs);
+        near(lane < qn, lane < qn ? queue[w][lane] : 0);
+        if (lane == 0) left[w] = cn;  // at most 31
+        __syncthreads();
+        int at = threadIdx.x, v = 0;
+        while (v < kW && at >= left[v]) at -= left[v++];
+        if (v < kW) exact(close[v][at]);
     } else {
         for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
             my += contact_candidate<T, TC, kPT, kRel, 0>(cand[t], X, Xh, Xl, mass, cc, diag, rhs);

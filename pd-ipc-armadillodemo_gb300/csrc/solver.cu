@@ -616,7 +616,7 @@ private:
             PD_CK(cudaMemcpyAsync(d_.Pl, saveL, sizeof(V4<T>) * ns, cudaMemcpyDeviceToDevice, s_));
         }
         float collBest = -1.f;
-        const int grids[] = {152 * 16, 152 * 4, 152 * 8, 152 * 32};
+        const int grids[] = {152 * 4, 152 * 8, 152 * 16, 152 * 32};
         const int tblocks[] = {128, 64};
         const int eblocks[] = {256, 128};
         for (int g : grids)
