@@ -34,98 +34,12 @@
 #include <algorithm>
 #include <type_traits>
 
-#include "kernels.cuh"
 #include "svd3.cuh"
-#include "tile.h"
+#include "tile_device.cuh"
 
 namespace pdipc {
 
 namespace {
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ TileWord ld_word(const TileWord* p) {
-    TileWord w;
-    asm volatile(
-        "{\n\t.reg .b128 v;\n\t"
-        "ld.relaxed.gpu.global.b128 v, [%2];\n\t"
-        "mov.b128 {%0, %1}, v;\n\t}"
-        : "=l"(w.lo), "=l"(w.hi)
-        : "l"(p)
-        : "memory");
-    return w;
-}
-__device__ __forceinline__ void st_word(TileWord* p, unsigned long long lo, unsigned long long hi) {
-    asm volatile(
-        "{\n\t.reg .b128 v;\n\t"
-        "mov.b128 v, {%1, %2};\n\t"
-        "st.relaxed.gpu.global.b128 [%0], v;\n\t}" ::"l"(p),
-        "l"(lo), "l"(hi)
-        : "memory");
-}
-__device__ __forceinline__ unsigned long long pack2(unsigned a, unsigned b) {
-    return (unsigned long long)a | ((unsigned long long)b << 32);
-}
-
-
-// ---- the arithmetic, with its rounding spelled out: the results keep the bits
-// of the launches this solve stands in for (one per sweep in the direct form, the
-// band in the correction form), whatever the compiler would contract ----
-__device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
-__device__ __forceinline__ float mul_(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float add_(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ double add_(double a, double b) { return __dadd_rn(a, b); }
-// (1 - w) c + w ((s + b) / D): one weighted-Jacobi update
-template <bool kCorr, typename T>
-__device__ __forceinline__ T jacobi(T om1, T c, T w, T s, T b, T id) {
-    const T t = mul_(add_(s, b), id);
-    return kCorr ? fma_(w, t, mul_(om1, c)) : fma_(om1, c, mul_(w, t));
-}
-template <typename T>
-__device__ __forceinline__ T norm2(T x, T y, T z) {
-    return fma_(z, z, fma_(x, x, mul_(y, y)));
-}
-// Sum2 (common.cuh) with the products it adds fused
-struct Acc {
-    float s = 0.f, c = 0.f;
-    __device__ __forceinline__ void step(float t, float bp, float e) {
-        c = add_(c, add_(add_(s, -add_(t, -bp)), e));
-        s = t;
-    }
-    __device__ __forceinline__ void add(float x) {
-        const float t = add_(s, x), bp = add_(t, -s);
-        step(t, bp, add_(x, -bp));
-    }
-    __device__ __forceinline__ void add(float a, float b) {
-        const float t = fma_(a, b, s), bp = add_(t, -s);
-        step(t, bp, fma_(a, b, -bp));
-    }
-    __device__ __forceinline__ float value() const { return add_(s, c); }
-};
-
-template <typename T>
-struct alignas(2 * sizeof(T)) Pair {
-    T x, y;
-};
-
-// the values of consecutive entries of one row: 16 bytes
-template <typename T>
-struct alignas(16) Group {
-    T v[16 / sizeof(T)];
-};
-
-template <typename S>
-__device__ __forceinline__ V4<S> ldg_state(const V4<S>* p, int i) {  // written by this thread or an earlier kernel
-    return p[i];
-}
 
 // One tet's strain projection (solveVolumetricStrainConstraintKernel,
 // PdIpcGpuFunc.cu:439-599): w R G of its four vertices (three of a cloth
@@ -757,8 +671,7 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
 template <typename T, typename S, bool kCorr>
 const void* tile_kernel(int R, bool tets) {
     if constexpr (sizeof(T) == 8) {
-        if (tets || R != 1) return nullptr;
-        return (const void*)k_pd_tile<T, S, kCorr, false, 1>;
+        return tets || R != 1 ? nullptr : (const void*)k_pd_tile<T, S, kCorr, false, 1>;
     } else {
         if (R != 1 && R != 2) return nullptr;
         if (tets) return R == 1 ? (const void*)k_pd_tile<T, S, kCorr, true, 1> : (const void*)k_pd_tile<T, S, kCorr, true, 2>;

@@ -1933,20 +1933,35 @@ private:
         PD_CK(cudaDeviceGetAttribute(&sm_smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
         PD_CK(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
         if (!coop) return PDIPC_OK;
-        TileLimits lim;
-        lim.value_bytes = (int)sizeof(T);
-        lim.vectors = kCorrection ? 3 : 2;
-        lim.max_warps = kTileMaxWarps;
-        lim.max_rows_per_thread = fp64 ? 1 : 2;
-        lim.min_rows = fp64 ? 32 : 128;
-        lim.co_resident = 2 * nsm;
-        lim.smem = (size_t)(sm_smem / 2 - reserved);
-        if (prm_.pd_group_ctas > 0) lim.group_cap = prm_.pd_group_ctas;
-        build_tile_plan(H, lim, order_block, tile_);
-        if (!tile_.ok) return PDIPC_OK;
-        const int held = tile_residents<T, TC>(tile_.rows_per_thread, H.ntet > 0, tile_.threads, tile_.smem_bytes, nsm);
-        for (const TileGroup& g : tile_.groups)
-            if (g.hi - g.lo + 1 > held) tile_.ok = false;
+        // FP64: a component per thread while an SM has few rows, two tiles per SM of
+        // a row per thread beyond (kTile3Rows), or where that does not fit
+        for (int split = fp64 && H.nsim <= kTile3Rows * nsm ? 1 : 0; split >= 0; --split) {
+            tile3_ = split == 1;
+            TileLimits lim;
+            lim.value_bytes = (int)sizeof(T);
+            lim.vectors = kCorrection ? 3 : 2;
+            lim.max_warps = tile3_ ? kTile3Warps : kTileMaxWarps;
+            lim.max_rows_per_thread = fp64 ? 1 : 2;
+            lim.min_rows = fp64 ? 32 : 128;
+            lim.sms = nsm;
+            lim.co_resident = tile3_ ? nsm : 2 * nsm;
+            lim.slot_rhs = tile3_;
+            lim.smem = (size_t)((tile3_ ? sm_smem : sm_smem / 2) - reserved);
+            if (prm_.pd_group_ctas > 0) lim.group_cap = prm_.pd_group_ctas;
+            build_tile_plan(H, lim, order_block, tile_);
+            if (!tile_.ok) continue;
+            int held = 0;
+            if (tile3_) {
+                tile_.threads *= 3;
+                held = tile3_residents(tile_.threads, tile_.smem_bytes, nsm);
+            } else {
+                held =
+                    tile_residents<T, TC>(tile_.rows_per_thread, H.ntet > 0, tile_.threads, tile_.smem_bytes, nsm);
+            }
+            for (const TileGroup& g : tile_.groups)
+                if (g.hi - g.lo + 1 > held) tile_.ok = false;
+            if (tile_.ok) break;
+        }
         if (!tile_.ok) return PDIPC_OK;
         Dev<T, TC>& d = d_;
         TileArgs<T, TC>& a = targs_;
@@ -2053,8 +2068,12 @@ private:
             // fresh tags and phase counts: every earlier launch's lie below them
             targs_.epoch0 = targs_.flag0 = epoch_;
             epoch_ += tile_phases(c_.lg, c_.cheby);
-            const cudaError_t e = launch_pd_tile<T, TC>(targs_, g.hi - g.lo + 1, tile_.rows_per_thread, d_.ntet > 0,
-                                                        tile_.threads, tile_.smem_bytes, s_);
+            cudaError_t e = cudaErrorInvalidConfiguration;
+            if (!tile3_)
+                e = launch_pd_tile<T, TC>(targs_, g.hi - g.lo + 1, tile_.rows_per_thread, d_.ntet > 0, tile_.threads,
+                                          tile_.smem_bytes, s_);
+            else if constexpr (std::is_same<T, double>::value)
+                e = launch_pd_tile3(targs_, g.hi - g.lo + 1, tile_.threads, tile_.smem_bytes, s_);
             if (e != cudaSuccess) return e;
             if (launched) ++*launched;
         }
@@ -2568,6 +2587,7 @@ private:
     std::vector<PersistGroup> groups_;  // launches of one persistent PD solve
     TilePlan tile_;                     // compact tiles (ok: their tables are on the device)
     bool tile_on_ = false;              // the PD solve runs over them
+    bool tile3_ = false;                // by the FP64 kernel with a component per thread
     TileArgs<T, TC> targs_{};
     // the matrix in SELL-32 over slots (slot_of) for the persistent solve
     int* pSOff_ = nullptr;

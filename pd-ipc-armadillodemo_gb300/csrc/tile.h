@@ -103,4 +103,14 @@ template <typename T, typename S>
 cudaError_t launch_pd_tile(const TileArgs<T, S>& args, int tiles, int rows_per_thread, bool tets, int threads,
                            size_t smem, cudaStream_t s);
 
+// FP64 with three warps per slice, one component each (pd_tile3.cu); no tets.
+// threads: 96 per slice.  Up to kTile3Rows rows per SM: one solve of 10 local-global
+// iterations, a component against a row per thread, 0.99 / 1.66 ms at 64x64 (27
+// rows per SM), 1.56 / 1.77 at 128x128 (108), 2.28 / 2.56 at 180x180 (213); beyond,
+// a tile per SM no longer holds the rows.
+constexpr int kTile3Warps = 9;  // slices of a tile
+constexpr int kTile3Rows = 216;
+int tile3_residents(int threads, size_t smem, int sms);
+cudaError_t launch_pd_tile3(const TileArgs<double, double>& args, int tiles, int threads, size_t smem, cudaStream_t s);
+
 }  // namespace pdipc

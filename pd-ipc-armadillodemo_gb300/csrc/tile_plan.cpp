@@ -147,10 +147,10 @@ bool cut_model(const HostTables& H, const Model& m, int k, int max_slices, std::
 
 }  // namespace
 
-size_t tile_smem_bytes(const TileInfo& t, int pat_stride, int value_bytes, int vectors) {
+size_t tile_smem_bytes(const TileInfo& t, int pat_stride, int value_bytes, int vectors, bool slot_rhs) {
     auto a16 = [](size_t b) { return (b + 15) / 16 * 16; };
     return a16((size_t)t.nent * value_bytes) + a16((size_t)t.npat * pat_stride * sizeof(int16_t)) +
-           vectors * a16(3 * (size_t)t.nloc * value_bytes);
+           vectors * a16(3 * (size_t)t.nloc * value_bytes) + (slot_rhs ? 96 * (size_t)t.nslice * value_bytes : 0);
 }
 
 void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block, TilePlan& P) {
@@ -192,7 +192,7 @@ void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block
         }
         return true;
     };
-    const int sms = lim.co_resident / 2, one_row = lim.max_warps * kLanes;
+    const int sms = lim.sms, one_row = lim.max_warps * kLanes;
     int most_tiles = ns <= one_row / 10 * 9 * sms ? sms : lim.co_resident;
     int target = std::min(max_rows, std::max(lim.min_rows, (ns + most_tiles - 1) / most_tiles));
     if (ns <= one_row && models.size() == 1) target = one_row;  // one tile: no exchange at all
@@ -203,7 +203,7 @@ void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block
             fits = true;
             break;
         }
-        if (target >= (most_tiles == sms ? one_row : max_rows)) {
+        if (target >= (most_tiles < lim.co_resident ? one_row : max_rows)) {
             if (most_tiles == lim.co_resident) break;
             most_tiles = lim.co_resident;
             target = std::max(lim.min_rows, (ns + most_tiles - 1) / most_tiles);
@@ -430,8 +430,8 @@ void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block
             T.ntet = (int)tetsOf[t].size();
             P.tet.insert(P.tet.end(), tetsOf[t].begin(), tetsOf[t].end());
         }
-        const size_t sm = tile_smem_bytes(T, P.pat_stride, lim.value_bytes, 2);
-        if (lim.vectors > 2) most3 = std::max(most3, tile_smem_bytes(T, P.pat_stride, lim.value_bytes, lim.vectors));
+        const size_t sm = tile_smem_bytes(T, P.pat_stride, lim.value_bytes, 2, lim.slot_rhs);
+        if (lim.vectors > 2) most3 = std::max(most3, tile_smem_bytes(T, P.pat_stride, lim.value_bytes, lim.vectors, lim.slot_rhs));
         if (sm > lim.smem) return;
         P.smem_bytes = std::max(P.smem_bytes, sm);
         P.tiles.push_back(T);

@@ -51,7 +51,9 @@ struct TileLimits {
     int max_warps = 14;       // row warps a CTA can have
     int max_rows_per_thread = 2;
     int min_rows = 128;       // rows of a tile at least, where the mesh has them
-    int co_resident = 304;    // CTAs one cooperative launch holds: two per SM
+    int sms = 152;
+    int co_resident = 304;    // CTAs one cooperative launch holds: one or two per SM
+    bool slot_rhs = false;    // a tile also holds three values per slot (pd_tile3.cu)
     int group_cap = 1 << 30;  // pdipc_params.pd_group_ctas
     size_t smem = 113 * 1024; // per CTA
 };
@@ -80,7 +82,7 @@ struct TilePlan {
 
 // Shared memory of one tile: values, patterns and the vectors of its local
 // vertices.
-size_t tile_smem_bytes(const TileInfo& t, int pat_stride, int value_bytes, int vectors);
+size_t tile_smem_bytes(const TileInfo& t, int pat_stride, int value_bytes, int vectors, bool slot_rhs);
 
 // order_block > 0: a row sums its entries in the order [columns of its own block
 // of order_block rows][lower columns][higher columns], each part ascending;
