@@ -10,7 +10,9 @@
 //   * an exchanged vertex is one 16-byte word that carries the phase's tag, so
 //     a reader polls the data itself: one L2 write and one L2 read per phase
 //     instead of data, a release of a flag, polls of the flag and a copy;
-//   * two CTAs share an SM, so one tile sums while the other waits;
+//   * few tiles form one thread-block cluster (kCl) and write their boundary rows
+//     straight into the readers' shared memory;
+//   * otherwise two CTAs share an SM, so one tile sums while the other waits;
 //   * matrix values, column offsets and both copies of the iterate stay in
 //     shared memory for the launch; the local step's neighbour differences come
 //     from the same memory (positions, or their high and low halves, occupy the
@@ -18,15 +20,16 @@
 //     and the Chebyshev history in registers.
 //
 // Measured (GB300, one solve, before: the row-block launches of pd_persistent.cuh
-// or, FP64, one launch per sweep): mixed 16x16 0.97 -> 0.35 ms, 64x64 0.96 -> 0.49,
-// 181x181 1.31 -> 0.69, 512x512 4.35 -> 3.42, four 256x256 10.6 -> 3.4; FP32 96x96
-// 1.34 -> 0.47; FP64 64x64 2.88 -> 1.62, 257x257 9.2 -> 8.0.
+// or, FP64, one launch per sweep): mixed 16x16 0.97 -> 0.34 ms, 64x64 0.96 -> 0.42,
+// 181x181 1.31 -> 0.67, 512x512 4.35 -> 3.26, four 256x256 10.6 -> 3.5; FP32 96x96
+// 1.34 -> 0.45; FP64 257x257 9.2 -> 8.0 (smaller FP64 meshes: pd_tile3.cu).
 //
 // Double buffering of the exchange: in phase p a tile writes its boundary rows
 // to parity p & 1 and then reads its halo there.  It overwrites that parity in
 // phase p + 2, after it has read every neighbour's phase p + 1, which a
 // neighbour publishes only after a CTA barrier that follows its own reads of
-// phase p (the plan makes reading mutual).
+// phase p (the plan makes reading mutual).  In a cluster no tile starts a phase
+// before all have ended the one before, so two copies of the iterate do.
 //
 // Every wait is clock-bounded: past the limit it raises kErrBarrier, the tile
 // leaves together at its next barrier, and the others' waits end on the error
@@ -87,7 +90,7 @@ __device__ __noinline__ void tile_tet(int e, const int4* __restrict__ Tets, cons
         __stcg((float4*)Out + 4 * (size_t)e + c, make_float4(out[c][0], out[c][1], out[c][2], 0.f));
 }
 
-template <typename T, typename S, bool kCorr, bool kTets, int R>
+template <typename T, typename S, bool kCorr, bool kTets, int R, bool kCl>
 __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_constant__ TileArgs<T, S> a) {
     constexpr int kW = kTileWords<T, S>;
     constexpr int kG = kTileGroup<T>;
@@ -102,13 +105,16 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
     // ---- shared memory: values, offset patterns, two vectors of the local
     // vertices as (x, y) pairs and z ----
     auto a16 = [](size_t b) { return (b + 15) / 16 * 16; };
-    T* sval = reinterpret_cast<T*>(smem);
-    int16_t* spat = reinterpret_cast<int16_t*>(smem + a16((size_t)ti.nent * sizeof(T)));
+    // (in a cluster the vectors come first and are laid out alike in every CTA)
+    const int nl = kCl ? a.nlocMax : ti.nloc;
+    const int vecBytes = (int)a16(3 * (size_t)nl * sizeof(T));
+    unsigned char* tab = smem + (kCl ? (kCorr ? 3 : 2) * (size_t)vecBytes : 0);
+    T* sval = reinterpret_cast<T*>(tab);
+    int16_t* spat = reinterpret_cast<int16_t*>(tab + a16((size_t)ti.nent * sizeof(T)));
     unsigned char* vec0 =
-        smem + a16((size_t)ti.nent * sizeof(T)) + a16((size_t)ti.npat * a.patStride * sizeof(int16_t));
-    const int vecBytes = (int)a16(3 * (size_t)ti.nloc * sizeof(T));
+        kCl ? smem : tab + a16((size_t)ti.nent * sizeof(T)) + a16((size_t)ti.npat * a.patStride * sizeof(int16_t));
     auto XY = [&](int b) { return reinterpret_cast<Pair<T>*>(vec0 + b * vecBytes); };
-    auto Z = [&](int b) { return reinterpret_cast<T*>(XY(b) + ti.nloc); };
+    auto Z = [&](int b) { return reinterpret_cast<T*>(XY(b) + nl); };
     for (int q = threadIdx.x; q < ti.nent; q += blockDim.x) sval[q] = __ldg(a.val + ti.ent0 + q);
     for (int q = threadIdx.x; q < ti.npat * a.patStride; q += blockDim.x)
         spat[q] = __ldg(a.pat + (size_t)ti.pat0 * a.patStride + q);
@@ -170,6 +176,33 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
             st_word(words(2) + g, (unsigned long long)__double_as_longlong(z), tag);
         }
     };
+    // cluster: the row's readers, whose shared memory this thread writes
+    int4 to = make_int4(-1, -1, -1, -1);
+    if constexpr (kCl)
+        if (live(0)) to = __ldg(a.push + slot(0));
+    auto push = [&](int b, int d, T x, T y, T z) {
+        if (d < 0) return;
+        const int q = d & 0xffff;
+        st_remote(remote_addr(XY(b) + q, (unsigned)d >> 16), x, y);
+        st_remote(remote_addr(Z(b) + q, (unsigned)d >> 16), z);
+    };
+    // row r's new vector (place b; word w of the phase) to whoever reads it
+    auto send = [&](int w, int b, int r, T x, T y, T z) {
+        if (!pub(r)) return;
+        if constexpr (kCl) {
+            push(b, to.x, x, y, z);
+            push(b, to.y, x, y, z);
+            push(b, to.z, x, y, z);
+            push(b, to.w, x, y, z);
+        } else {
+            publish(w, row(r), x, y, z);
+        }
+    };
+    // every CTA that might write here, or be written to, is at the same point
+    auto sync_all = [&]() {
+        if constexpr (kCl) cluster_sync();
+        else __syncthreads();
+    };
     // wait for the word at p to carry the current tag
     auto wait_word = [&](const TileWord* p, TileWord& w) -> bool {
         w = ld_word(p);
@@ -217,6 +250,10 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
     };
     // end of a phase: the halo is in, every own value is written; false: the launch ends
     auto arrive = [&](int b, int b2 = -1) -> bool {
+        if constexpr (kCl) {
+            cluster_sync();
+            return true;
+        }
         if (ti.nhalo == 0) {
             __syncthreads();
             return true;
@@ -323,8 +360,9 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
         const TileHalo q = a.halo[ti.halo0 + h];
         load_pos(q.row, q.pos);
     }
-    __syncthreads();
+    sync_all();  // also: every CTA of a cluster runs before its shared memory is written
 
+    const bool third = kCl || a.third;
     int cur = 0;  // the vector that holds the positions (direct form) at the start of an iteration
     for (int lg = 0; lg < a.lg; ++lg) {
         if constexpr (kTets) {
@@ -423,7 +461,7 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
                     r1.add(rc, d1);
                     r2.add(rc, d2);
                 }
-                if (!a.third) matrix_part(r, r0, r1, r2);
+                if (!third) matrix_part(r, r0, r1, r2);
                 acc[r][0] = r0;
                 acc[r][1] = r1;
                 acc[r][2] = r2;
@@ -471,13 +509,13 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
         // ---- the curvature vectors go into the third vector, or where the
         // positions' high halves were (correction form), or into the free vector
         // (direct form) ----
-        const int qb = kCorr ? (a.third ? 2 : 0) : cur ^ 1;
-        if (kCorr && !a.third) __syncthreads();
+        const int qb = kCorr ? (third ? 2 : 0) : cur ^ 1;
+        if (kCorr && !third) sync_all();
         ++tag;
 #pragma unroll
         for (int r = 0; r < R; ++r)
             if (live(r)) {
-                if (pub(r)) publish(0, row(r), aq[r][0], aq[r][1], aq[r][2]);
+                send(0, qb, r, aq[r][0], aq[r][1], aq[r][2]);
                 put(qb, lp(r), aq[r][0], aq[r][1], aq[r][2]);
             }
         if (!arrive(qb)) return;
@@ -510,7 +548,7 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
                         r1.add(t.y);
                         r2.add(t.z);
                     }
-                if (a.third) matrix_part(r, r0, r1, r2);
+                if (third) matrix_part(r, r0, r1, r2);
                 rh[r][0] = r0.value();
                 rh[r][1] = r1.value();
                 rh[r][2] = r2.value();
@@ -566,14 +604,17 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
                 y[r][0] = jacobi<kCorr>(om1, c0, w, s0, rh[r][0], id[r]);
                 y[r][1] = jacobi<kCorr>(om1, c1, w, s1, rh[r][1], id[r]);
                 y[r][2] = jacobi<kCorr>(om1, c2, w, s2, rh[r][2], id[r]);
-                if (pub(r)) publish(0, row(r), y[r][0], y[r][1], y[r][2]);
+                if (!kCl && pub(r)) publish(0, row(r), y[r][0], y[r][1], y[r][2]);
             }
             // the curvature vectors (direct form), or the positions, have been read
-            if (!kCorr || a.third) __syncthreads();
+            if (!kCorr || third) sync_all();
             cur = kCorr ? 1 : cur ^ 1;
 #pragma unroll
             for (int r = 0; r < R; ++r)
-                if (live(r)) put(cur, lp(r), y[r][0], y[r][1], y[r][2]);
+                if (live(r)) {
+                    if (kCl) send(0, cur, r, y[r][0], y[r][1], y[r][2]);
+                    put(cur, lp(r), y[r][0], y[r][1], y[r][2]);
+                }
         }
         if (!arrive(cur)) return;
         for (int it = 0; it < a.cheby; ++it) {
@@ -606,7 +647,7 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
                 }
                 if (!live(r)) continue;
                 if (!(kCorr && last)) {
-                    if (pub(r)) publish(0, row(r), n[0], n[1], n[2]);
+                    send(0, cur ^ 1, r, n[0], n[1], n[2]);
                     put(cur ^ 1, lp(r), n[0], n[1], n[2]);
                 }
                 if (!kCorr && last && (kTets || lg == a.lg - 1)) a.P[row(r)] = V4<S>{n[0], n[1], n[2], S(0)};
@@ -626,7 +667,7 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
                 const T y1 = jacobi<kCorr>(om1, c1, w, s1, rh[r][1], id[r]);
                 const T y2 = jacobi<kCorr>(om1, c2, w, s2, rh[r][2], id[r]);
                 if (!live(r)) continue;
-                if (pub(r)) publish(0, row(r), y0, y1, y2);
+                send(0, cur ^ 1, r, y0, y1, y2);
                 put(cur ^ 1, lp(r), y0, y1, y2);
             }
             cur ^= 1;
@@ -634,7 +675,7 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
         }
         // ---- the new positions ----
         if constexpr (kCorr) {
-            __syncthreads();  // both vectors have been read
+            sync_all();  // both vectors have been read
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 if (!live(r)) continue;
@@ -649,10 +690,8 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
                     a.Ph[row(r)] = V4<T>{hx, hy, hz, T(0)};
                     a.Pl[row(r)] = V4<T>{lx, ly, lz, T(0)};
                 }
-                if (pub(r)) {
-                    publish(0, row(r), hx, hy, hz);
-                    publish(1, row(r), lx, ly, lz);
-                }
+                send(0, 0, r, hx, hy, hz);
+                send(1, 1, r, lx, ly, lz);
                 put(0, lp(r), hx, hy, hz);
                 put(1, lp(r), lx, ly, lz);
             }
@@ -666,16 +705,17 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
         if constexpr (kTets)
             if (!global_sync()) return;
     }
+    if constexpr (kCl) cluster_sync();  // nobody leaves while another may write to its shared memory
 }
 
 template <typename T, typename S, bool kCorr>
 const void* tile_kernel(int R, bool tets) {
     if constexpr (sizeof(T) == 8) {
-        return tets || R != 1 ? nullptr : (const void*)k_pd_tile<T, S, kCorr, false, 1>;
+        return tets || R != 1 ? nullptr : (const void*)k_pd_tile<T, S, kCorr, false, 1, false>;
     } else {
         if (R != 1 && R != 2) return nullptr;
-        if (tets) return R == 1 ? (const void*)k_pd_tile<T, S, kCorr, true, 1> : (const void*)k_pd_tile<T, S, kCorr, true, 2>;
-        return R == 1 ? (const void*)k_pd_tile<T, S, kCorr, false, 1> : (const void*)k_pd_tile<T, S, kCorr, false, 2>;
+        if (tets) return R == 1 ? (const void*)k_pd_tile<T, S, kCorr, true, 1, false> : (const void*)k_pd_tile<T, S, kCorr, true, 2, false>;
+        return R == 1 ? (const void*)k_pd_tile<T, S, kCorr, false, 1, false> : (const void*)k_pd_tile<T, S, kCorr, false, 2, false>;
     }
 }
 
@@ -705,8 +745,70 @@ cudaError_t launch_pd_tile(const TileArgs<T, S>& args, int tiles, int R, bool te
     return cudaLaunchCooperativeKernel(f, dim3(tiles), dim3(threads), params, smem, s);
 }
 
+namespace {
+
+template <typename T, typename S>
+const void* cluster_kernel() {
+    return (const void*)k_pd_tile<T, S, !std::is_same<T, S>::value, false, 1, true>;
+}
+cudaLaunchConfig_t cluster_config(int tiles, int threads, size_t smem, cudaStream_t s, cudaLaunchAttribute* at) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(tiles);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = tiles;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    return c;
+}
+
+}  // namespace
+
+template <typename T, typename S>
+bool tile_cluster_fits(int tiles, int threads, size_t smem) {
+    if constexpr (sizeof(T) == 8) {
+        return false;
+    } else {
+        const void* f = cluster_kernel<T, S>();
+        if (threads > kTileMaxWarps * 32 || tiles > kTileCluster) return false;
+        cudaFuncAttributes fa;
+        if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) return false;
+        if ((size_t)fa.maxDynamicSharedSizeBytes < smem &&
+            cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+            return false;
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return false;
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t c = cluster_config(tiles, threads, smem, nullptr, &at);
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, f, &c) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        return n > 0;
+    }
+}
+
+template <typename T, typename S>
+cudaError_t launch_pd_tile_cluster(const TileArgs<T, S>& args, int tiles, int threads, size_t smem,
+                                   cudaStream_t s) {
+    if constexpr (sizeof(T) == 8) {
+        return cudaErrorInvalidConfiguration;
+    } else {
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t c = cluster_config(tiles, threads, smem, s, &at);
+        void* params[] = {(void*)&args};
+        return cudaLaunchKernelExC(&c, cluster_kernel<T, S>(), params);
+    }
+}
+
 #define PDIPC_INST_TILE(T, S)                                                                     \
     template int tile_residents<T, S>(int, bool, int, size_t, int);                               \
+    template bool tile_cluster_fits<T, S>(int, int, size_t);                                      \
+    template cudaError_t launch_pd_tile_cluster<T, S>(const TileArgs<T, S>&, int, int, size_t,    \
+                                                      cudaStream_t);                              \
     template cudaError_t launch_pd_tile<T, S>(const TileArgs<T, S>&, int, int, bool, int, size_t, \
                                               cudaStream_t);
 PDIPC_INST_TILE(float, float)

@@ -1948,8 +1948,21 @@ private:
             lim.slot_rhs = tile3_;
             lim.smem = (size_t)((tile3_ ? sm_smem : sm_smem / 2) - reserved);
             if (prm_.pd_group_ctas > 0) lim.group_cap = prm_.pd_group_ctas;
+            // all tiles in one launch, none of which leaves early: the barriers of a
+            // cluster wait for all
+            if (!fp64 && H.ntet == 0 && !prm_.instance_stop && lim.group_cap >= kTileCluster) {
+                lim.cluster = kTileCluster;
+                lim.cluster_min = kTileClusterMin;
+                lim.cluster_rows = kTileClusterRows;
+            }
             build_tile_plan(H, lim, order_block, tile_);
+            if (tile_.ok && tile_.cluster &&
+                !tile_cluster_fits<T, TC>((int)tile_.tiles.size(), tile_.threads, tile_.smem_bytes)) {
+                lim.cluster = 0;
+                build_tile_plan(H, lim, order_block, tile_);
+            }
             if (!tile_.ok) continue;
+            if (tile_.cluster) break;
             int held = 0;
             if (tile3_) {
                 tile_.threads *= 3;
@@ -1985,6 +1998,13 @@ private:
         PD_CK(up(halo, tile_.halo));
         PD_CK(up(nbr, tile_.nbr));
         PD_CK(up(tet, tile_.tet));
+        std::vector<int4> push(tile_.push.size() / 4);
+        for (size_t q = 0; q < push.size(); ++q)
+            push[q] = make_int4(tile_.push[4 * q], tile_.push[4 * q + 1], tile_.push[4 * q + 2], tile_.push[4 * q + 3]);
+        int4* pushd = nullptr;
+        PD_CK(up(pushd, push));
+        a.push = pushd;
+        a.nlocMax = tile_.nloc_max;
         PD_CK(zeros(a.ex, 2 * (size_t)kTileWords<T, TC> * H.nsim));
         PD_CK(zeros(a.flags, tile_.tiles.size()));
         PD_CK(cudaStreamSynchronize(s_));
@@ -2069,7 +2089,9 @@ private:
             targs_.epoch0 = targs_.flag0 = epoch_;
             epoch_ += tile_phases(c_.lg, c_.cheby);
             cudaError_t e = cudaErrorInvalidConfiguration;
-            if (!tile3_)
+            if (tile_.cluster)
+                e = launch_pd_tile_cluster<T, TC>(targs_, g.hi - g.lo + 1, tile_.threads, tile_.smem_bytes, s_);
+            else if (!tile3_)
                 e = launch_pd_tile<T, TC>(targs_, g.hi - g.lo + 1, tile_.rows_per_thread, d_.ntet > 0, tile_.threads,
                                           tile_.smem_bytes, s_);
             else if constexpr (std::is_same<T, double>::value)

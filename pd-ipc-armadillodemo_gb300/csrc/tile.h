@@ -83,6 +83,8 @@ struct TileArgs {
     const unsigned* instStop;  // per-instance stopping: tiles of a stopped model return at entry
     V4<T>* tape;               // direct form: the positions at the start of every local-global iteration, or null
     int lo;                    // first tile of this launch
+    const int4* push;          // cluster: the readers of every slot's row (TilePlan::push)
+    int nlocMax;               // cluster: places of each vector
     int third;                 // correction form: the tiles hold a third vector
 };
 
@@ -102,6 +104,22 @@ int tile_residents(int rows_per_thread, bool tets, int threads, size_t smem, int
 template <typename T, typename S>
 cudaError_t launch_pd_tile(const TileArgs<T, S>& args, int tiles, int rows_per_thread, bool tets, int threads,
                            size_t smem, cudaStream_t s);
+// The tiles as one thread-block cluster (FP32 arithmetic, a row per thread): a
+// thread writes its new vector into the shared memory of the tiles that read it,
+// and the cluster's barrier ends the sweep, in place of words in global memory that
+// the readers poll.  One solve of 10 x (local step + 30 sweeps), mixed, words ->
+// cluster: 20x20 0.50 -> 0.37 ms, 32x32 0.46 -> 0.36, 48x48 0.49 -> 0.44,
+// 64x64 0.50 -> 0.42; FP32 0.42 -> 0.33, 0.39 -> 0.33, 0.45 -> 0.38, 0.46 -> 0.37.
+// Up to kTileClusterMin rows one tile alone is as fast (16x16 0.340 ms, 0.344 in a
+// cluster; FP32 0.285, 0.307); beyond kTileClusterRows rows per CTA the sums of so
+// few SMs cost more than the words of many (66x66: 0.550, 0.552 in a cluster).  With
+// tets their projection wants the SMs (block of 8^3 cubes: 0.74, 0.81 in a cluster).
+constexpr int kTileCluster = 16, kTileClusterMin = 320, kTileClusterRows = 272;
+// Whether the device holds such a cluster, and the launch.
+template <typename T, typename S>
+bool tile_cluster_fits(int tiles, int threads, size_t smem);
+template <typename T, typename S>
+cudaError_t launch_pd_tile_cluster(const TileArgs<T, S>& args, int tiles, int threads, size_t smem, cudaStream_t s);
 
 // FP64 with three warps per slice, one component each (pd_tile3.cu); no tets.
 // threads: 96 per slice.  Up to kTile3Rows rows per SM: one solve of 10 local-global

@@ -36,6 +36,26 @@ __device__ __forceinline__ void st_word(TileWord* p, unsigned long long lo, unsi
         "l"(lo), "l"(hi)
         : "memory");
 }
+// ---- thread-block cluster: the same place in another CTA's shared memory, and the
+// barrier of all its threads (release, acquire: it orders the remote writes) ----
+__device__ __forceinline__ unsigned remote_addr(const void* p, unsigned rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(r)
+                 : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_remote(unsigned addr, float x, float y) {
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(x), "f"(y) : "memory");
+}
+__device__ __forceinline__ void st_remote(unsigned addr, float x) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(x) : "memory");
+}
+__device__ __forceinline__ void st_remote(unsigned, double, double) {}
+__device__ __forceinline__ void st_remote(unsigned, double) {}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
 __device__ __forceinline__ unsigned long long pack2(unsigned a, unsigned b) {
     return (unsigned long long)a | ((unsigned long long)b << 32);
 }

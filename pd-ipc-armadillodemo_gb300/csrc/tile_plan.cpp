@@ -197,7 +197,16 @@ void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block
     int target = std::min(max_rows, std::max(lim.min_rows, (ns + most_tiles - 1) / most_tiles));
     if (ns <= one_row && models.size() == 1) target = one_row;  // one tile: no exchange at all
     bool fits = false;
-    for (;;) {
+    // few rows: the tiles of one cluster, a row per thread
+    if (lim.cluster > 0 && ns > lim.cluster_min && ns <= lim.cluster * lim.cluster_rows) {
+        for (int t = (ns + lim.cluster - 1) / lim.cluster; !P.cluster && t <= lim.cluster_rows; t += std::max(4, t / 16)) {
+            if (!cut_all(t)) return;
+            P.cluster = (int)own.size() <= lim.cluster;
+            for (const auto& o : own) P.cluster = P.cluster && (int)o.size() <= one_row;
+        }
+        fits = P.cluster;
+    }
+    while (!fits) {
         if (!cut_all(target)) return;
         if ((int)own.size() <= most_tiles) {
             fits = true;
@@ -435,6 +444,38 @@ void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block
         if (sm > lim.smem) return;
         P.smem_bytes = std::max(P.smem_bytes, sm);
         P.tiles.push_back(T);
+    }
+    for (const TileInfo& T : P.tiles) P.nloc_max = std::max(P.nloc_max, T.nloc);
+    if (P.cluster) {
+        // whom each row goes to; the vectors are laid out alike in every tile
+        std::unordered_map<int, int> slotOf;
+        for (size_t q = 0; q < P.slots.size(); ++q)
+            if (P.slots[q].row >= 0) slotOf[P.slots[q].row] = (int)q;
+        P.push.assign(4 * P.slots.size(), -1);
+        for (int t = 0; t < nt && P.cluster; ++t)
+            for (int h = 0; h < P.tiles[t].nhalo; ++h) {
+                const TileHalo& q = P.halo[P.tiles[t].halo0 + h];
+                int* d = &P.push[4 * (size_t)slotOf[q.row]];
+                int k = 0;
+                while (k < 4 && d[k] >= 0) ++k;
+                if (k == 4) P.cluster = false;  // a fifth reader
+                else d[k] = t << 16 | q.pos;
+            }
+        size_t sm = 0;
+        for (const TileInfo& T : P.tiles) {
+            TileInfo u = T;
+            u.nloc = P.nloc_max;
+            sm = std::max(sm, tile_smem_bytes(u, P.pat_stride, lim.value_bytes, lim.vectors, lim.slot_rhs));
+        }
+        if (sm > lim.smem || most > lim.max_warps) P.cluster = false;
+        if (!P.cluster) {  // larger tiles have fewer readers
+            TileLimits l = lim;
+            l.cluster = lim.cluster >= 8 ? lim.cluster / 2 : 0;
+            build_tile_plan(H, l, order_block, P);
+            return;
+        }
+        P.smem_bytes = sm;
+        most3 = sm;
     }
     P.rows_per_thread = (most + lim.max_warps - 1) / lim.max_warps;
     P.threads = (most + P.rows_per_thread - 1) / P.rows_per_thread * kLanes;

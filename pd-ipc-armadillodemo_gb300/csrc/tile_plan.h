@@ -53,6 +53,9 @@ struct TileLimits {
     int min_rows = 128;       // rows of a tile at least, where the mesh has them
     int sms = 152;
     int co_resident = 304;    // CTAs one cooperative launch holds: one or two per SM
+    int cluster = 0;          // CTAs of a cluster at most (0: none),
+    int cluster_min = 0;      // where there are more rows than this,
+    int cluster_rows = 0;     // and no more than this many per CTA
     bool slot_rhs = false;    // a tile also holds three values per slot (pd_tile3.cu)
     int group_cap = 1 << 30;  // pdipc_params.pd_group_ctas
     size_t smem = 113 * 1024; // per CTA
@@ -65,6 +68,12 @@ struct TilePlan {
     int pat_stride = 0;  // elements of one pattern, a multiple of 8 (16 bytes)
     size_t smem_bytes = 0;
     int vectors = 2;
+    // the tiles form one thread-block cluster: vectors at the start of shared
+    // memory, nloc_max places each, and up to four readers of every slot's row,
+    // tile << 16 | place there (-1: none)
+    bool cluster = false;
+    int nloc_max = 0;
+    std::vector<int> push;
     std::vector<TileInfo> tiles;
     std::vector<TileSlot> slots;
     std::vector<TileSlice> slices;

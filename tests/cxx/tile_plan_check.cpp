@@ -71,7 +71,9 @@ static bool check(const HostTables& H, const TileLimits& L, int block) {
     for (size_t t = 0; t < P.tiles.size(); ++t) {
         const TileInfo& T = P.tiles[t];
         if (T.nslice > P.rows_per_thread * P.threads / 32) FAIL("tile %zu: too many slices", t);
-        smem = std::max(smem, tile_smem_bytes(T, P.pat_stride, L.value_bytes, P.vectors, L.slot_rhs));
+        TileInfo room = T;  // a cluster's vectors are laid out alike
+        if (P.cluster) room.nloc = P.nloc_max;
+        smem = std::max(smem, tile_smem_bytes(room, P.pat_stride, L.value_bytes, P.vectors, L.slot_rhs));
         std::vector<int> at(T.nloc, -1);
         auto place = [&](int pos, int row) {
             if (pos < 0 || pos >= T.nloc || at[pos] != -1) return false;
@@ -137,6 +139,18 @@ static bool check(const HostTables& H, const TileLimits& L, int block) {
             }
         }
     }
+    if (P.cluster) {  // every halo place is written once, by its row's owner, and nothing else is
+        if ((int)P.tiles.size() > L.cluster || P.rows_per_thread != 1 || P.groups.size() != 1) FAIL("cluster shape");
+        std::set<std::pair<int, int>> want, got;
+        for (size_t t = 0; t < P.tiles.size(); ++t)
+            for (int h = 0; h < P.tiles[t].nhalo; ++h) {
+                const TileHalo& q = P.halo[P.tiles[t].halo0 + h];
+                want.insert({(int)t << 16 | q.pos, q.row});
+            }
+        for (size_t q = 0; q < P.push.size(); ++q)
+            if (P.push[q] >= 0 && !got.insert({P.push[q], P.slots[q / 4].row}).second) FAIL("written twice");
+        if (P.push.size() != 4 * P.slots.size() || want != got) FAIL("cluster readers");
+    }
     if (smem != P.smem_bytes || smem > L.smem) FAIL("shared memory");
     int next = 0;
     for (const TileGroup& g : P.groups) {
@@ -149,7 +163,7 @@ static bool check(const HostTables& H, const TileLimits& L, int block) {
 }
 
 int main() {
-    auto run = [](std::vector<ModelInput> ms, int block, int value_bytes, int cap) {
+    auto run = [](std::vector<ModelInput> ms, int block, int value_bytes, int cap, int cluster = 0) {
         HostTables H;
         const std::string e = build_host_tables(ms, -9.8, H);
         if (!e.empty()) {
@@ -168,6 +182,9 @@ int main() {
             L.smem = 226 * 1024;
         }
         if (cap) L.group_cap = cap;
+        L.cluster = cluster;
+        L.cluster_min = 320;
+        L.cluster_rows = 272;
         return check(H, L, block);
     };
     bool ok = true;
@@ -179,6 +196,9 @@ int main() {
     ok = ok && run({grid(20, 20, 0, false), grid(48, 40, 1, false), grid(33, 33, 2, false)}, 64, 4, 16);
     ok = ok && run({grid(170, 170, 0, false)}, 0, 8, 0) && run({grid(64, 64, 0, false)}, 0, 8, 0);
     ok = ok && run({grid(400, 340, 0, false)}, 0, 4, 0);  // two CTAs per SM, two rows per thread
+    for (int n : {18, 25, 33, 49, 65, 66}) ok = ok && run({grid(n, n, 0, false)}, 64, 4, 0, 16);
+    ok = ok && run({grid(40, 31, 0, true)}, 64, 4, 0, 16) && run({grid(300, 3, 0, false)}, 0, 4, 0, 16);
+    ok = ok && run({grid(20, 20, 0, false), grid(18, 40, 1, false), grid(7, 9, 2, true)}, 64, 4, 0, 16);
     if (ok) printf("ok\n");
     return ok ? 0 : 1;
 }

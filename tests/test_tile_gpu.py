@@ -24,20 +24,33 @@ def _solve(sc, prec, **kw):
     return x, sim.tuning()
 
 
-# 21^2 = 441 rows: one FP32 tile; 22^2: several; 65: odd edges; 224: past a component
+# 18, 24, 65: the smallest cluster of tiles, one of eight, the largest; 66: past it; 224: past a component
 # per thread in FP64; 300: two tiles per SM; 430: with two rows per thread
-@pytest.mark.parametrize("prec,n", [(p, n) for p in ("fp32", "fp64") for n in (2, 21, 22, 65, 224)] +
-                         [("fp64", 300), ("fp32", 430), ("mixed", 21), ("mixed", 22), ("mixed", 430)])
+@pytest.mark.parametrize("prec,n", [(p, n) for p in ("fp32", "fp64") for n in (2, 18, 24, 65, 66, 224)] +
+                         [("fp64", 300), ("fp32", 430), ("mixed", 18), ("mixed", 24), ("mixed", 65), ("mixed", 430)])
 def test_tiled_solve_against_one_launch_per_sweep(prec, n, built_lib):
     sc = scenes.cloth_drop(n, 1, with_sphere=False, lg=3)
     a, t = _solve(sc, prec)
     b, u = _solve(sc, prec, persistent=0)
     assert t["pd_rows_per_thread"] == (2 if n == 430 else 1) and u["pd_rows_per_thread"] == 0
-    assert t["pd_ctas"] == 1 if n == 2 else t["pd_ctas"] > 1 if n > 21 else t["pd_ctas"] < 20
+    assert t["pd_ctas"] == 1 if n == 2 else t["pd_ctas"] > 1
+    if prec != "fp64":
+        assert (t["pd_ctas"] <= 16) == (n <= 65)
     if prec == "mixed":
         assert np.abs(a - b).max() < 1e-6
     else:
         assert np.array_equal(a, b)
+
+
+# three cloths in one cluster, against tiles that exchange words (a model may stop by
+# itself: no cluster)
+@pytest.mark.parametrize("prec", ["fp32", "mixed"])
+def test_cluster_of_several_models(prec, built_lib):
+    sc = scenes.batched(3, 18, 30, seed=4)
+    a, t = _solve(sc, prec)
+    b, _ = _solve(sc, prec, instance_stop=1)
+    assert t["pd_ctas"] <= 16
+    assert np.array_equal(a, b)
 
 
 def test_tiled_groups_and_stopped_models_give_the_bits_of_one_launch(built_lib):
