@@ -12,6 +12,7 @@
 //     instead of data, a release of a flag, polls of the flag and a copy;
 //   * few tiles form one thread-block cluster (kCl) and write their boundary rows
 //     straight into the readers' shared memory;
+//   * many rows are summed in pairs with their values in tensor memory (kPairs);
 //   * otherwise two CTAs share an SM, so one tile sums while the other waits;
 //   * matrix values, column offsets and both copies of the iterate stay in
 //     shared memory for the launch; the local step's neighbour differences come
@@ -21,7 +22,7 @@
 //
 // Measured (GB300, one solve, before: the row-block launches of pd_persistent.cuh
 // or, FP64, one launch per sweep): mixed 16x16 0.97 -> 0.34 ms, 64x64 0.96 -> 0.42,
-// 181x181 1.31 -> 0.67, 512x512 4.35 -> 3.26, four 256x256 10.6 -> 3.5; FP32 96x96
+// 181x181 1.31 -> 0.67, 512x512 4.35 -> 2.90, four 256x256 10.6 -> 2.93; FP32 96x96
 // 1.34 -> 0.45; FP64 257x257 9.2 -> 8.0 (smaller FP64 meshes: pd_tile3.cu).
 //
 // Double buffering of the exchange: in phase p a tile writes its boundary rows
@@ -90,17 +91,53 @@ __device__ __noinline__ void tile_tet(int e, const int4* __restrict__ Tets, cons
         __stcg((float4*)Out + 4 * (size_t)e + c, make_float4(out[c][0], out[c][1], out[c][2], 0.f));
 }
 
-template <typename T, typename S, bool kCorr, bool kTets, int R, bool kCl>
-__global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_constant__ TileArgs<T, S> a) {
+// How rows exchange and sum: words in global memory; a cluster's shared memory;
+// words, with two neighbours of a grid row summed together by one thread.
+enum TileForm { kWords, kCluster, kPairs };
+
+template <typename T, typename S, bool kCorr, bool kTets, int R, TileForm kForm>
+__global__ void __launch_bounds__(kTileMaxWarps * (kForm == kPairs ? 64 : 32), kForm == kPairs ? 1 : 2)
+    k_pd_tile(const __grid_constant__ TileArgs<T, S> a) {
     constexpr int kW = kTileWords<T, S>;
     constexpr int kG = kTileGroup<T>;
+    constexpr bool kCl = kForm == kCluster, kPair = kForm == kPairs;
     constexpr int kUnroll = R == 1 ? 2 : 1;  // two rows per thread leave no registers for more
     extern __shared__ __align__(16) unsigned char smem[];
     if (outer_stopped(a.gate)) return;
-    const int tile = (int)blockIdx.x + a.lo;
+    // pairs: a CTA is several tiles, of as many threads each, with barriers of their own
+    const int nthr = kPair ? (int)blockDim.x / kPairTiles : (int)blockDim.x, part = kPair ? (int)threadIdx.x / nthr : 0;
+    const int tid = (int)threadIdx.x - part * nthr;
+    const int tile = a.lo + (kPair ? kPairTiles * (int)blockIdx.x + part : (int)blockIdx.x);
+    unsigned tmem = 0;
+    __shared__ unsigned tmem_base;
+    auto finish = [&]() {  // every way out from here on
+        if constexpr (kPair) {
+            tmem_fence_before();
+            __syncthreads();
+            tmem_fence_after();
+            if (threadIdx.x < 32) tmem_free(tmem_base, kPairColumns);
+        }
+    };
+    if constexpr (kPair) {
+        if (threadIdx.x < 32) tmem_alloc(&tmem_base, kPairColumns);
+        tmem_fence_before();
+        __syncthreads();
+        tmem_fence_after();
+        const unsigned w = threadIdx.x >> 5;
+        tmem = tmem_base + ((w & 3u) << 21) + 2u * kPairEntries * (w >> 2);
+        if (tile > a.hi) return finish();
+    }
     const TileInfo ti = a.tiles[tile];
-    if (a.instStop && a.instStop[ti.model]) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    if (a.instStop && a.instStop[ti.model]) return finish();
+    auto sync = [&]() {  // of the tile's threads
+        if constexpr (kPair) half_sync(1 + part, nthr);
+        else __syncthreads();
+    };
+    auto sync_or = [&](bool v) -> bool {
+        if constexpr (kPair) return half_sync_or(1 + part, nthr, v);
+        else return __syncthreads_or(v);
+    };
+    const int warp = tid >> 5, lane = tid & 31, nw = nthr >> 5;
 
     // ---- shared memory: values, offset patterns, two vectors of the local
     // vertices as (x, y) pairs and z ----
@@ -108,15 +145,16 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
     // (in a cluster the vectors come first and are laid out alike in every CTA)
     const int nl = kCl ? a.nlocMax : ti.nloc;
     const int vecBytes = (int)a16(3 * (size_t)nl * sizeof(T));
-    unsigned char* tab = smem + (kCl ? (kCorr ? 3 : 2) * (size_t)vecBytes : 0);
+    unsigned char* tab = smem + part * (size_t)a.partSmem + (kCl ? (kCorr ? 3 : 2) * (size_t)vecBytes : 0);
     T* sval = reinterpret_cast<T*>(tab);
-    int16_t* spat = reinterpret_cast<int16_t*>(tab + a16((size_t)ti.nent * sizeof(T)));
+    int16_t* spat = reinterpret_cast<int16_t*>(tab + (kPair ? 0 : a16((size_t)ti.nent * sizeof(T))));
     unsigned char* vec0 =
-        kCl ? smem : tab + a16((size_t)ti.nent * sizeof(T)) + a16((size_t)ti.npat * a.patStride * sizeof(int16_t));
+        kCl ? smem : reinterpret_cast<unsigned char*>(spat) + a16((size_t)ti.npat * a.patStride * sizeof(int16_t));
     auto XY = [&](int b) { return reinterpret_cast<Pair<T>*>(vec0 + b * vecBytes); };
     auto Z = [&](int b) { return reinterpret_cast<T*>(XY(b) + nl); };
-    for (int q = threadIdx.x; q < ti.nent; q += blockDim.x) sval[q] = __ldg(a.val + ti.ent0 + q);
-    for (int q = threadIdx.x; q < ti.npat * a.patStride; q += blockDim.x)
+    if constexpr (!kPair)
+        for (int q = tid; q < ti.nent; q += nthr) sval[q] = __ldg(a.val + ti.ent0 + q);
+    for (int q = tid; q < ti.npat * a.patStride; q += nthr)
         spat[q] = __ldg(a.pat + (size_t)ti.pat0 * a.patStride + q);
 
     // ---- this thread's rows: slice r nw + warp, this lane.  Packed, two rows per
@@ -126,20 +164,23 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
     int gp[R];
     unsigned lpe[R], eol[R];
     T id[R];
-    auto slot = [&](int r) { return ti.slot0 + 32 * (r * nw + warp) + lane; };
+    auto slice = [&](int r) { return kPair ? 2 * warp + r : r * nw + warp; };
+    auto slot = [&](int r) { return ti.slot0 + 32 * slice(r) + lane; };
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        const int s = r * nw + warp;
+        const int s = slice(r);
         gp[r] = -1;
         lpe[r] = eol[r] = 0u;
         id[r] = T(0);
         if (s < ti.nslice) {
             const TileSlot sl = a.slots[slot(r)];
             const TileSlice sc = a.slices[ti.slice0 + s];
-            if (sl.row >= 0) {
-                gp[r] = sl.row | ((sl.pub & 1) << 30);
+            if (kPair || sl.row >= 0) {  // (pairs: an empty lane takes part in its warp's sums)
                 lpe[r] = (unsigned)sl.pos | ((unsigned)sl.pat << 16);
                 eol[r] = (unsigned)(sc.off + kG * lane) | ((unsigned)sc.len << 20);
+            }
+            if (sl.row >= 0) {
+                gp[r] = sl.row | ((sl.pub & 1) << 30);
                 id[r] = T(1) / ((a.Delastic[sl.row] + a.Dinert[sl.row]) + a.CollDiag[sl.row]);
             }
         }
@@ -152,7 +193,7 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
     auto eo = [&](int r) { return (int)(eol[r] & 0xfffffu); };
     auto el = [&](int r) { return (int)(eol[r] >> 20); };
     // the first halo row this thread polls (others through the table)
-    const TileHalo h0 = (int)threadIdx.x < ti.nhalo ? a.halo[ti.halo0 + threadIdx.x] : TileHalo{-1, 0};
+    const TileHalo h0 = tid < ti.nhalo ? a.halo[ti.halo0 + tid] : TileHalo{-1, 0};
 
     auto put = [&](int b, int q, T x, T y, T z) {
         XY(b)[q] = Pair<T>{x, y};
@@ -201,7 +242,7 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
     // every CTA that might write here, or be written to, is at the same point
     auto sync_all = [&]() {
         if constexpr (kCl) cluster_sync();
-        else __syncthreads();
+        else sync();
     };
     // wait for the word at p to carry the current tag
     auto wait_word = [&](const TileWord* p, TileWord& w) -> bool {
@@ -242,7 +283,7 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
     };
     auto fetch = [&](int b, int b2) -> bool {
         bool ok = h0.row < 0 || fetch_one(h0.row, h0.pos, b, b2);
-        for (int h = (int)(threadIdx.x + blockDim.x); ok && h < ti.nhalo; h += blockDim.x) {
+        for (int h = tid + nthr; ok && h < ti.nhalo; h += nthr) {
             const TileHalo q = a.halo[ti.halo0 + h];
             ok = fetch_one(q.row, q.pos, b, b2);
         }
@@ -255,21 +296,21 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
             return true;
         }
         if (ti.nhalo == 0) {
-            __syncthreads();
+            sync();
             return true;
         }
-        return !__syncthreads_or(!fetch(b, b2));
+        return !sync_or(!fetch(b, b2));
     };
     // tets only: what neighbours wrote to global memory before their same call
     // is visible after it (release and acquire of the tiles' phase counts)
     unsigned fl = a.flag0;
     auto global_sync = [&]() -> bool {
-        __syncthreads();
+        sync();
         ++fl;
-        if (threadIdx.x == 0) st_release(a.flags + tile, fl);
+        if (tid == 0) st_release(a.flags + tile, fl);
         bool ok = true;
         const long long t0 = clock64();
-        for (int q = (int)threadIdx.x; ok && q < ti.nnbr; q += blockDim.x) {
+        for (int q = tid; ok && q < ti.nnbr; q += nthr) {
             const int n = a.nbr[ti.nbr0 + q];
             while ((int)(ld_acquire(a.flags + n) - fl) < 0) {
                 if (clock64() - t0 > a.timeout || (ld_acquire(a.err) & kErrBarrier)) {
@@ -279,9 +320,51 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
                 }
             }
         }
-        return !__syncthreads_or(!ok);
+        return !sync_or(!ok);
     };
 
+    // pairs: the values of a warp's 32 pairs go to 64 columns of tensor memory
+    if constexpr (kPair) {
+        const float4* vp = reinterpret_cast<const float4*>(a.val + ti.ent0 + eo(0));
+        __syncwarp();
+        for (int k = 0; k < el(0); k += 2) tmem_store4(tmem + 2 * k, __ldg(vp + 16 * k));
+        tmem_store_wait();
+    }
+    // the same sums of both rows of a pair: each place is read once for the two,
+    // each with its own values (zero where a row has no such column)
+    auto pair_sum = [&](int b, T (&s)[R][3]) {
+        if constexpr (kPair) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) s[r][0] = s[r][1] = s[r][2] = T(0);
+            const uint2* pp = reinterpret_cast<const uint2*>(spat + pe(0));
+            const Pair<T>* xy = XY(b) + lp(0);
+            const T* z = Z(b) + lp(0);
+            __syncwarp();
+            for (int k = 0; k < el(0); k += 4) {
+                unsigned v[8];
+                tmem_load8(tmem + 2 * k, v);
+                const uint2 o2 = pp[k >> 2];
+                const unsigned o[2] = {o2.x, o2.y};
+                Pair<T> p[4];
+                T q[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int j = (e & 1) ? (int)o[e >> 1] >> 16 : (int)(short)(o[e >> 1] & 0xffffu);
+                    p[e] = xy[j];
+                    q[e] = z[j];
+                }
+                tmem_wait8(v);
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+#pragma unroll
+                    for (int r = 0; r < R; ++r) {
+                        s[r][0] = fma_(__uint_as_float(v[2 * e + r]), p[e].x, s[r][0]);
+                        s[r][1] = fma_(__uint_as_float(v[2 * e + r]), p[e].y, s[r][1]);
+                        s[r][2] = fma_(__uint_as_float(v[2 * e + r]), q[e], s[r][2]);
+                    }
+            }
+        }
+    };
     // sum_k N_ik z_k of owned row r over vector b, in the stored order.  Batches
     // of entries whose loads are all in flight before the first sum: a 16-byte
     // load brings eight offsets (one address in most warps), another the values
@@ -340,6 +423,15 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
             batch(std::integral_constant<int, 4>(), o, v);
         }
     };
+    auto sum_of = [&](int r, int b, const T (&ps)[R][3], T& s0, T& s1, T& s2) {
+        if constexpr (kPair) {
+            s0 = ps[r][0];
+            s1 = ps[r][1];
+            s2 = ps[r][2];
+        } else {
+            row_sum(r, b, s0, s1, s2);
+        }
+    };
     const T w = a.relax, om1 = T(1) - a.relax;
 
     // ---- positions of the local vertices: own rows and halo ----
@@ -356,19 +448,19 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
 #pragma unroll
     for (int r = 0; r < R; ++r)
         if (live(r)) load_pos(row(r), lp(r));
-    for (int h = threadIdx.x; h < ti.nhalo; h += blockDim.x) {
+    for (int h = tid; h < ti.nhalo; h += nthr) {
         const TileHalo q = a.halo[ti.halo0 + h];
         load_pos(q.row, q.pos);
     }
     sync_all();  // also: every CTA of a cluster runs before its shared memory is written
 
-    const bool third = kCl || a.third;
+    const bool third = kCl || kPair || a.third;
     int cur = 0;  // the vector that holds the positions (direct form) at the start of an iteration
     for (int lg = 0; lg < a.lg; ++lg) {
         if constexpr (kTets) {
-            for (int q = threadIdx.x; q < ti.ntet; q += blockDim.x)
+            for (int q = tid; q < ti.ntet; q += nthr)
                 tile_tet<S, kCorr>(a.tet[ti.tet0 + q], a.Tets, a.TetIdm, a.TetW, a.P, a.Ph, a.Pl, a.TetOut);
-            if (!global_sync()) return;
+            if (!global_sync()) return finish();
         }
         // correction form: the residual's matrix part of owned row r, in column
         // order (the entries below the row's own block, those in it, those above)
@@ -394,6 +486,50 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
             part(0, ka);
             part(kb, el(r));
         };
+        // the same for both rows of a pair.  The parts' bounds differ between lanes only
+        // near a block's edge: the warp runs over all its lanes' ranges, each lane
+        // adding its own.
+        auto pair_matrix = [&](Acc (&ac)[kCorr ? R : 1][3]) {
+            if constexpr (kPair && kCorr) {
+                const int16_t* pp = spat + pe(0);
+                const Pair<T>*hp = XY(0) + lp(0), *lpp = XY(1) + lp(0);
+                const T *hz = Z(0) + lp(0), *lz = Z(1) + lp(0);
+                T h[R][3], l[R][3];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    own(0, r, h[r][0], h[r][1], h[r][2]);
+                    own(1, r, l[r][0], l[r][1], l[r][2]);
+                }
+                auto range = [&](int k0, int k1, int lo, int hi) {
+                    for (int k = k0; k < k1; ++k) {
+                        unsigned v[2];
+                        tmem_load2(tmem + 2 * k, v);
+                        const int j = pp[k];
+                        const Pair<T> p = hp[j], q = lpp[j];
+                        const T pz = hz[j], qz = lz[j];
+                        tmem_wait2(v);
+                        if (k >= lo && k < hi) {
+#pragma unroll
+                            for (int r = 0; r < R; ++r) {
+                                const T vr = __uint_as_float(v[r]);
+                                if (vr == T(0)) continue;  // its partner's column
+                                ac[r][0].add(vr, diff_ff(p.x, q.x, h[r][0], l[r][0]));
+                                ac[r][1].add(vr, diff_ff(p.y, q.y, h[r][1], l[r][1]));
+                                ac[r][2].add(vr, diff_ff(pz, qz, h[r][2], l[r][2]));
+                            }
+                        }
+                        __syncwarp();
+                    }
+                };
+                const int n = el(0);
+                if (n == 0) return;  // no slice
+                const int parts = __ldg(&a.slots[slot(0)].pub), ka = (parts >> 8) & 255, kb = (parts >> 16) & 255;
+                __syncwarp();
+                range(__reduce_min_sync(~0u, ka), __reduce_max_sync(~0u, kb), ka, kb);
+                range(0, __reduce_max_sync(~0u, ka), 0, ka);
+                range(__reduce_min_sync(~0u, kb), n, kb, n);
+            }
+        };
         // ---- local step: curvature vectors, springs and (correction form without
         // a third vector) the matrix part of the residual, all from shared memory ----
         T aq[R][3], rh[R][3], px[R][3];
@@ -405,8 +541,7 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
             px[r][0] = px[r][1] = px[r][2] = T(0);
             if (!live(r)) continue;
             const int i = row(r);
-            const int s = r * nw + warp;
-            const int st = __ldg(a.stencil + ti.slice0 + s) + lane, nst = __ldg(&a.slots[slot(r)].pub) >> 24;
+            const int st = __ldg(a.stencil + ti.slice0 + slice(r)) + lane, nst = __ldg(&a.slots[slot(r)].pub) >> 24;
             const T strain = a.Strain[i];
             T a0, a1, a2;
             if constexpr (kCorr) {
@@ -518,13 +653,13 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
                 send(0, qb, r, aq[r][0], aq[r][1], aq[r][2]);
                 put(qb, lp(r), aq[r][0], aq[r][1], aq[r][2]);
             }
-        if (!arrive(qb)) return;
+        if (!arrive(qb)) return finish();
         // ---- bending, then the right-hand side (direct) or residual (correction) ----
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             if (!live(r)) continue;
             const int i = row(r);
-            const int st = __ldg(a.stencil + ti.slice0 + r * nw + warp) + lane, nst = __ldg(&a.slots[slot(r)].pub) >> 24;
+            const int st = __ldg(a.stencil + ti.slice0 + slice(r)) + lane, nst = __ldg(&a.slots[slot(r)].pub) >> 24;
             const Pair<T>* qp = XY(qb) + lp(r);
             const T* qz = Z(qb) + lp(r);
             const T b0 = a.tBend0[i];
@@ -548,6 +683,12 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
                         r1.add(t.y);
                         r2.add(t.z);
                     }
+                if constexpr (kPair) {
+                    acc[r][0] = r0;
+                    acc[r][1] = r1;
+                    acc[r][2] = r2;
+                    continue;
+                }
                 if (third) matrix_part(r, r0, r1, r2);
                 rh[r][0] = r0.value();
                 rh[r][1] = r1.value();
@@ -588,17 +729,29 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
             }
         }
 
+        if constexpr (kPair && kCorr) {
+            pair_matrix(acc);
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (live(r)) {
+                    rh[r][0] = acc[r][0].value();
+                    rh[r][1] = acc[r][1].value();
+                    rh[r][2] = acc[r][2].value();
+                }
+        }
+
         // ---- Chebyshev-accelerated R2 iteration as two J sweeps per step ----
         // direct form: on x from the positions; correction form: on delta from 0
         ++tag;
         {
-            T y[R][3];
+            T y[R][3], ps[R][3];
+            if (kPair && !kCorr) pair_sum(cur, ps);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 T s0 = T(0), s1 = T(0), s2 = T(0);
                 T c0 = T(0), c1 = T(0), c2 = T(0);
                 if (!kCorr) {
-                    row_sum(r, cur, s0, s1, s2);
+                    sum_of(r, cur, ps, s0, s1, s2);
                     own(cur, r, c0, c1, c2);
                 }
                 y[r][0] = jacobi<kCorr>(om1, c0, w, s0, rh[r][0], id[r]);
@@ -616,16 +769,18 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
                     put(cur, lp(r), y[r][0], y[r][1], y[r][2]);
                 }
         }
-        if (!arrive(cur)) return;
+        if (!arrive(cur)) return finish();
         for (int it = 0; it < a.cheby; ++it) {
             const bool last = it == a.cheby - 1;
             const T om = a.omega[it];
             // x = S(y), Chebyshev-combined with the step before the last
             ++tag;
+            T ps[R][3];
+            pair_sum(cur, ps);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 T s0, s1, s2, n[3];
-                row_sum(r, cur, s0, s1, s2);
+                sum_of(r, cur, ps, s0, s1, s2);
                 T c0, c1, c2;
                 own(cur, r, c0, c1, c2);
                 n[0] = jacobi<kCorr>(om1, c0, w, s0, rh[r][0], id[r]);
@@ -654,13 +809,14 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
             }
             if (last) break;
             cur ^= 1;
-            if (!arrive(cur)) return;
+            if (!arrive(cur)) return finish();
             // y = S(x)
             ++tag;
+            pair_sum(cur, ps);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 T s0, s1, s2;
-                row_sum(r, cur, s0, s1, s2);
+                sum_of(r, cur, ps, s0, s1, s2);
                 T c0, c1, c2;
                 own(cur, r, c0, c1, c2);
                 const T y0 = jacobi<kCorr>(om1, c0, w, s0, rh[r][0], id[r]);
@@ -671,7 +827,7 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
                 put(cur ^ 1, lp(r), y0, y1, y2);
             }
             cur ^= 1;
-            if (!arrive(cur)) return;
+            if (!arrive(cur)) return finish();
         }
         // ---- the new positions ----
         if constexpr (kCorr) {
@@ -696,35 +852,45 @@ __global__ void __launch_bounds__(kTileMaxWarps * 32, 2) k_pd_tile(const __grid_
                 put(1, lp(r), lx, ly, lz);
             }
             if (lg == a.lg - 1) break;
-            if (!arrive(0, 1)) return;
+            if (!arrive(0, 1)) return finish();
         } else {
             cur ^= 1;
             if (lg == a.lg - 1) break;
-            if (!arrive(cur)) return;
+            if (!arrive(cur)) return finish();
         }
         if constexpr (kTets)
-            if (!global_sync()) return;
+            if (!global_sync()) return finish();
     }
     if constexpr (kCl) cluster_sync();  // nobody leaves while another may write to its shared memory
+    finish();
 }
 
-template <typename T, typename S, bool kCorr>
-const void* tile_kernel(int R, bool tets) {
+template <typename T, typename S>
+const void* tile_kernel(int R, bool tets, bool pairs) {
+    constexpr bool kCorr = !std::is_same<T, S>::value;
     if constexpr (sizeof(T) == 8) {
-        return tets || R != 1 ? nullptr : (const void*)k_pd_tile<T, S, kCorr, false, 1, false>;
+        return tets || pairs || R != 1 ? nullptr : (const void*)k_pd_tile<T, S, kCorr, false, 1, kWords>;
     } else {
         if (R != 1 && R != 2) return nullptr;
-        if (tets) return R == 1 ? (const void*)k_pd_tile<T, S, kCorr, true, 1, false> : (const void*)k_pd_tile<T, S, kCorr, true, 2, false>;
-        return R == 1 ? (const void*)k_pd_tile<T, S, kCorr, false, 1, false> : (const void*)k_pd_tile<T, S, kCorr, false, 2, false>;
+        if (pairs) return tets || R != 2 ? nullptr : (const void*)k_pd_tile<T, S, kCorr, false, 2, kPairs>;
+        if (tets) return R == 1 ? (const void*)k_pd_tile<T, S, kCorr, true, 1, kWords> : (const void*)k_pd_tile<T, S, kCorr, true, 2, kWords>;
+        return R == 1 ? (const void*)k_pd_tile<T, S, kCorr, false, 1, kWords> : (const void*)k_pd_tile<T, S, kCorr, false, 2, kWords>;
     }
+}
+
+// Pairs: the CTA's tiles, and more than half of an SM's shared memory: the CTA takes all
+// columns of tensor memory, so another launch's must not share the SM.
+size_t cta_smem(bool pairs, size_t smem) {
+    return pairs ? std::max(kPairTiles * smem, (size_t)(116 * 1024)) : smem;
 }
 
 }  // namespace
 
 template <typename T, typename S>
-int tile_residents(int R, bool tets, int threads, size_t smem, int sms) {
-    const void* f = tile_kernel<T, S, !std::is_same<T, S>::value>(R, tets);
+int tile_residents(int R, bool tets, bool pairs, int threads, size_t smem, int sms) {
+    const void* f = tile_kernel<T, S>(R, tets, pairs);
     if (!f || threads > kTileMaxWarps * 32) return 0;
+    smem = cta_smem(pairs, smem);
     // the kernel's limit is raised only: other contexts may hold larger tiles
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) return 0;
@@ -732,24 +898,28 @@ int tile_residents(int R, bool tets, int threads, size_t smem, int sms) {
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return 0;
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem) != cudaSuccess) return 0;
-    return per_sm * sms;
+    const int per_cta = pairs ? kPairTiles : 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads * per_cta, smem) != cudaSuccess)
+        return 0;
+    return per_sm * sms * per_cta;
 }
 
 template <typename T, typename S>
-cudaError_t launch_pd_tile(const TileArgs<T, S>& args, int tiles, int R, bool tets, int threads, size_t smem,
+cudaError_t launch_pd_tile(const TileArgs<T, S>& args, int tiles, int R, bool tets, bool pairs, int threads, size_t smem,
                            cudaStream_t s) {
-    const void* f = tile_kernel<T, S, !std::is_same<T, S>::value>(R, tets);
+    const void* f = tile_kernel<T, S>(R, tets, pairs);
     if (!f || tiles < 1) return cudaErrorInvalidConfiguration;
     void* params[] = {(void*)&args};
-    return cudaLaunchCooperativeKernel(f, dim3(tiles), dim3(threads), params, smem, s);
+    const int per_cta = pairs ? kPairTiles : 1;
+    return cudaLaunchCooperativeKernel(f, dim3((tiles + per_cta - 1) / per_cta), dim3(threads * per_cta), params,
+                                       cta_smem(pairs, smem), s);
 }
 
 namespace {
 
 template <typename T, typename S>
 const void* cluster_kernel() {
-    return (const void*)k_pd_tile<T, S, !std::is_same<T, S>::value, false, 1, true>;
+    return (const void*)k_pd_tile<T, S, !std::is_same<T, S>::value, false, 1, kCluster>;
 }
 cudaLaunchConfig_t cluster_config(int tiles, int threads, size_t smem, cudaStream_t s, cudaLaunchAttribute* at) {
     cudaLaunchConfig_t c = {};
@@ -805,11 +975,11 @@ cudaError_t launch_pd_tile_cluster(const TileArgs<T, S>& args, int tiles, int th
 }
 
 #define PDIPC_INST_TILE(T, S)                                                                     \
-    template int tile_residents<T, S>(int, bool, int, size_t, int);                               \
+    template int tile_residents<T, S>(int, bool, bool, int, size_t, int);                         \
     template bool tile_cluster_fits<T, S>(int, int, size_t);                                      \
     template cudaError_t launch_pd_tile_cluster<T, S>(const TileArgs<T, S>&, int, int, size_t,    \
                                                       cudaStream_t);                              \
-    template cudaError_t launch_pd_tile<T, S>(const TileArgs<T, S>&, int, int, bool, int, size_t, \
+    template cudaError_t launch_pd_tile<T, S>(const TileArgs<T, S>&, int, int, bool, bool, int, size_t, \
                                               cudaStream_t);
 PDIPC_INST_TILE(float, float)
 PDIPC_INST_TILE(float, double)

@@ -1955,7 +1955,11 @@ private:
                 lim.cluster_min = kTileClusterMin;
                 lim.cluster_rows = kTileClusterRows;
             }
+            lim.pairs = !fp64;
+            lim.pairs = !fp64;
+            lim.pair_rows = kPairRows;
             build_tile_plan(H, lim, order_block, tile_);
+            tile_.smem_bytes = (tile_.smem_bytes + 15) / 16 * 16;
             if (tile_.ok && tile_.cluster &&
                 !tile_cluster_fits<T, TC>((int)tile_.tiles.size(), tile_.threads, tile_.smem_bytes)) {
                 lim.cluster = 0;
@@ -1969,7 +1973,7 @@ private:
                 held = tile3_residents(tile_.threads, tile_.smem_bytes, nsm);
             } else {
                 held =
-                    tile_residents<T, TC>(tile_.rows_per_thread, H.ntet > 0, tile_.threads, tile_.smem_bytes, nsm);
+                    tile_residents<T, TC>(tile_.rows_per_thread, H.ntet > 0, tile_.pairs, tile_.threads, tile_.smem_bytes, nsm);
             }
             for (const TileGroup& g : tile_.groups)
                 if (g.hi - g.lo + 1 > held) tile_.ok = false;
@@ -2069,6 +2073,7 @@ private:
         a.instStop = prm_.instance_stop ? d.InstStop : nullptr;
         a.tape = nullptr;
         a.third = tile_.vectors > 2;
+        a.partSmem = (int)tile_.smem_bytes;
         tile_on_ = true;
         return PDIPC_OK;
     }
@@ -2085,6 +2090,7 @@ private:
         }
         for (const TileGroup& g : tile_.groups) {
             targs_.lo = g.lo;
+            targs_.hi = g.hi;
             // fresh tags and phase counts: every earlier launch's lie below them
             targs_.epoch0 = targs_.flag0 = epoch_;
             epoch_ += tile_phases(c_.lg, c_.cheby);
@@ -2092,7 +2098,7 @@ private:
             if (tile_.cluster)
                 e = launch_pd_tile_cluster<T, TC>(targs_, g.hi - g.lo + 1, tile_.threads, tile_.smem_bytes, s_);
             else if (!tile3_)
-                e = launch_pd_tile<T, TC>(targs_, g.hi - g.lo + 1, tile_.rows_per_thread, d_.ntet > 0, tile_.threads,
+                e = launch_pd_tile<T, TC>(targs_, g.hi - g.lo + 1, tile_.rows_per_thread, d_.ntet > 0, tile_.pairs, tile_.threads,
                                           tile_.smem_bytes, s_);
             else if constexpr (std::is_same<T, double>::value)
                 e = launch_pd_tile3(targs_, g.hi - g.lo + 1, tile_.threads, tile_.smem_bytes, s_);

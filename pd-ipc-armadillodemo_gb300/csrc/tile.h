@@ -11,6 +11,19 @@
 
 namespace pdipc {
 
+// Pairs (FP32 arithmetic on a grid, no tets): a thread sums two neighbours of a grid
+// row over the union of their columns, 28 in place of 24 + 20, so that a place of the
+// iterate is read once for both; the values, two per entry, lie in tensor memory (a
+// warp's 32 pairs take 64 of the columns of its quarter of the lanes), where reading
+// them takes nothing of shared memory's bandwidth, which bounded these sums.  A
+// kernel that uses tensor memory runs one CTA per SM: it is two tiles, half of the
+// threads each, and takes all 512 columns.
+// One sweep of a mixed solve, before -> with pairs: 512x512 4.47 -> 3.73 us, four
+// 256x256 4.84 -> 3.65; one solve 3.24 -> 2.90 ms and 3.49 -> 2.93, 40 cloths of 16^2
+// to 126^2 1.93 -> 1.74, 430x430 1.40 -> 1.30 (FP32 1.17 -> 1.11).  Up to kPairRows
+// rows per tile the sweeps wait for each other's words rather than for the sums, and
+// half the threads take longer (333x333: 1.32, 1.44 with pairs; 380x380: 1.25, 1.20).
+constexpr int kPairColumns = 512, kPairTiles = 2, kPairRows = 400;
 constexpr int kTileMaxWarps = 14;  // row warps per CTA; two CTAs share an SM (72 registers per thread)
 
 // A published value: 16 bytes read and written as one, the phase's tag in the
@@ -82,7 +95,8 @@ struct TileArgs {
     const OuterGate* gate;
     const unsigned* instStop;  // per-instance stopping: tiles of a stopped model return at entry
     V4<T>* tape;               // direct form: the positions at the start of every local-global iteration, or null
-    int lo;                    // first tile of this launch
+    int lo, hi;                // tiles of this launch
+    int partSmem;              // pairs: shared memory of one of a CTA's tiles
     const int4* push;          // cluster: the readers of every slot's row (TilePlan::push)
     int nlocMax;               // cluster: places of each vector
     int third;                 // correction form: the tiles hold a third vector
@@ -100,9 +114,9 @@ inline unsigned tile_phases(int lg, int cheby) { return (unsigned)(lg * (2 * che
 
 // Residents: CTAs of the variant one cooperative launch can hold (0: no such variant).
 template <typename T, typename S>
-int tile_residents(int rows_per_thread, bool tets, int threads, size_t smem, int sms);
+int tile_residents(int rows_per_thread, bool tets, bool pairs, int threads, size_t smem, int sms);
 template <typename T, typename S>
-cudaError_t launch_pd_tile(const TileArgs<T, S>& args, int tiles, int rows_per_thread, bool tets, int threads,
+cudaError_t launch_pd_tile(const TileArgs<T, S>& args, int tiles, int rows_per_thread, bool tets, bool pairs, int threads,
                            size_t smem, cudaStream_t s);
 // The tiles as one thread-block cluster (FP32 arithmetic, a row per thread): a
 // thread writes its new vector into the shared memory of the tiles that read it,

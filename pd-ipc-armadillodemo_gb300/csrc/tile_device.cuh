@@ -56,6 +56,57 @@ __device__ __forceinline__ void st_remote(unsigned, double) {}
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
 }
+// ---- barrier of some of a CTA's threads, and whether any of them says so ----
+__device__ __forceinline__ void half_sync(int id, int threads) {
+    asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ bool half_sync_or(int id, int threads, bool v) {
+    int any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 q, %1, 0;\n\tbarrier.red.or.pred p, %2, %3, q;\n\t"
+        "selp.s32 %0, 1, 0, p;\n\t}"
+        : "=r"(any)
+        : "r"((int)v), "r"(id), "r"(threads)
+        : "memory");
+    return any != 0;
+}
+// ---- tensor memory as a store of constants: 512 columns x 128 lanes of 32 bits per
+// SM, of which a warp reads and writes the 32 lanes of its quarter (warp % 4).  All
+// of a warp's threads take part in each of these. ----
+__device__ __forceinline__ void tmem_alloc(unsigned* where, unsigned columns) {  // one warp
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n\t"
+                 "tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(where)),
+                 "r"(columns)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_free(unsigned base, unsigned columns) {  // one warp
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(columns) : "memory");
+}
+__device__ __forceinline__ void tmem_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tmem_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tmem_store4(unsigned addr, float4 v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(__float_as_uint(v.x)),
+                 "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w))
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// a load is under way until the wait that names its registers
+__device__ __forceinline__ void tmem_load8(unsigned addr, unsigned (&u)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void tmem_wait8(unsigned (&u)[8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(u[0]), "+r"(u[1]), "+r"(u[2]), "+r"(u[3]), "+r"(u[4]), "+r"(u[5]), "+r"(u[6]), "+r"(u[7]));
+}
+__device__ __forceinline__ void tmem_load2(unsigned addr, unsigned (&u)[2]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(u[0]), "=r"(u[1]) : "r"(addr));
+}
+__device__ __forceinline__ void tmem_wait2(unsigned (&u)[2]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(u[0]), "+r"(u[1]));
+}
 __device__ __forceinline__ unsigned long long pack2(unsigned a, unsigned b) {
     return (unsigned long long)a | ((unsigned long long)b << 32);
 }

@@ -147,14 +147,17 @@ bool cut_model(const HostTables& H, const Model& m, int k, int max_slices, std::
 
 }  // namespace
 
-size_t tile_smem_bytes(const TileInfo& t, int pat_stride, int value_bytes, int vectors, bool slot_rhs) {
+size_t tile_smem_bytes(const TileInfo& t, int pat_stride, int value_bytes, int vectors, bool slot_rhs, bool pairs) {
     auto a16 = [](size_t b) { return (b + 15) / 16 * 16; };
-    return a16((size_t)t.nent * value_bytes) + a16((size_t)t.npat * pat_stride * sizeof(int16_t)) +
+    return (pairs ? 0 : a16((size_t)t.nent * value_bytes)) + a16((size_t)t.npat * pat_stride * sizeof(int16_t)) +
            vectors * a16(3 * (size_t)t.nloc * value_bytes) + (slot_rhs ? 96 * (size_t)t.nslice * value_bytes : 0);
 }
 
-void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block, TilePlan& P) {
-    P = TilePlan();
+namespace {
+
+// pairs: slices are of pairs of rows; the tiles are cut for `spare` slices less than
+// they may have, since rows without a partner take more.
+void try_plan(const HostTables& H, const TileLimits& lim, int order_block, bool pairs, int spare, TilePlan& P) {
     const int ns = H.nsim;
     if (ns == 0 || ns >= 1 << 30) return;
     std::vector<Model> models;
@@ -165,7 +168,7 @@ void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block
         i = e;
     }
     const int max_slices = lim.max_warps * lim.max_rows_per_thread;
-    const int max_rows = max_slices * kLanes;
+    const int cut_slices = max_slices - spare, max_rows = cut_slices * kLanes;
 
     // ---- rows per tile: one tile per SM where a tile then has at most one row
     // per thread, else two per SM (a count in between leaves SMs with half the
@@ -184,7 +187,7 @@ void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block
             bool done = false;
             for (int tries = 0; tries < 64 && !done; ++tries) {
                 own.resize(first);
-                done = cut_model(H, models[q], k, max_slices, own);
+                done = cut_model(H, models[q], k, cut_slices, own);
                 if (!done) k += 1 + k / 16;
             }
             if (!done) return false;
@@ -221,6 +224,9 @@ void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block
         target = std::min(max_rows, target + std::max(8, target / 16));
     }
     if (!fits && (models.size() < 2 || H.ntet > 0)) return;
+    P.pairs = pairs && most_tiles == lim.co_resident;
+    for (const Model& m : models) P.pairs = P.pairs && m.stride > 0;
+    if (pairs && !P.pairs) return;
     const int nt = (int)own.size();
 
     // ---- launches: runs of whole models ----
@@ -242,7 +248,10 @@ void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block
         if (P.groups.size() > 1 && H.ntet > 0) return;
     }
 
-    std::vector<int> tileOf(ns, -1), cls(ns, 0);
+    std::vector<int> tileOf(ns, -1), cls(ns, 0), modelOf(P.pairs ? ns : 0);
+    if (P.pairs)
+        for (size_t q = 0; q < models.size(); ++q)
+            std::fill(modelOf.begin() + models[q].lo, modelOf.begin() + models[q].hi, (int)q);
     for (int t = 0; t < nt; ++t)
         for (int v : own[t]) tileOf[v] = t;
     for (const Model& m : models)
@@ -305,7 +314,15 @@ void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block
     int patW = 2;
     for (int i = 0; i < ns; ++i) patW = std::max(patW, H.nPtr[i + 1] - H.nPtr[i]);
     if (patW > 255) return;
-    P.pat_stride = (patW + 7) / 8 * 8;
+    P.pat_stride = P.pairs ? kPairEntries : (patW + 7) / 8 * 8;
+    // the other row of v's pair: its neighbour in the grid row, of the same tile and
+    // in the same block of the summation order; -1: none
+    auto partner = [&](int v) {
+        const Model& m = models[modelOf[v]];
+        const int x = (v - m.lo) % m.stride, u = x % 2 ? v - 1 : v + 1;
+        if (u >= m.hi || (x % 2 == 0 && x + 1 >= m.stride) || tileOf[u] != tileOf[v]) return -1;
+        return order_block > 0 && u / order_block != v / order_block ? -1 : u;
+    };
 
     // ---- tables, tile by tile ----
     std::vector<int> pos(ns, 0), ext, ent(patW);
@@ -325,38 +342,119 @@ void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block
         // slices: runs of own rows of one parity; kept within 32 consecutive
         // places of the local vectors (no two lanes in one bank) when that
         // costs at most 15% more slices
-        std::vector<int> rows = own[t];
-        std::sort(rows.begin(), rows.end(), order);
+        // (of pairs: the first rows, in the order of the grid)
+        std::vector<int> rows;
+        for (int v : own[t]) {
+            const int u = P.pairs ? partner(v) : -1;
+            if (u < 0 || order(v, u)) rows.push_back(v);
+        }
+        if (!P.pairs) std::sort(rows.begin(), rows.end(), order);
+        const int per = P.pairs ? 2 : 1;  // slices of a run
         std::vector<int> beg;  // first row of each slice
         for (int span = 1; span >= 0; --span) {
             std::vector<int> b;
             for (int q = 0; q < (int)rows.size(); ++q) {
-                const bool brk = b.empty() || q - b.back() >= kLanes || cls[rows[q]] != cls[rows[b.back()]] ||
-                                 (span && pos[rows[q]] - pos[rows[b.back()]] >= kLanes);
+                const bool brk = b.empty() || q - b.back() >= kLanes ||
+                                 (!P.pairs && cls[rows[q]] != cls[rows[b.back()]]) ||
+                                 (span && std::abs(pos[rows[q]] - pos[rows[b.back()]]) >= kLanes);
                 if (brk) b.push_back(q);
             }
             if (span) {
                 beg = b;
-            } else if ((int)beg.size() > max_slices || beg.size() * 100 > b.size() * 115) {
+            } else if ((int)beg.size() * per > max_slices || beg.size() * 100 > b.size() * 115) {
                 beg = b;
             }
         }
-        if ((int)beg.size() > max_slices) return;
-        most = std::max(most, (int)beg.size());
+        if ((int)beg.size() * per > max_slices) return;
+        most = std::max(most, (int)beg.size() * per);
         T.model = tileModel[t];
-        T.nslice = (int)beg.size();
+        T.nslice = (int)beg.size() * per;
         T.slot0 = (int)P.slots.size();
         T.slice0 = (int)P.slices.size();
         T.ent0 = (int)P.val.size();
         T.pat0 = (int)(P.pat.size() / P.pat_stride);
         std::unordered_map<uint64_t, std::vector<int>> seen;  // hash of the offsets -> pattern ids
         int npat = 0;
-        for (int s = 0; s < T.nslice; ++s) {
-            const int q0 = beg[s], q1 = s + 1 < T.nslice ? beg[s + 1] : (int)rows.size();
+        auto pattern = [&]() {  // of the offsets o
+            uint64_t h = 1469598103934665603ull;
+            for (int16_t v : o) h = (h ^ (uint16_t)v) * 1099511628211ull;
+            for (int c : seen[h])
+                if (std::memcmp(&P.pat[(size_t)(T.pat0 + c) * P.pat_stride], o.data(), sizeof(int16_t) * P.pat_stride) == 0)
+                    return c;
+            seen[h].push_back(npat);
+            P.pat.insert(P.pat.end(), o.begin(), o.end());
+            return npat++;
+        };
+        // entry e's part in the order of row r's sum: own block, below it, above it
+        auto part = [&](int r, int e) {
+            if (order_block <= 0) return 0;
+            const int lo = r / order_block * order_block;
+            return H.nCol[e] < lo ? 1 : H.nCol[e] < lo + order_block ? 0 : 2;
+        };
+        for (int s = 0; s < (int)beg.size(); ++s) {
+            const int q0 = beg[s], q1 = s + 1 < (int)beg.size() ? beg[s + 1] : (int)rows.size();
+            const size_t base = P.val.size();
+            if (P.pairs) {
+                std::vector<TileSlot> second(kLanes, TileSlot{-1, 0, 0, 0});
+                std::vector<double> v(2 * kPairEntries * kLanes, 0.0);  // by entry, lane, row
+                int len = 0;
+                TileSlot last{-1, 0, 0, 0};
+                for (int lane = 0; lane < kLanes; ++lane) {
+                    if (q0 + lane >= q1) {  // an empty lane sums zeros at valid places
+                        P.slots.push_back(last);
+                        second[lane] = last;
+                        continue;
+                    }
+                    const int r = rows[q0 + lane], u = partner(r);
+                    struct Entry {
+                        int part, col;
+                        double v[2];
+                    };
+                    std::vector<Entry> m;
+                    for (int w = 0; w < (u < 0 ? 1 : 2); ++w)
+                        for (int row = w ? u : r, e = H.nPtr[row]; e < H.nPtr[row + 1]; ++e) {
+                            Entry x{part(row, e), H.nCol[e], {0.0, 0.0}};
+                            x.v[w] = H.nVal[e];
+                            m.push_back(x);
+                        }
+                    std::sort(m.begin(), m.end(), [](const Entry& x, const Entry& y) {
+                        return x.part != y.part ? x.part < y.part : x.col < y.col;
+                    });
+                    int n = 0, ka = 0, kb = 0;
+                    for (size_t q = 0; q < m.size(); ++q) {
+                        if (n > 0 && m[n - 1].col == m[q].col && m[n - 1].part == m[q].part) {
+                            for (int w = 0; w < 2; ++w) m[n - 1].v[w] += m[q].v[w];  // one of the two is zero
+                        } else {
+                            m[n++] = m[q];
+                        }
+                    }
+                    if (n > kPairEntries) return;
+                    for (int k = 0; k < n; ++k) {
+                        ka += order_block > 0 && m[k].part == 0;
+                        kb += order_block > 0 && m[k].part < 2;
+                        for (int w = 0; w < 2; ++w) v[2 * (kLanes * k + lane) + w] = m[k].v[w];
+                    }
+                    len = std::max(len, n);
+                    for (int k = 0; k < P.pat_stride; ++k)
+                        o[k] = n > 0 ? (int16_t)(pos[m[std::min(k, n - 1)].col] - pos[r]) : (int16_t)0;
+                    const int pat = pattern() * P.pat_stride, parts = (ka << 8) | (kb << 16);
+                    P.slots.push_back(TileSlot{r, pos[r], pat, pub[r] | parts});
+                    last = TileSlot{-1, pos[r], pat, parts};
+                    second[lane] = u < 0 ? last : TileSlot{u, pos[u], pat, pub[u] | parts};
+                }
+                P.slots.insert(P.slots.end(), second.begin(), second.end());
+                len = (len + 3) / 4 * 4;
+                P.slices.push_back(TileSlice{(int)(base - T.ent0), len});
+                P.slices.push_back(TileSlice{(int)(base - T.ent0), 0});
+                P.val.resize(base + 2 * (size_t)len * kLanes);
+                for (int k = 0; k < len; ++k)
+                    for (int q = 0; q < 2 * kLanes; ++q)
+                        P.val[base + 128 * (size_t)(k / 2) + 4 * (q / 2) + 2 * (k % 2) + q % 2] = v[2 * kLanes * (size_t)k + q];
+                continue;
+            }
             int len = 0;
             for (int q = q0; q < q1; ++q) len = std::max(len, H.nPtr[rows[q] + 1] - H.nPtr[rows[q]]);
             len = (len + 3) / 4 * 4;
-            const size_t base = P.val.size();
             P.slices.push_back(TileSlice{(int)(base - T.ent0), len});
             P.val.resize(base + (size_t)len * kLanes, 0.0);
             for (int lane = 0; lane < kLanes; ++lane) {
@@ -368,34 +466,17 @@ void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block
                 for (int k = 0; k < n; ++k) ent[k] = b + k;
                 int ka = 0, kb = 0;
                 if (order_block > 0) {  // own block first, then the columns below it, then those above
-                    const int lo = r / order_block * order_block, hi = lo + order_block;
-                    std::stable_sort(ent.begin(), ent.begin() + n, [&](int x, int y) {
-                        auto part = [&](int e) { return H.nCol[e] < lo ? 1 : H.nCol[e] < hi ? 0 : 2; };
-                        return part(x) < part(y);
-                    });
+                    std::stable_sort(ent.begin(), ent.begin() + n, [&](int x, int y) { return part(r, x) < part(r, y); });
                     for (int k = 0; k < n; ++k) {
-                        const int c = H.nCol[ent[k]];
-                        ka += c >= lo && c < hi;
-                        kb += c < hi;
+                        ka += part(r, ent[k]) == 0;
+                        kb += part(r, ent[k]) < 2;
                     }
                 }
                 std::fill(o.begin(), o.end(), (int16_t)0);
                 for (int k = 0; k < P.pat_stride; ++k)
                     o[k] = n > 0 ? (int16_t)(pos[H.nCol[ent[std::min(k, n - 1)]]] - pos[r]) : (int16_t)0;
                 for (int k = 0; k < n; ++k) P.val[base + (size_t)kLanes * G * (k / G) + (size_t)G * lane + k % G] = H.nVal[ent[k]];
-                uint64_t h = 1469598103934665603ull;
-                for (int16_t v : o) h = (h ^ (uint16_t)v) * 1099511628211ull;
-                int id = -1;
-                for (int c : seen[h])
-                    if (std::memcmp(&P.pat[(size_t)(T.pat0 + c) * P.pat_stride], o.data(),
-                                    sizeof(int16_t) * P.pat_stride) == 0)
-                        id = c;
-                if (id < 0) {
-                    id = npat++;
-                    seen[h].push_back(id);
-                    P.pat.insert(P.pat.end(), o.begin(), o.end());
-                }
-                P.slots.push_back(TileSlot{r, pos[r], id * P.pat_stride, pub[r] | (ka << 8) | (kb << 16)});
+                P.slots.push_back(TileSlot{r, pos[r], pattern() * P.pat_stride, pub[r] | (ka << 8) | (kb << 16)});
             }
         }
         for (int s = 0; s < T.nslice; ++s) {
@@ -439,8 +520,10 @@ void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block
             T.ntet = (int)tetsOf[t].size();
             P.tet.insert(P.tet.end(), tetsOf[t].begin(), tetsOf[t].end());
         }
-        const size_t sm = tile_smem_bytes(T, P.pat_stride, lim.value_bytes, 2, lim.slot_rhs);
-        if (lim.vectors > 2) most3 = std::max(most3, tile_smem_bytes(T, P.pat_stride, lim.value_bytes, lim.vectors, lim.slot_rhs));
+        const size_t sm = tile_smem_bytes(T, P.pat_stride, lim.value_bytes, 2, lim.slot_rhs, P.pairs);
+        if (lim.vectors > 2)
+            most3 = std::max(most3,
+                             tile_smem_bytes(T, P.pat_stride, lim.value_bytes, lim.vectors, lim.slot_rhs, P.pairs));
         if (sm > lim.smem) return;
         P.smem_bytes = std::max(P.smem_bytes, sm);
         P.tiles.push_back(T);
@@ -471,19 +554,34 @@ void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block
         if (!P.cluster) {  // larger tiles have fewer readers
             TileLimits l = lim;
             l.cluster = lim.cluster >= 8 ? lim.cluster / 2 : 0;
-            build_tile_plan(H, l, order_block, P);
+            P = TilePlan();
+            try_plan(H, l, order_block, pairs, spare, P);
             return;
         }
         P.smem_bytes = sm;
         most3 = sm;
     }
-    P.rows_per_thread = (most + lim.max_warps - 1) / lim.max_warps;
+    P.rows_per_thread = P.pairs ? 2 : (most + lim.max_warps - 1) / lim.max_warps;
     P.threads = (most + P.rows_per_thread - 1) / P.rows_per_thread * kLanes;
     if (lim.vectors > 2 && most3 <= lim.smem) {
         P.vectors = lim.vectors;
         P.smem_bytes = most3;
     }
-    P.ok = true;
+    P.ok = !P.pairs || P.vectors == lim.vectors;
+}
+
+}  // namespace
+
+void build_tile_plan(const HostTables& H, const TileLimits& lim, int order_block, TilePlan& P) {
+    if (lim.pairs && H.ntet == 0 && H.nsim > lim.pair_rows * lim.co_resident)
+        for (int spare = 0; spare <= 6; spare += 2) {
+            P = TilePlan();
+            try_plan(H, lim, order_block, true, spare, P);
+            if (P.ok || !P.pairs) break;
+        }
+    if (P.ok && P.pairs) return;
+    P = TilePlan();
+    try_plan(H, lim, order_block, false, 0, P);
 }
 
 }  // namespace pdipc

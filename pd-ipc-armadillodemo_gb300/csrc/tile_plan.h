@@ -56,6 +56,8 @@ struct TileLimits {
     int cluster = 0;          // CTAs of a cluster at most (0: none),
     int cluster_min = 0;      // where there are more rows than this,
     int cluster_rows = 0;     // and no more than this many per CTA
+    bool pairs = false;       // a thread may sum two neighbours of a grid row together, where the
+    int pair_rows = 0;        // tiles of one launch would hold more rows than this each
     bool slot_rhs = false;    // a tile also holds three values per slot (pd_tile3.cu)
     int group_cap = 1 << 30;  // pdipc_params.pd_group_ctas
     size_t smem = 113 * 1024; // per CTA
@@ -74,6 +76,13 @@ struct TilePlan {
     bool cluster = false;
     int nloc_max = 0;
     std::vector<int> push;
+    // slices 2u and 2u + 1 hold, lane by lane, two neighbours of a grid row whose
+    // sums run together over the union of their columns (places relative to the
+    // first row's; parts [0, a) [a, b) [b, ...) of the union).  Only slice 2u has
+    // entries: k of lane l for the first and second row at off + 128 (k / 2) + 4 l +
+    // 2 (k % 2), + 1 (zero where the row has no such column).  Values stay outside
+    // of shared memory.
+    bool pairs = false;
     std::vector<TileInfo> tiles;
     std::vector<TileSlot> slots;
     std::vector<TileSlice> slices;
@@ -91,7 +100,9 @@ struct TilePlan {
 
 // Shared memory of one tile: values, patterns and the vectors of its local
 // vertices.
-size_t tile_smem_bytes(const TileInfo& t, int pat_stride, int value_bytes, int vectors, bool slot_rhs);
+size_t tile_smem_bytes(const TileInfo& t, int pat_stride, int value_bytes, int vectors, bool slot_rhs,
+                       bool pairs = false);
+constexpr int kPairEntries = 32;  // of a union at most: 64 values of a slice's pairs per lane
 
 // order_block > 0: a row sums its entries in the order [columns of its own block
 // of order_block rows][lower columns][higher columns], each part ascending;

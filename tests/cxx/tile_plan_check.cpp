@@ -73,7 +73,7 @@ static bool check(const HostTables& H, const TileLimits& L, int block) {
         if (T.nslice > P.rows_per_thread * P.threads / 32) FAIL("tile %zu: too many slices", t);
         TileInfo room = T;  // a cluster's vectors are laid out alike
         if (P.cluster) room.nloc = P.nloc_max;
-        smem = std::max(smem, tile_smem_bytes(room, P.pat_stride, L.value_bytes, P.vectors, L.slot_rhs));
+        smem = std::max(smem, tile_smem_bytes(room, P.pat_stride, L.value_bytes, P.vectors, L.slot_rhs, P.pairs));
         std::vector<int> at(T.nloc, -1);
         auto place = [&](int pos, int row) {
             if (pos < 0 || pos >= T.nloc || at[pos] != -1) return false;
@@ -84,6 +84,7 @@ static bool check(const HostTables& H, const TileLimits& L, int block) {
         for (int q = 0; q < T.nslice * 32; ++q) {
             const TileSlot& S = P.slots[T.slot0 + q];
             if (S.row >= 0 && !place(S.pos, S.row)) FAIL("tile %zu: place of row %d", t, S.row);
+            if (P.pairs && S.row < 0 && (S.pos < 0 || S.pos >= T.nloc)) FAIL("tile %zu: place of an empty lane", t);
         }
         for (int h = 0; h < T.nhalo; ++h) {
             const TileHalo& q = P.halo[T.halo0 + h];
@@ -101,26 +102,49 @@ static bool check(const HostTables& H, const TileLimits& L, int block) {
             if (!pub) FAIL("halo row %d not published", q.row);
         }
         for (int s = 0; s < T.nslice; ++s) {
-            const TileSlice& sc = P.slices[T.slice0 + s];
-            if (sc.len % 4 || sc.off % (32 * G) || sc.off + 32 * sc.len > T.nent) FAIL("slice range");
+            const int w = P.pairs ? s & 1 : 0;
+            const TileSlice& sc = P.slices[T.slice0 + s - w];
+            if (P.pairs && sc.len > kPairEntries) FAIL("tile %zu: union too long", t);
+            if (P.pairs ? sc.len % 4 || sc.off % 128 || sc.off + 64 * sc.len > T.nent : sc.len % 4 || sc.off % (32 * G) || sc.off + 32 * sc.len > T.nent) FAIL("slice range");
             for (int l = 0; l < 32; ++l) {
                 const TileSlot& S = P.slots[T.slot0 + 32 * s + l];
-                auto val = [&](int k) { return P.val[(size_t)T.ent0 + sc.off + 32 * G * (k / G) + G * l + k % G]; };
+                auto val = [&](int k) {
+                    if (P.pairs) return P.val[(size_t)T.ent0 + sc.off + 128 * (k / 2) + 4 * l + 2 * (k % 2) + w];
+                    return P.val[(size_t)T.ent0 + sc.off + 32 * G * (k / G) + G * l + k % G];
+                };
                 auto col = [&](int k) {
-                    const int p = S.pos + P.pat[((size_t)T.pat0) * P.pat_stride + S.pat + k];
+                    const int p = P.slots[T.slot0 + 32 * (s - w) + l].pos + P.pat[((size_t)T.pat0) * P.pat_stride + S.pat + k];
                     return p < 0 || p >= T.nloc ? -1 : at[p];
                 };
+                if (P.pairs)  // every lane reads within the tile, whatever it sums
+                    for (int k = 0; k < sc.len; ++k)
+                        if (col(k) < 0) FAIL("tile %zu: lane outside", t);
                 if (S.row < 0) continue;
                 const int r = S.row, b = H.nPtr[r], n = H.nPtr[r + 1] - b, ka = (S.pub >> 8) & 255, kb = (S.pub >> 16) & 255;
                 if (n > sc.len) FAIL("row %d cut", r);
-                for (int k = n; k < sc.len; ++k)
+                int ne = n;  // of the union: what either row of the pair has
+                if (P.pairs) {
+                    const int q = P.slots[T.slot0 + 32 * (s ^ 1) + l].row;
+                    std::set<int> cols(H.nCol.begin() + b, H.nCol.begin() + b + n);
+                    if (q >= 0) cols.insert(H.nCol.begin() + H.nPtr[q], H.nCol.begin() + H.nPtr[q + 1]);
+                    if (q >= 0 && (std::abs(q - r) != 1 || (block > 0 && q / block != r / block))) FAIL("row %d: pair", r);
+                    ne = (int)cols.size();
+                }
+                for (int k = ne; k < sc.len; ++k)
                     if (val(k) != 0.0 || col(k) < 0) FAIL("row %d padding", r);
                 // stored order: [0, ka) own block, [ka, kb) below, the rest above; in
                 // the order (ka..kb), (0..ka), (kb..) the columns ascend
                 std::vector<int> ord;
                 for (int k = ka; k < kb; ++k) ord.push_back(k);
                 for (int k = 0; k < ka; ++k) ord.push_back(k);
-                for (int k = kb; k < n; ++k) ord.push_back(k);
+                for (int k = kb; k < ne; ++k) ord.push_back(k);
+                if (P.pairs)  // the partner's own columns weigh nothing
+                    for (size_t q = ord.size(); q-- > 0;)
+                        if (!std::binary_search(H.nCol.begin() + b, H.nCol.begin() + b + n, col(ord[q]))) {
+                            if (val(ord[q]) != 0.0) FAIL("row %d: weight of its partner's column", r);
+                            ord.erase(ord.begin() + q);
+                        }
+                if ((int)ord.size() != n) FAIL("row %d: %d of %d entries", r, (int)ord.size(), n);
                 if (block == 0 && (ka || kb)) FAIL("row %d: parts without a block", r);
                 for (int k = 0; k < n; ++k) {
                     if (col(ord[k]) != H.nCol[b + k] || val(ord[k]) != H.nVal[b + k]) FAIL("row %d entry %d", r, k);
@@ -163,7 +187,7 @@ static bool check(const HostTables& H, const TileLimits& L, int block) {
 }
 
 int main() {
-    auto run = [](std::vector<ModelInput> ms, int block, int value_bytes, int cap, int cluster = 0) {
+    auto run = [](std::vector<ModelInput> ms, int block, int value_bytes, int cap, int cluster = 0, bool pairs = false) {
         HostTables H;
         const std::string e = build_host_tables(ms, -9.8, H);
         if (!e.empty()) {
@@ -183,6 +207,17 @@ int main() {
         }
         if (cap) L.group_cap = cap;
         L.cluster = cluster;
+        if (pairs) {  // as on four SMs
+            L.pairs = true;
+            L.sms = 4;
+            L.co_resident = 8;
+            TilePlan P;
+            build_tile_plan(H, L, block, P);
+            if (!P.ok || !P.pairs) {
+                printf("no pairs for %d rows\n", H.nsim);
+                return false;
+            }
+        }
         L.cluster_min = 320;
         L.cluster_rows = 272;
         return check(H, L, block);
@@ -199,6 +234,9 @@ int main() {
     for (int n : {18, 25, 33, 49, 65, 66}) ok = ok && run({grid(n, n, 0, false)}, 64, 4, 0, 16);
     ok = ok && run({grid(40, 31, 0, true)}, 64, 4, 0, 16) && run({grid(300, 3, 0, false)}, 0, 4, 0, 16);
     ok = ok && run({grid(20, 20, 0, false), grid(18, 40, 1, false), grid(7, 9, 2, true)}, 64, 4, 0, 16);
+    for (int n : {48, 57, 64, 80}) ok = ok && run({grid(n, n, 0, false)}, 0, 4, 0, 0, true) && run({grid(n, n, 0, false)}, 70, 4, 0, 0, true);
+    ok = ok && run({grid(41, 60, 0, false), grid(37, 33, 0, false), grid(20, 51, 0, false)}, 93, 4, 0, 0, true);
+    ok = ok && run({grid(64, 64, 0, false), grid(64, 64, 0, false), grid(64, 64, 0, false)}, 0, 4, 0, 0, true);  // launches
     if (ok) printf("ok\n");
     return ok ? 0 : 1;
 }

@@ -25,7 +25,7 @@ def _solve(sc, prec, **kw):
 
 
 # 18, 24, 65: the smallest cluster of tiles, one of eight, the largest; 66: past it; 224: past a component
-# per thread in FP64; 300: two tiles per SM; 430: with two rows per thread
+# per thread in FP64; 300: two tiles per SM; 430: with pairs of rows
 @pytest.mark.parametrize("prec,n", [(p, n) for p in ("fp32", "fp64") for n in (2, 18, 24, 65, 66, 224)] +
                          [("fp64", 300), ("fp32", 430), ("mixed", 18), ("mixed", 24), ("mixed", 65), ("mixed", 430)])
 def test_tiled_solve_against_one_launch_per_sweep(prec, n, built_lib):
@@ -51,6 +51,30 @@ def test_cluster_of_several_models(prec, built_lib):
     b, _ = _solve(sc, prec, instance_stop=1)
     assert t["pd_ctas"] <= 16
     assert np.array_equal(a, b)
+
+
+def test_large_meshes_with_and_without_pairs_of_rows(built_lib):
+    grids = scenes.batched(12, 100, 127, seed=6)  # odd row lengths: some rows have no partner
+    other = scenes.cloth_drop(380, 1, with_sphere=False, lg=2)  # numbered at random: none has
+    c = other.cloths[0]
+    new = np.random.default_rng(1).permutation(len(c.X))
+    X = np.empty_like(c.X)
+    X[new] = c.X
+    c.X, c.F, c.pins = X, new[c.F].astype(c.F.dtype), new[c.pins].astype(c.pins.dtype)
+    for sc in (grids, other):
+        a, t = _solve(sc, "fp32")
+        b, _ = _solve(sc, "fp32", persistent=0)
+        assert t["pd_rows_per_thread"] == 2 and t["pd_ctas"] > 152
+        assert np.array_equal(a, b)
+    # launches of groups, models that stop by themselves (FP32 contact sums of large
+    # batches depend on the order of their atomics: the mixed form)
+    one = pdipc.Simulator(grids, "mixed", instance_stop=1)
+    many = pdipc.Simulator(grids, "mixed", instance_stop=1, pd_group_ctas=one.tuning()["pd_ctas"] // 2)
+    assert many.tuning()["pd_launches"] > 1
+    for _ in range(2):
+        one.step(1)
+        many.step(1)
+        assert np.array_equal(one.positions(), many.positions())
 
 
 def test_tiled_groups_and_stopped_models_give_the_bits_of_one_launch(built_lib):
