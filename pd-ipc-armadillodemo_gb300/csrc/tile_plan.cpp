@@ -7,9 +7,13 @@
 #include "tile_plan.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
+#include <new>
 #include <numeric>
+#include <system_error>
+#include <thread>
 #include <unordered_map>
 
 namespace pdipc {
@@ -324,13 +328,11 @@ void try_plan(const HostTables& H, const TileLimits& lim, int order_block, bool 
         return order_block > 0 && u / order_block != v / order_block ? -1 : u;
     };
 
-    // ---- tables, tile by tile ----
-    std::vector<int> pos(ns, 0), ext, ent(patW);
-    int most = 0;
-    size_t most3 = 0;
+    // ---- tables, tile by tile, each by itself (several threads), then joined ----
     const int G = 16 / lim.value_bytes;
-    std::vector<int16_t> o(P.pat_stride);
-    for (int t = 0; t < nt; ++t) {
+    auto build = [&](int t, std::vector<int>& pos, TilePlan& Q) -> bool {
+        std::vector<int> ext, ent(patW);
+        std::vector<int16_t> o(P.pat_stride);
         TileInfo T{};
         auto order = [&](int a, int b) { return cls[a] != cls[b] ? cls[a] < cls[b] : a < b; };
         ext = own[t];
@@ -338,7 +340,7 @@ void try_plan(const HostTables& H, const TileLimits& lim, int order_block, bool 
         std::sort(ext.begin(), ext.end(), order);
         for (size_t q = 0; q < ext.size(); ++q) pos[ext[q]] = (int)q;
         T.nloc = (int)ext.size();
-        if (T.nloc > 32767) return;
+        if (T.nloc > 32767) return false;
         // slices: runs of own rows of one parity; kept within 32 consecutive
         // places of the local vectors (no two lanes in one bank) when that
         // costs at most 15% more slices
@@ -365,24 +367,23 @@ void try_plan(const HostTables& H, const TileLimits& lim, int order_block, bool 
                 beg = b;
             }
         }
-        if ((int)beg.size() * per > max_slices) return;
-        most = std::max(most, (int)beg.size() * per);
+        if ((int)beg.size() * per > max_slices) return false;
         T.model = tileModel[t];
         T.nslice = (int)beg.size() * per;
-        T.slot0 = (int)P.slots.size();
-        T.slice0 = (int)P.slices.size();
-        T.ent0 = (int)P.val.size();
-        T.pat0 = (int)(P.pat.size() / P.pat_stride);
+        T.slot0 = (int)Q.slots.size();
+        T.slice0 = (int)Q.slices.size();
+        T.ent0 = (int)Q.val.size();
+        T.pat0 = (int)(Q.pat.size() / P.pat_stride);
         std::unordered_map<uint64_t, std::vector<int>> seen;  // hash of the offsets -> pattern ids
         int npat = 0;
         auto pattern = [&]() {  // of the offsets o
             uint64_t h = 1469598103934665603ull;
             for (int16_t v : o) h = (h ^ (uint16_t)v) * 1099511628211ull;
             for (int c : seen[h])
-                if (std::memcmp(&P.pat[(size_t)(T.pat0 + c) * P.pat_stride], o.data(), sizeof(int16_t) * P.pat_stride) == 0)
+                if (std::memcmp(&Q.pat[(size_t)(T.pat0 + c) * P.pat_stride], o.data(), sizeof(int16_t) * P.pat_stride) == 0)
                     return c;
             seen[h].push_back(npat);
-            P.pat.insert(P.pat.end(), o.begin(), o.end());
+            Q.pat.insert(Q.pat.end(), o.begin(), o.end());
             return npat++;
         };
         // entry e's part in the order of row r's sum: own block, below it, above it
@@ -393,7 +394,7 @@ void try_plan(const HostTables& H, const TileLimits& lim, int order_block, bool 
         };
         for (int s = 0; s < (int)beg.size(); ++s) {
             const int q0 = beg[s], q1 = s + 1 < (int)beg.size() ? beg[s + 1] : (int)rows.size();
-            const size_t base = P.val.size();
+            const size_t base = Q.val.size();
             if (P.pairs) {
                 std::vector<TileSlot> second(kLanes, TileSlot{-1, 0, 0, 0});
                 std::vector<double> v(2 * kPairEntries * kLanes, 0.0);  // by entry, lane, row
@@ -401,7 +402,7 @@ void try_plan(const HostTables& H, const TileLimits& lim, int order_block, bool 
                 TileSlot last{-1, 0, 0, 0};
                 for (int lane = 0; lane < kLanes; ++lane) {
                     if (q0 + lane >= q1) {  // an empty lane sums zeros at valid places
-                        P.slots.push_back(last);
+                        Q.slots.push_back(last);
                         second[lane] = last;
                         continue;
                     }
@@ -428,7 +429,7 @@ void try_plan(const HostTables& H, const TileLimits& lim, int order_block, bool 
                             m[n++] = m[q];
                         }
                     }
-                    if (n > kPairEntries) return;
+                    if (n > kPairEntries) return false;
                     for (int k = 0; k < n; ++k) {
                         ka += order_block > 0 && m[k].part == 0;
                         kb += order_block > 0 && m[k].part < 2;
@@ -438,28 +439,28 @@ void try_plan(const HostTables& H, const TileLimits& lim, int order_block, bool 
                     for (int k = 0; k < P.pat_stride; ++k)
                         o[k] = n > 0 ? (int16_t)(pos[m[std::min(k, n - 1)].col] - pos[r]) : (int16_t)0;
                     const int pat = pattern() * P.pat_stride, parts = (ka << 8) | (kb << 16);
-                    P.slots.push_back(TileSlot{r, pos[r], pat, pub[r] | parts});
+                    Q.slots.push_back(TileSlot{r, pos[r], pat, pub[r] | parts});
                     last = TileSlot{-1, pos[r], pat, parts};
                     second[lane] = u < 0 ? last : TileSlot{u, pos[u], pat, pub[u] | parts};
                 }
-                P.slots.insert(P.slots.end(), second.begin(), second.end());
+                Q.slots.insert(Q.slots.end(), second.begin(), second.end());
                 len = (len + 3) / 4 * 4;
-                P.slices.push_back(TileSlice{(int)(base - T.ent0), len});
-                P.slices.push_back(TileSlice{(int)(base - T.ent0), 0});
-                P.val.resize(base + 2 * (size_t)len * kLanes);
+                Q.slices.push_back(TileSlice{(int)(base - T.ent0), len});
+                Q.slices.push_back(TileSlice{(int)(base - T.ent0), 0});
+                Q.val.resize(base + 2 * (size_t)len * kLanes);
                 for (int k = 0; k < len; ++k)
                     for (int q = 0; q < 2 * kLanes; ++q)
-                        P.val[base + 128 * (size_t)(k / 2) + 4 * (q / 2) + 2 * (k % 2) + q % 2] = v[2 * kLanes * (size_t)k + q];
+                        Q.val[base + 128 * (size_t)(k / 2) + 4 * (q / 2) + 2 * (k % 2) + q % 2] = v[2 * kLanes * (size_t)k + q];
                 continue;
             }
             int len = 0;
             for (int q = q0; q < q1; ++q) len = std::max(len, H.nPtr[rows[q] + 1] - H.nPtr[rows[q]]);
             len = (len + 3) / 4 * 4;
-            P.slices.push_back(TileSlice{(int)(base - T.ent0), len});
-            P.val.resize(base + (size_t)len * kLanes, 0.0);
+            Q.slices.push_back(TileSlice{(int)(base - T.ent0), len});
+            Q.val.resize(base + (size_t)len * kLanes, 0.0);
             for (int lane = 0; lane < kLanes; ++lane) {
                 if (q0 + lane >= q1) {
-                    P.slots.push_back(TileSlot{-1, 0, 0, 0});
+                    Q.slots.push_back(TileSlot{-1, 0, 0, 0});
                     continue;
                 }
                 const int r = rows[q0 + lane], b = H.nPtr[r], n = H.nPtr[r + 1] - b;
@@ -475,51 +476,109 @@ void try_plan(const HostTables& H, const TileLimits& lim, int order_block, bool 
                 std::fill(o.begin(), o.end(), (int16_t)0);
                 for (int k = 0; k < P.pat_stride; ++k)
                     o[k] = n > 0 ? (int16_t)(pos[H.nCol[ent[std::min(k, n - 1)]]] - pos[r]) : (int16_t)0;
-                for (int k = 0; k < n; ++k) P.val[base + (size_t)kLanes * G * (k / G) + (size_t)G * lane + k % G] = H.nVal[ent[k]];
-                P.slots.push_back(TileSlot{r, pos[r], pattern() * P.pat_stride, pub[r] | (ka << 8) | (kb << 16)});
+                for (int k = 0; k < n; ++k) Q.val[base + (size_t)kLanes * G * (k / G) + (size_t)G * lane + k % G] = H.nVal[ent[k]];
+                Q.slots.push_back(TileSlot{r, pos[r], pattern() * P.pat_stride, pub[r] | (ka << 8) | (kb << 16)});
             }
         }
         for (int s = 0; s < T.nslice; ++s) {
-            TileSlot* sl = &P.slots[T.slot0 + (size_t)kLanes * s];
+            TileSlot* sl = &Q.slots[T.slot0 + (size_t)kLanes * s];
             int len = 0;
             for (int lane = 0; lane < kLanes; ++lane)
                 if (sl[lane].row >= 0) len = std::max(len, H.lPtr[sl[lane].row + 1] - H.lPtr[sl[lane].row] - 1);
-            const size_t base = P.st_pos.size(), n = base + (size_t)len * kLanes;
-            P.stencil.push_back((int)base);
-            P.st_pos.resize(n, 0);
-            P.st_rest.resize(n, 0.0);
-            P.st_lbo.resize(n, 0.0);
-            P.st_bend.resize(n, 0.0);
+            const size_t base = Q.st_pos.size(), n = base + (size_t)len * kLanes;
+            Q.stencil.push_back((int)base);
+            Q.st_pos.resize(n, 0);
+            Q.st_rest.resize(n, 0.0);
+            Q.st_lbo.resize(n, 0.0);
+            Q.st_bend.resize(n, 0.0);
             for (int lane = 0; lane < kLanes; ++lane) {
                 const int r = sl[lane].row;
                 if (r < 0) continue;
                 const int nst = H.lPtr[r + 1] - H.lPtr[r] - 1;
-                if (nst > 127) return;
+                if (nst > 127) return false;
                 sl[lane].pub |= nst << 24;
                 for (int e = H.lPtr[r] + 1, k = 0; e < H.lPtr[r + 1]; ++e, ++k) {
                     const size_t q = base + (size_t)kLanes * k + lane;
-                    P.st_pos[q] = (int16_t)(pos[H.lNbr[e]] - pos[r]);
-                    P.st_rest[q] = H.lRest[e];
-                    P.st_lbo[q] = H.lLbo[e];
-                    P.st_bend[q] = H.lBendT[e];
+                    Q.st_pos[q] = (int16_t)(pos[H.lNbr[e]] - pos[r]);
+                    Q.st_rest[q] = H.lRest[e];
+                    Q.st_lbo[q] = H.lLbo[e];
+                    Q.st_bend[q] = H.lBendT[e];
                 }
             }
         }
         T.npat = npat;
-        T.nent = (int)P.val.size() - T.ent0;
-        if (T.nent >= 1 << 20 || npat * P.pat_stride > 65535) return;  // packed in the kernel
-        T.halo0 = (int)P.halo.size();
+        T.nent = (int)Q.val.size() - T.ent0;
+        if (T.nent >= 1 << 20 || npat * P.pat_stride > 65535) return false;  // packed in the kernel
+        T.halo0 = (int)Q.halo.size();
         T.nhalo = (int)halo[t].size();
         std::sort(halo[t].begin(), halo[t].end());
-        for (int c : halo[t]) P.halo.push_back(TileHalo{c, pos[c]});
-        T.nbr0 = (int)P.nbr.size();
+        for (int c : halo[t]) Q.halo.push_back(TileHalo{c, pos[c]});
+        T.nbr0 = (int)Q.nbr.size();
         T.nnbr = (int)nbr[t].size();
-        P.nbr.insert(P.nbr.end(), nbr[t].begin(), nbr[t].end());
-        T.tet0 = (int)P.tet.size();
+        Q.nbr.insert(Q.nbr.end(), nbr[t].begin(), nbr[t].end());
+        T.tet0 = (int)Q.tet.size();
         if (H.ntet > 0) {
             T.ntet = (int)tetsOf[t].size();
-            P.tet.insert(P.tet.end(), tetsOf[t].begin(), tetsOf[t].end());
+            Q.tet.insert(Q.tet.end(), tetsOf[t].begin(), tetsOf[t].end());
         }
+        Q.tiles.push_back(T);
+        return true;
+    };
+    std::vector<TilePlan> piece(nt);
+    {
+        std::atomic<int> next{0};
+        std::atomic<bool> ok{true};
+        auto work = [&]() {
+            try {
+                std::vector<int> pos(ns, 0);
+                for (int t; ok && (t = next++) < nt;)
+                    if (!build(t, pos, piece[t])) ok = false;
+            } catch (const std::bad_alloc&) {  // no plan
+                ok = false;
+            }
+        };
+        std::vector<std::thread> team;
+        for (int k = std::min({nt / 16, 7, (int)std::thread::hardware_concurrency() - 1}); k > 0; --k) {
+            try {
+                team.emplace_back(work);
+            } catch (const std::system_error&) {
+                break;  // fewer threads
+            }
+        }
+        work();
+        for (std::thread& th : team) th.join();
+        if (!ok) return;
+    }
+    int most = 0;
+    size_t most3 = 0;
+    for (TilePlan& Q : piece) {
+        TileInfo T = Q.tiles[0];
+        T.slot0 = (int)P.slots.size();
+        T.slice0 = (int)P.slices.size();
+        T.ent0 = (int)P.val.size();
+        T.pat0 = (int)(P.pat.size() / P.pat_stride);
+        T.halo0 = (int)P.halo.size();
+        T.nbr0 = (int)P.nbr.size();
+        T.tet0 = (int)P.tet.size();
+        for (int& q : Q.stencil) q += (int)P.st_pos.size();
+        auto join = [](auto& to, auto& from) {
+            to.insert(to.end(), from.begin(), from.end());
+            from.clear();
+            from.shrink_to_fit();
+        };
+        join(P.slots, Q.slots);
+        join(P.slices, Q.slices);
+        join(P.val, Q.val);
+        join(P.pat, Q.pat);
+        join(P.stencil, Q.stencil);
+        join(P.st_pos, Q.st_pos);
+        join(P.st_rest, Q.st_rest);
+        join(P.st_lbo, Q.st_lbo);
+        join(P.st_bend, Q.st_bend);
+        join(P.halo, Q.halo);
+        join(P.nbr, Q.nbr);
+        join(P.tet, Q.tet);
+        most = std::max(most, T.nslice);
         const size_t sm = tile_smem_bytes(T, P.pat_stride, lim.value_bytes, 2, lim.slot_rhs, P.pairs);
         if (lim.vectors > 2)
             most3 = std::max(most3,
