@@ -433,6 +433,7 @@ __global__ void __launch_bounds__(kTileMaxWarps * (kForm == kPairs ? 64 : 32), k
         }
     };
     const T w = a.relax, om1 = T(1) - a.relax;
+    const bool kept_first = kCorr && (kCl || a.keptFirst);  // known in a cluster, whose sweeps it would lengthen by 3%
 
     // ---- positions of the local vertices: own rows and halo ----
     auto load_pos = [&](int row, int pos) {
@@ -754,9 +755,9 @@ __global__ void __launch_bounds__(kTileMaxWarps * (kForm == kPairs ? 64 : 32), k
                     sum_of(r, cur, ps, s0, s1, s2);
                     own(cur, r, c0, c1, c2);
                 }
-                y[r][0] = jacobi<kCorr>(om1, c0, w, s0, rh[r][0], id[r]);
-                y[r][1] = jacobi<kCorr>(om1, c1, w, s1, rh[r][1], id[r]);
-                y[r][2] = jacobi<kCorr>(om1, c2, w, s2, rh[r][2], id[r]);
+                y[r][0] = jacobi(om1, c0, w, s0, rh[r][0], id[r], kept_first);
+                y[r][1] = jacobi(om1, c1, w, s1, rh[r][1], id[r], kept_first);
+                y[r][2] = jacobi(om1, c2, w, s2, rh[r][2], id[r], kept_first);
                 if (!kCl && pub(r)) publish(0, row(r), y[r][0], y[r][1], y[r][2]);
             }
             // the curvature vectors (direct form), or the positions, have been read
@@ -783,9 +784,9 @@ __global__ void __launch_bounds__(kTileMaxWarps * (kForm == kPairs ? 64 : 32), k
                 sum_of(r, cur, ps, s0, s1, s2);
                 T c0, c1, c2;
                 own(cur, r, c0, c1, c2);
-                n[0] = jacobi<kCorr>(om1, c0, w, s0, rh[r][0], id[r]);
-                n[1] = jacobi<kCorr>(om1, c1, w, s1, rh[r][1], id[r]);
-                n[2] = jacobi<kCorr>(om1, c2, w, s2, rh[r][2], id[r]);
+                n[0] = jacobi(om1, c0, w, s0, rh[r][0], id[r], kept_first);
+                n[1] = jacobi(om1, c1, w, s1, rh[r][1], id[r], kept_first);
+                n[2] = jacobi(om1, c2, w, s2, rh[r][2], id[r], kept_first);
                 if (it > 0) {
                     n[0] = fma_(om, add_(n[0], -px[r][0]), px[r][0]);
                     n[1] = fma_(om, add_(n[1], -px[r][1]), px[r][1]);
@@ -819,9 +820,9 @@ __global__ void __launch_bounds__(kTileMaxWarps * (kForm == kPairs ? 64 : 32), k
                 sum_of(r, cur, ps, s0, s1, s2);
                 T c0, c1, c2;
                 own(cur, r, c0, c1, c2);
-                const T y0 = jacobi<kCorr>(om1, c0, w, s0, rh[r][0], id[r]);
-                const T y1 = jacobi<kCorr>(om1, c1, w, s1, rh[r][1], id[r]);
-                const T y2 = jacobi<kCorr>(om1, c2, w, s2, rh[r][2], id[r]);
+                const T y0 = jacobi(om1, c0, w, s0, rh[r][0], id[r], kept_first);
+                const T y1 = jacobi(om1, c1, w, s1, rh[r][1], id[r], kept_first);
+                const T y2 = jacobi(om1, c2, w, s2, rh[r][2], id[r], kept_first);
                 if (!live(r)) continue;
                 send(0, cur ^ 1, r, y0, y1, y2);
                 put(cur ^ 1, lp(r), y0, y1, y2);

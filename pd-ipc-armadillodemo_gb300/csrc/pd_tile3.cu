@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(kTile3Warps * 96, 1) k_pd_tile3(const __grid_c
         __syncthreads();  // the right-hand sides are there, and the curvature vectors have been read
         if (row >= 0) {
             rh = srhs[comp * nslot + 32 * warp + lane];
-            y = jacobi<false>(om1, plane(cur, comp)[pos], w, y, rh, id);
+            y = jacobi(om1, plane(cur, comp)[pos], w, y, rh, id, false);
             if (pub) publish(comp, row, y);
             plane(cur ^ 1, comp)[pos] = y;
         }
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(kTile3Warps * 96, 1) k_pd_tile3(const __grid_c
             const bool last = it == a.cheby - 1;
             const F om = a.omega[it];
             ++tag;
-            F n = jacobi<false>(om1, plane(cur, comp)[pos], w, row_sum(cur), rh, id);
+            F n = jacobi(om1, plane(cur, comp)[pos], w, row_sum(cur), rh, id, false);
             if (it > 0) n = fma_(om, add_(n, -px), px);
             px = plane(cur ^ 1, comp)[pos];  // still this row's current x
             if (row >= 0) {
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(kTile3Warps * 96, 1) k_pd_tile3(const __grid_c
             if (last) break;
             if (!arrive(cur)) return;
             ++tag;
-            const F v = jacobi<false>(om1, plane(cur, comp)[pos], w, row_sum(cur), rh, id);
+            const F v = jacobi(om1, plane(cur, comp)[pos], w, row_sum(cur), rh, id, false);
             if (row >= 0) {
                 if (pub) publish(comp, row, v);
                 plane(cur ^ 1, comp)[pos] = v;

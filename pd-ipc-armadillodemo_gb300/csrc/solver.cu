@@ -1441,7 +1441,7 @@ private:
             tile_on_ = tile_.ok;
             return PDIPC_OK;
         }
-        if constexpr (!std::is_same<T, float>::value) return plan_tiles(H, 0, err);
+        if constexpr (!std::is_same<T, float>::value) return plan_tiles(H, 0, false, err);
         Dev<T, TC>& d = d_;
         const int ns = d.nsim;
         int dev = 0, nsm = 0, smem_optin = 0, coop = 0;
@@ -1602,7 +1602,10 @@ private:
         };
         const int group_cap = prm_.pd_group_ctas > 0 ? prm_.pd_group_ctas : INT_MAX;
         std::vector<Cand> cands;
-        int order_block = -1;  // the default configuration's rows per CTA on the band path (whatever the launches)
+        // the default configuration's rows per CTA on the band path (whatever the
+        // launches), and which product of a sweep's update it rounds (jacobi, tile_device.cuh)
+        int order_block = -1;
+        bool kept_first = false;
         const bool dflt_l1 = prm_.persistent != 2, dflt_ls = prm_.persistent != 3;
         for (int pass = 0; pass < 2; ++pass) {
             const bool smem_mat = pass == 0 && fits16;
@@ -1652,8 +1655,10 @@ private:
                     PD_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, c.threads, c.sm));
                     if (per_sm < 1) continue;
                     if (order_block < 0 && c.ch.l1_gather == dflt_l1 && c.ch.local_sync == dflt_ls &&
-                        form_groups(c.spc, c.ctas, per_sm * nsm, c.groups))
+                        form_groups(c.spc, c.ctas, per_sm * nsm, c.groups)) {
                         order_block = c.ch.band ? c.spc * kSlice : 0;
+                        kept_first = c.ch.band && R == 1;
+                    }
                     if (!form_groups(c.spc, c.ctas, std::min(per_sm * nsm, group_cap), c.groups)) continue;
                     cands.push_back(std::move(c));
                 }
@@ -1676,7 +1681,7 @@ private:
         if (!force && prm_.persistent == 1) {
             // compact tiles where a partition fits; a row sums in the order of
             // the configuration they stand in for, so the results keep its bits
-            pdipc_status r = plan_tiles(H, std::max(order_block, 0), err);
+            pdipc_status r = plan_tiles(H, std::max(order_block, 0), kept_first, err);
             if (r != PDIPC_OK || tile_on_) return r;
         }
         if (!pick) return PDIPC_OK;
@@ -1920,10 +1925,11 @@ private:
         return PDIPC_OK;
     }
 
-    // The tile partition and its tables (order_block: build_tile_plan), built
+    // The tile partition and its tables (order_block: build_tile_plan; kept_first:
+    // jacobi in tile_device.cuh), built
     // once per context; leaves tile_on_ false when no partition fits.  The FP64
     // form is built for cloths under the scene's own stopping rule.
-    pdipc_status plan_tiles(const HostTables& H, int order_block, std::string& err) {
+    pdipc_status plan_tiles(const HostTables& H, int order_block, bool kept_first, std::string& err) {
         constexpr bool fp64 = std::is_same<T, double>::value;
         if (prm_.persistent != 1 || H.nsim == 0 || (fp64 && (H.ntet > 0 || prm_.instance_stop))) return PDIPC_OK;
         int dev = 0, nsm = 0, coop = 0, sm_smem = 0, reserved = 0;
@@ -1950,7 +1956,8 @@ private:
             if (prm_.pd_group_ctas > 0) lim.group_cap = prm_.pd_group_ctas;
             // all tiles in one launch, none of which leaves early: the barriers of a
             // cluster wait for all
-            if (!fp64 && H.ntet == 0 && !prm_.instance_stop && lim.group_cap >= kTileCluster) {
+            if (!fp64 && H.ntet == 0 && !prm_.instance_stop && lim.group_cap >= kTileCluster &&
+                (!kCorrection || kept_first)) {
                 lim.cluster = kTileCluster;
                 lim.cluster_min = kTileClusterMin;
                 lim.cluster_rows = kTileClusterRows;
@@ -2073,6 +2080,7 @@ private:
         a.instStop = prm_.instance_stop ? d.InstStop : nullptr;
         a.tape = nullptr;
         a.third = tile_.vectors > 2;
+        a.keptFirst = kept_first;
         a.partSmem = (int)tile_.smem_bytes;
         tile_on_ = true;
         return PDIPC_OK;

@@ -100,6 +100,7 @@ struct TileArgs {
     const int4* push;          // cluster: the readers of every slot's row (TilePlan::push)
     int nlocMax;               // cluster: places of each vector
     int third;                 // correction form: the tiles hold a third vector
+    int keptFirst;             // correction form: which product of a sweep's update is rounded (jacobi)
 };
 
 // Words of one vertex in a phase: the correction form publishes the two halves

@@ -121,11 +121,12 @@ __device__ __forceinline__ float mul_(float a, float b) { return __fmul_rn(a, b)
 __device__ __forceinline__ double mul_(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float add_(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double add_(double a, double b) { return __dadd_rn(a, b); }
-// (1 - w) c + w ((s + b) / D): one weighted-Jacobi update
-template <bool kCorr, typename T>
-__device__ __forceinline__ T jacobi(T om1, T c, T w, T s, T b, T id) {
+// (1 - w) c + w ((s + b) / D): one weighted-Jacobi update; which of the two products
+// is rounded by itself: the second, or the first (kept_first)
+template <typename T>
+__device__ __forceinline__ T jacobi(T om1, T c, T w, T s, T b, T id, bool kept_first) {
     const T t = mul_(add_(s, b), id);
-    return kCorr ? fma_(w, t, mul_(om1, c)) : fma_(om1, c, mul_(w, t));
+    return fma_(kept_first ? w : om1, kept_first ? t : c, mul_(kept_first ? om1 : w, kept_first ? c : t));
 }
 template <typename T>
 __device__ __forceinline__ T norm2(T x, T y, T z) {
