@@ -260,7 +260,7 @@ def measured_peak_hbm():
 def profiled_traffic(prec: str):
     """DRAM bytes per launch of the persistent PD solve from the committed ncu
     summary, if present."""
-    p = os.path.join(ROOT, "profiles", f"pd_persistent_c1_{prec}.md")
+    p = os.path.join(ROOT, "profiles", f"pd_tile_c1_{prec}.md")
     try:
         for ln in open(p):
             if ln.startswith("traffic_bytes_per_launch:"):
@@ -520,9 +520,9 @@ def run_ours(args):
     sweep_gbs = sweep_bytes / (sweep_ms * 1e-3) / 1e9
     local_ms, local_bytes = sim.local_timing(400)
     local_gbs = local_bytes / (local_ms * 1e-3) / 1e9
-    pd_kernel = {3: "k_pd_persistent (cooperative, matrix values and the iterate's band in shared memory, "
-                    "halo by bulk copies)",
-                 2: "k_pd_persistent (cooperative, matrix values in shared memory)",
+    pd_kernel = {3: "k_pd_tile (cooperative, compact tiles of rows: matrix values and the iterate on chip, boundary "
+                    "rows exchanged as tagged words; k_pd_persistent where no tiling fits)",
+                 2: "k_pd_tile or k_pd_tile3 (the same, direct form; k_pd_persistent where no tiling fits)",
                  1: "k_pd_persistent (cooperative, matrix from L2)",
                  0: "PD solve as a CUDA graph of per-sweep kernels"}[st_end["pd_path"]]
     state_bytes = 16 if args.precision == "fp32" else 32

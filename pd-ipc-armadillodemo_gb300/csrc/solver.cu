@@ -1984,6 +1984,10 @@ private:
             }
             for (const TileGroup& g : tile_.groups)
                 if (g.hi - g.lo + 1 > held) tile_.ok = false;
+            // FP64 rows beyond one launch: a launch per sweep fills the chip better than
+            // groups of tiles (four 256x256: 7.4 ms per solve of 5 local-global
+            // iterations, 12.4 in four groups; 40 cloths 6.3, 8.0 in two)
+            if (fp64 && (int)tile_.tiles.size() > held) tile_.ok = false;
             if (tile_.ok) break;
         }
         if (!tile_.ok) return PDIPC_OK;

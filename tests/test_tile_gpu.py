@@ -66,6 +66,7 @@ def test_large_meshes_with_and_without_pairs_of_rows(built_lib):
         b, _ = _solve(sc, "fp32", persistent=0)
         assert t["pd_rows_per_thread"] == 2 and t["pd_ctas"] > 152
         assert np.array_equal(a, b)
+    assert pdipc.Simulator(grids, "fp64").tuning()["pd_rows_per_thread"] == 0  # more rows than one launch holds
     # launches of groups, models that stop by themselves (FP32 contact sums of large
     # batches depend on the order of their atomics: the mixed form)
     one = pdipc.Simulator(grids, "mixed", instance_stop=1)
