@@ -81,16 +81,17 @@ typedef struct {
     int device;              /* CUDA device ordinal */
     int rebuild_bvh;         /* 0: build the patch BVH once at initialize and refit per step
                                 (reference behaviour, cpp:1296-1320); 1: rebuild every step */
-    int persistent;          /* FP32/mixed PD solve of an outer iteration as one cooperative launch when
-                                the mesh allows it (matrix slice per CTA): 1 CTAs wait only for the CTAs
-                                they exchange rows with; in mixed precision the CTA's column band of the
-                                iterate lives in shared memory when it fits and each sweep sums the
-                                entries on the CTA's own rows while the neighbours' rows are copied in
-                                (else, and in FP32, gathers through L1); 2 neighbour waits, L2-only
+    int persistent;          /* PD solve of an outer iteration as one launch when the mesh allows it: 1 over
+                                compact tiles of rows that exchange their boundary rows (also FP64 cloths
+                                under the scene's own stopping rule, while one launch holds them); where no
+                                tiling fits, FP32 and mixed run row blocks that wait only for the blocks
+                                they exchange rows with, in mixed precision with the block's column band of
+                                the iterate in shared memory when it fits.  The others are row blocks, FP32
+                                and mixed only: 2 neighbour waits, L2-only
                                 gathers; 3 grid-wide barriers, gathers through L1; 4 neighbour waits,
                                 gathers through L1 (no band); 0 one launch per sweep */
-    int wait_limit_us;       /* limit of every device-side wait of the persistent solve (neighbour flags,
-                                grid barrier, halo copies), in microseconds at the maximum SM clock; past
+    int wait_limit_us;       /* limit of every device-side wait of the persistent solve (exchanged rows,
+                                neighbour flags, grid barrier, halo copies), in microseconds at the maximum SM clock; past
                                 it the launch ends and the step returns PDIPC_ERR_CUDA; 0 = 2 s.  The
                                 reference has no device-side waits (one launch per kernel). */
     int autotune;            /* 1: choose launch shapes by timing candidates at pdipc_initialize (see
@@ -109,9 +110,10 @@ typedef struct {
                                 that touch one another should keep 0.  A stopped model's rows leave the
                                 persistent PD solve (its CTAs return at entry when all their rows have
                                 stopped). */
-    int pd_group_ctas;       /* persistent PD solve: at most this many CTAs per launch (0: every CTA the
-                                device holds at once).  A plan with more CTAs runs as one launch per group
-                                of whole models (models share no matrix entry), in order. */
+    int pd_group_ctas;       /* persistent PD solve: at most this many tiles or CTAs per launch (0: as many as
+                                the device holds at once).  A plan with more runs as one launch per group of
+                                whole models (models share no matrix entry), in order; FP64 beyond what one
+                                launch holds runs one launch per sweep. */
     int reserved[1];
 } pdipc_params;
 
@@ -136,9 +138,10 @@ typedef struct {
     double device_ms;            /* device time of the last pdipc_step call: CUDA events recorded on the
                                     context's stream around every step, summed */
     int32_t pd_path;             /* 0: one launch per sweep; 1: persistent, matrix from L2;
-                                    2: persistent, matrix values in shared memory; 3: persistent,
-                                    matrix values and the iterate's band in shared memory */
-    int32_t pd_ctas;             /* CTAs of the persistent solve (0 if not used) */
+                                    2: persistent, matrix values on chip (FP32 and FP64 tiles, row blocks);
+                                    3: persistent, matrix values and the iterate on chip (mixed tiles, row
+                                    blocks with the band) */
+    int32_t pd_ctas;             /* tiles or CTAs of the persistent solve (0 if not used) */
     int64_t pd_solves;           /* projective-dynamics solves (one per outer iteration) in the last call */
     double pd_solve_ms;          /* their device time: CUDA events on the context's stream around each solve */
     double pd_solve_bytes;       /* algorithmic bytes of one solve: per vertex i and local-global iteration,
@@ -164,7 +167,7 @@ typedef struct {
     int32_t from_cache;         /* 1: taken from an earlier context of the same shape in this process */
     int32_t pd_rows_per_thread; /* persistent PD solve: rows per thread (slices per warp); 0: one launch
                                    per sweep */
-    int32_t pd_ctas;            /* CTAs of the persistent solve */
+    int32_t pd_ctas;            /* tiles or CTAs of the persistent solve */
     int32_t pd_band;            /* 1: the iterate's column band in shared memory */
     int32_t pd_l1_gather;       /* 1: gathers through L1 */
     int32_t pd_local_sync;      /* 1: neighbour waits, 0: grid barriers */
