@@ -96,7 +96,7 @@ __device__ __noinline__ void tile_tet(int e, const int4* __restrict__ Tets, cons
 enum TileForm { kWords, kCluster, kPairs };
 
 template <typename T, typename S, bool kCorr, bool kTets, int R, TileForm kForm>
-__global__ void __launch_bounds__(kTileMaxWarps * (kForm == kPairs ? 64 : 32), kForm == kPairs ? 1 : 2)
+__global__ void __launch_bounds__(kTileMaxWarps * (kForm == kPairs ? 64 : 32), kForm == kWords ? 2 : 1)
     k_pd_tile(const __grid_constant__ TileArgs<T, S> a) {
     constexpr int kW = kTileWords<T, S>;
     constexpr int kG = kTileGroup<T>;

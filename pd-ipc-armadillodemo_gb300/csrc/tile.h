@@ -122,9 +122,11 @@ cudaError_t launch_pd_tile(const TileArgs<T, S>& args, int tiles, int rows_per_t
 // The tiles as one thread-block cluster (FP32 arithmetic, a row per thread): a
 // thread writes its new vector into the shared memory of the tiles that read it,
 // and the cluster's barrier ends the sweep, in place of words in global memory that
-// the readers poll.  One solve of 10 x (local step + 30 sweeps), mixed, words ->
-// cluster: 20x20 0.50 -> 0.37 ms, 32x32 0.46 -> 0.36, 48x48 0.49 -> 0.44,
-// 64x64 0.50 -> 0.42; FP32 0.42 -> 0.33, 0.39 -> 0.33, 0.45 -> 0.38, 0.46 -> 0.37.
+// the readers poll; one CTA per SM, so a thread takes 120 registers (20x20 0.377 ->
+// 0.352 ms, 64x64 0.437 -> 0.428; the words' kernels are no faster with more than
+// 72).  One solve of 10 x (local step + 30 sweeps), mixed, words -> cluster: 20x20
+// 0.50 -> 0.35 ms, 32x32 0.46 -> 0.36, 48x48 0.49 -> 0.44, 64x64 0.50 -> 0.43; FP32
+// 0.42 -> 0.31, 0.39 -> 0.31, 0.45 -> 0.37, 0.46 -> 0.38.
 // Up to kTileClusterMin rows one tile alone is as fast (16x16 0.340 ms, 0.344 in a
 // cluster; FP32 0.285, 0.307); beyond kTileClusterRows rows per CTA the sums of so
 // few SMs cost more than the words of many (66x66: 0.550, 0.552 in a cluster).  With
