@@ -1411,15 +1411,20 @@ struct Sim {
         TC w_aiji = dot3(d, tmp);
         cross3(xai, xba, tmp);
         TC w_aiba = dot3(d, tmp);
+        // the reference leaves the weights unset where none names a side (parallel and
+        // degenerate edges): there, the closest of the four ends
+        *r = 0;
+        *s = 0;
+        const bool all = w_aiji >= 0 && w_aiji <= nn && w_aiba >= 0 && w_aiba <= nn;
         if (nn > (TC)1e-24f && w_aiji >= 0 && w_aiji <= nn && w_aiba >= 0 && w_aiba <= nn) {
             *r = w_aiba / nn;
             *s = w_aiji / nn;
         } else {
             TC best = (TC)999999999, dd, v, nd[3];
-            if (w_aiba < 0 && ((dd = vtx_edge_sq(xi, xa, xb, &v, nd)) < best)) { best = dd; *r = 0; *s = v; }
-            if (w_aiba > nn && ((dd = vtx_edge_sq(xj, xa, xb, &v, nd)) < best)) { best = dd; *r = 1; *s = v; }
-            if (w_aiji < 0 && ((dd = vtx_edge_sq(xa, xi, xj, &v, nd)) < best)) { best = dd; *r = v; *s = 0; }
-            if (w_aiji > nn && ((dd = vtx_edge_sq(xb, xi, xj, &v, nd)) < best)) { best = dd; *r = v; *s = 1; }
+            if ((all || w_aiba < 0) && ((dd = vtx_edge_sq(xi, xa, xb, &v, nd)) < best)) { best = dd; *r = 0; *s = v; }
+            if ((all || w_aiba > nn) && ((dd = vtx_edge_sq(xj, xa, xb, &v, nd)) < best)) { best = dd; *r = 1; *s = v; }
+            if ((all || w_aiji < 0) && ((dd = vtx_edge_sq(xa, xi, xj, &v, nd)) < best)) { best = dd; *r = v; *s = 0; }
+            if ((all || w_aiji > nn) && ((dd = vtx_edge_sq(xb, xi, xj, &v, nd)) < best)) { best = dd; *r = v; *s = 1; }
         }
         for (int k = 0; k < 3; ++k)
             d[k] = xi[k] * (1 - *r) + xj[k] * *r - xa[k] * ((TC)1.0 - *s) - xb[k] * *s;
@@ -1434,15 +1439,18 @@ struct Sim {
         TC w_iaca = dot3(d, tmp);
         cross3(xba, xia, tmp);
         TC w_baia = dot3(d, tmp);
+        *ba = 1;
+        *bb = *bc = 0;
+        const bool all = w_iaca >= 0 && w_baia >= 0 && nn - w_iaca - w_baia >= 0;
         if (nn > (TC)1e-24f && w_iaca >= 0 && w_baia >= 0 && nn - w_iaca - w_baia >= 0) {
             *bb = w_iaca / nn;
             *bc = w_baia / nn;
             *ba = 1 - *bb - *bc;
         } else {
             TC best = (TC)999999999, r, dd, N[3];
-            if (nn - w_iaca - w_baia < 0 && ((dd = vtx_edge_sq(xi, xb, xc, &r, N)) < best)) { best = dd; *bb = 1 - r; *bc = r; *ba = 0; }
-            if (w_iaca < 0 && ((dd = vtx_edge_sq(xi, xa, xc, &r, N)) < best)) { best = dd; *bb = 0; *bc = r; *ba = 1 - *bb - *bc; }
-            if (w_baia < 0 && ((dd = vtx_edge_sq(xi, xa, xb, &r, N)) < best)) { best = dd; *bb = r; *bc = 0; *ba = 1 - *bb - *bc; }
+            if ((all || nn - w_iaca - w_baia < 0) && ((dd = vtx_edge_sq(xi, xb, xc, &r, N)) < best)) { best = dd; *bb = 1 - r; *bc = r; *ba = 0; }
+            if ((all || w_iaca < 0) && ((dd = vtx_edge_sq(xi, xa, xc, &r, N)) < best)) { best = dd; *bb = 0; *bc = r; *ba = 1 - *bb - *bc; }
+            if ((all || w_baia < 0) && ((dd = vtx_edge_sq(xi, xa, xb, &r, N)) < best)) { best = dd; *bb = r; *bc = 0; *ba = 1 - *bb - *bc; }
         }
         for (int k = 0; k < 3; ++k) d[k] = xi[k] - xa[k] * *ba - xb[k] * *bb - xc[k] * *bc;
         return dot3(d, d);

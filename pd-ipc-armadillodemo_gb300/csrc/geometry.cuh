@@ -48,7 +48,11 @@ __device__ __forceinline__ R vtx_edge_sq(const R* v, const R* ea, const R* eb, R
     return dot3(d, d);
 }
 
-// EdgeEdgeSqDistance (cu:2177-2237): d = closest(a) - closest(b)
+// EdgeEdgeSqDistance (cu:2177-2237): d = closest(a) - closest(b).  For parallel and
+// degenerate edges (nn about 0) no weight may name a side: the reference then reads
+// unset weights; here the closest of the four ends counts.  Weights are set whatever
+// the input, and lie in [0, 1] for finite ones, so the distance is that of two points
+// of the edges: never below their separation along any direction.
 template <typename R>
 __device__ __forceinline__ R edge_edge_sq(const R* xi, const R* xj, const R* xa, const R* xb, R* r, R* s, R* d) {
     R xba[3], xji[3], xai[3], tmp[3];
@@ -61,21 +65,25 @@ __device__ __forceinline__ R edge_edge_sq(const R* xi, const R* xj, const R* xa,
     const R w_aiji = dot3(d, tmp);
     cross3(xai, xba, tmp);
     const R w_aiba = dot3(d, tmp);
+    *r = R(0);
+    *s = R(0);
     if (nn > R(1e-24f) && w_aiji >= R(0) && w_aiji <= nn && w_aiba >= R(0) && w_aiba <= nn) {
         *r = w_aiba / nn;
         *s = w_aiji / nn;
     } else {
         R best = R(999999999), dd, v;
-        if (w_aiba < R(0) && ((dd = vtx_edge_sq(xi, xa, xb, &v)) < best)) { best = dd; *r = R(0); *s = v; }
-        if (w_aiba > nn && ((dd = vtx_edge_sq(xj, xa, xb, &v)) < best)) { best = dd; *r = R(1); *s = v; }
-        if (w_aiji < R(0) && ((dd = vtx_edge_sq(xa, xi, xj, &v)) < best)) { best = dd; *r = v; *s = R(0); }
-        if (w_aiji > nn && ((dd = vtx_edge_sq(xb, xi, xj, &v)) < best)) { best = dd; *r = v; *s = R(1); }
+        const bool all = w_aiji >= R(0) && w_aiji <= nn && w_aiba >= R(0) && w_aiba <= nn;
+        if ((all || w_aiba < R(0)) && ((dd = vtx_edge_sq(xi, xa, xb, &v)) < best)) { best = dd; *r = R(0); *s = v; }
+        if ((all || w_aiba > nn) && ((dd = vtx_edge_sq(xj, xa, xb, &v)) < best)) { best = dd; *r = R(1); *s = v; }
+        if ((all || w_aiji < R(0)) && ((dd = vtx_edge_sq(xa, xi, xj, &v)) < best)) { best = dd; *r = v; *s = R(0); }
+        if ((all || w_aiji > nn) && ((dd = vtx_edge_sq(xb, xi, xj, &v)) < best)) { best = dd; *r = v; *s = R(1); }
     }
     for (int k = 0; k < 3; ++k) d[k] = xi[k] * (R(1) - *r) + xj[k] * *r - xa[k] * (R(1) - *s) - xb[k] * *s;
     return dot3(d, d);
 }
 
-// VertexTriangleDistance (cu:2239-2292): d = x - closest point on the triangle
+// VertexTriangleDistance (cu:2239-2292): d = x - closest point on the triangle.  A
+// degenerate triangle counts as its three edges (as in edge_edge_sq).
 template <typename R>
 __device__ __forceinline__ R vtx_tri(const R* xi, const R* xa, const R* xb, const R* xc, R* ba, R* bb, R* bc, R* d) {
     R xba[3], xca[3], xia[3], tmp[3];
@@ -88,19 +96,22 @@ __device__ __forceinline__ R vtx_tri(const R* xi, const R* xa, const R* xb, cons
     const R w_iaca = dot3(d, tmp);
     cross3(xba, xia, tmp);
     const R w_baia = dot3(d, tmp);
+    *ba = R(1);
+    *bb = *bc = R(0);
     if (nn > R(1e-24f) && w_iaca >= R(0) && w_baia >= R(0) && nn - w_iaca - w_baia >= R(0)) {
         *bb = w_iaca / nn;
         *bc = w_baia / nn;
         *ba = R(1) - *bb - *bc;
     } else {
         R best = R(999999999), r, dd;
-        if (nn - w_iaca - w_baia < R(0) && ((dd = vtx_edge_sq(xi, xb, xc, &r)) < best)) {
+        const bool all = w_iaca >= R(0) && w_baia >= R(0) && nn - w_iaca - w_baia >= R(0);
+        if ((all || nn - w_iaca - w_baia < R(0)) && ((dd = vtx_edge_sq(xi, xb, xc, &r)) < best)) {
             best = dd; *bb = R(1) - r; *bc = r; *ba = R(0);
         }
-        if (w_iaca < R(0) && ((dd = vtx_edge_sq(xi, xa, xc, &r)) < best)) {
+        if ((all || w_iaca < R(0)) && ((dd = vtx_edge_sq(xi, xa, xc, &r)) < best)) {
             best = dd; *bb = R(0); *bc = r; *ba = R(1) - *bb - *bc;
         }
-        if (w_baia < R(0) && ((dd = vtx_edge_sq(xi, xa, xb, &r)) < best)) {
+        if ((all || w_baia < R(0)) && ((dd = vtx_edge_sq(xi, xa, xb, &r)) < best)) {
             best = dd; *bb = r; *bc = R(0); *ba = R(1) - *bb - *bc;
         }
     }
