@@ -577,7 +577,7 @@ __device__ __forceinline__ void toi_rel(const int* ids, const V4<T>* __restrict_
 // to the exact test.
 template <typename T, bool kPT>
 __device__ __forceinline__ bool toi_maybe(const int* ids, const V4<T>* __restrict__ X0h, const V4<T>* __restrict__ X1h,
-                                          T slack) {
+                                          T slack, int max_iter) {
     T xh[4][3], dh[4][3], m = T(0);
     const V4<T> o = ld4(X0h, ids[0]);
 #pragma unroll
@@ -599,7 +599,7 @@ __device__ __forceinline__ bool toi_maybe(const int* ids, const V4<T>* __restric
     // (m bounds |x|), so the margins below keep it conservative; most pairs
     // settle here without loading anything more
     const T eps = m * T(1.0 / 1048576.0);
-    return !geo::ccd_trivial_approx<T, kPT>(xh, dh, T(4) * eps, T(8) * eps);
+    return !geo::ccd_trivial_approx<T, kPT>(xh, dh, T(4) * eps, T(8) * eps, max_iter > 0);
 }
 
 template <bool kPT>
@@ -612,10 +612,11 @@ __device__ __forceinline__ bool shares_vertex(const int4 c) {
 // parts, then exactly; no motion, or the CCD's box-gap exit).
 template <typename T, bool kPT>
 __device__ __forceinline__ bool toi_needs_ccd(const int4 c, const V4<T>* __restrict__ X0h, const V4<T>* __restrict__ X0l,
-                                              const V4<T>* __restrict__ X1h, const V4<T>* __restrict__ X1l, T slack) {
+                                              const V4<T>* __restrict__ X1h, const V4<T>* __restrict__ X1l, T slack,
+                                              int max_iter) {
     if (shares_vertex<kPT>(c)) return false;
     const int ids[4] = {c.x, c.y, c.z, c.w};
-    if (!toi_maybe<T, kPT>(ids, X0h, X1h, slack)) return false;
+    if (!toi_maybe<T, kPT>(ids, X0h, X1h, slack, max_iter)) return false;
     T x[4][3], dx[4][3];
     toi_rel<T>(ids, X0h, X0l, X1h, X1l, x, dx);
     if (!(kPT ? geo::pt_ccd_broad<T>(x, dx, slack) : geo::ee_ccd_broad<T>(x, dx, slack))) return false;
@@ -699,7 +700,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_toi_f64(int64_t n, const int4* __
         if (t < n) {
             const int4 c = cand[t];
             const int ids[4] = {c.x, c.y, c.z, c.w};
-            need = !shares_vertex<kPT>(c) && toi_maybe<float, kPT>(ids, X0h, X1h, wide);
+            need = !shares_vertex<kPT>(c) && toi_maybe<float, kPT>(ids, X0h, X1h, wide, max_iter);
             if (!need && per) per[t] = 1.0;
         }
         const unsigned m = __ballot_sync(0xffffffffu, need);
@@ -744,7 +745,7 @@ __global__ void __launch_bounds__(kBlock, kCandBlocks<T>) k_toi(int64_t n, const
         const int64_t step = (int64_t)gridDim.x * (kBlock / 32) * 32;
         for (int64_t base = ((int64_t)blockIdx.x * (kBlock / 32) + w) * 32; base < n; base += step) {
             const int64_t t = base + lane;
-            const bool need = t < n && toi_needs_ccd<T, kPT>(cand[t], X0h, X0l, X1h, X1l, (T)slack);
+            const bool need = t < n && toi_needs_ccd<T, kPT>(cand[t], X0h, X0l, X1h, X1l, (T)slack, max_iter);
             if (t < n && !need && per) per[t] = TC(1);
             const unsigned m = __ballot_sync(0xffffffffu, need);
             if (need) queue[w][qn + __popc(m & ((1u << lane) - 1u))] = t;

@@ -250,9 +250,10 @@ __device__ __forceinline__ bool ccd_ee_trivial(const R (*x)[3], const R (*dx)[3]
 // the exact ones per component.  The motion bound is taken eps_m larger and the
 // box gap eps_g smaller (eps_m >= 8 eps, eps_g >= 4 eps cover the mean
 // subtraction, the norms and the box corners), so a true result implies that the
-// exact test returns 1.
+// exact test returns 1.  `steps`: the exact test takes a conservative step
+// (max_iter > 0); without one only its opening lines return 1.
 template <typename R, bool kPT>
-__device__ __forceinline__ bool ccd_trivial_approx(const R (*x)[3], const R (*dx)[3], R eps_g, R eps_m) {
+__device__ __forceinline__ bool ccd_trivial_approx(const R (*x)[3], const R (*dx)[3], R eps_g, R eps_m, bool steps) {
     R mov[3], d[4][3];
     for (int k = 0; k < 3; ++k) mov[k] = (dx[0][k] + dx[1][k] + dx[2][k] + dx[3][k]) / R(4);
     for (int j = 0; j < 4; ++j)
@@ -269,8 +270,9 @@ __device__ __forceinline__ bool ccd_trivial_approx(const R (*x)[3], const R (*dx
     R gap = dsqrt(kPT ? box_gap2<R, 1, 3>(x, x + 1) : box_gap2<R, 2, 2>(x, x + 2)) - eps_g;
     if (gap > R(0) && R(0.81) * gap * gap > R(4) * maxd * maxd) return true;
     // the diagonals bound the distance, not the boxes' gap: where only they clear
-    // the bound, the test goes on to its first distance d, and returns 1 all the
-    // same since 0.9 d > 2 maxd
+    // the bound, the test goes on to its first distance d, and its first step returns
+    // 1 all the same since 0.9 d > 2 maxd
+    if (!steps) return false;
     gap = (kPT ? diagonal_gap<R, 1, 3>(x, x + 1) : diagonal_gap<R, 2, 2>(x, x + 2)) - R(2) * eps_g;
     return gap > R(0) && R(0.81) * gap * gap > R(4) * maxd * maxd;
 }

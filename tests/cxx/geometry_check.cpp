@@ -1,8 +1,12 @@
-// Checks the closest-point distances of csrc/geometry.cuh, compiled for the host, where
-// their weights degenerate: parallel, collinear, coincident and zero-length edges,
-// triangles without area, NaN.  The weights go in poisoned and must come out set, in
-// [0, 1] for finite input, with the distance of the best end (edge) in long double.
-// Prints "ok" or what failed.
+// Checks of csrc/geometry.cuh, compiled for the host.  Prints "ok" or what failed.
+//   * The closest-point distances where their weights degenerate: parallel, collinear,
+//     coincident and zero-length edges, triangles without area, NaN.  The weights go in
+//     poisoned and must come out set, in [0, 1] for finite input, with the distance of
+//     the best end (edge) in long double.
+//   * The FP32 exit of the time-of-impact filters on rounded coordinates: wherever it
+//     says 1, the FP64 test must return 1, near its margins, far from the origin, on
+//     parallel edges, parted along an axis or a diagonal, with conservative steps and
+//     without.
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -86,8 +90,64 @@ static bool distances() {
     return true;
 }
 
+template <bool kPT>
+static bool filter() {
+    std::mt19937 g(11);
+    std::uniform_real_distribution<double> u(-1.0, 1.0);
+    int settled[2] = {0, 0};
+    for (int trial = 0; trial < 200000; ++trial) {
+        const double far = trial % 3 == 0 ? 0.0 : trial % 3 == 1 ? 10.0 : 1000.0, size = 0.01;
+        double o[3], dir[3] = {0, 0, 0}, x0[4][3], x1[4][3];
+        for (double& v : o) v = far * u(g);
+        // the second primitive is moved along an axis or a diagonal by about the
+        // distance at which the exit begins, or less
+        const int k = g() % 3, diag = g() % 3;
+        dir[k] = 1.0;
+        if (diag) dir[(k + 1) % 3] = diag == 1 ? 1.0 : -1.0;
+        const double move = size * 0.5, gap = move * u(g) * 8.0;
+        const bool flat = g() % 2;  // parallel edges, motion without a spread of its own
+        for (int j = 0; j < 4; ++j) {
+            const bool second = kPT ? j > 0 : j > 1;
+            for (int c = 0; c < 3; ++c) {
+                x0[j][c] = o[c] + (flat ? (j & 1) * (c == (k + 2) % 3) * size : size * 0.2 * u(g)) + second * gap * dir[c];
+                x1[j][c] = x0[j][c] + move * (second ? -0.3 : 0.3) * dir[c] + 0.1 * move * u(g);
+            }
+        }
+        float xh[4][3], dh[4][3], m = 0.f;
+        for (int j = 0; j < 4; ++j)
+            for (int c = 0; c < 3; ++c) {  // as toi_maybe (collision_kernels.cu) forms them
+                xh[j][c] = (float)x0[j][c] - (float)x0[0][c];
+                dh[j][c] = (float)x1[j][c] - (float)x0[j][c];
+                m = std::fmax(m, std::fmax(std::fabs((float)x0[j][c]), std::fabs((float)x1[j][c])));
+            }
+        const float eps = m / 1048576.f;
+        for (int steps = 0; steps < 2; ++steps) {
+            if (!geo::ccd_trivial_approx<float, kPT>(xh, dh, 4 * eps, 8 * eps, steps != 0)) continue;
+            ++settled[steps];
+            double x[4][3], dx[4][3];
+            for (int j = 0; j < 4; ++j)
+                for (int c = 0; c < 3; ++c) {
+                    x[j][c] = x0[j][c];
+                    dx[j][c] = x1[j][c] - x0[j][c];
+                }
+            const int it = steps ? 10 : 0;
+            const double toi = kPT ? geo::ccd_pt<double>(x, dx, 0.1, it) : geo::ccd_ee<double>(x, dx, 0.1, it);
+            if (toi != 1.0) {
+                printf("filter %d, trial %d, steps %d: the exact test gives %.17g\n", kPT, trial, steps, toi);
+                return false;
+            }
+        }
+    }
+    if (settled[0] < 1000 || settled[1] < settled[0] + 100) {  // the cases reach both exits
+        printf("filter %d: %d and %d settled\n", kPT, settled[0], settled[1]);
+        return false;
+    }
+    return true;
+}
+
 int main() {
     if (!distances<float>() || !distances<double>()) return 1;
+    if (!filter<true>() || !filter<false>()) return 1;
     printf("ok\n");
     return 0;
 }
