@@ -21,9 +21,9 @@
 #include <map>
 #include <mutex>
 #include <string>
-#include <thread>
 #include <type_traits>
 
+#include "host_copy.h"
 #include "kernels.cuh"
 #include "persistent.h"
 #include "solver.h"
@@ -739,28 +739,9 @@ public:
         PD_CK(cudaStreamSynchronize(s_));
         return PDIPC_OK;
     }
-    static void copy_host(double* dst, const double* src, size_t bytes) {
-        constexpr size_t kPart = (size_t)1 << 20;  // below, a thread costs more than it saves
-        const size_t parts = std::min<size_t>(6, bytes / kPart + 1);
-        const size_t len = (bytes / parts + 63) / 64 * 64;
-        auto part = [=](size_t k) {
-            const size_t b = std::min(bytes, k * len), e = std::min(bytes, b + len);
-            std::memcpy(reinterpret_cast<char*>(dst) + b, reinterpret_cast<const char*>(src) + b, e - b);
-        };
-        std::vector<std::thread> th;
-        size_t started = 1;
-        try {
-            for (; started < parts; ++started) th.emplace_back(part, started);
-        } catch (...) {  // no thread to be had: this one copies the rest
-        }
-        part(0);
-        for (size_t k = started; k < parts; ++k) part(k);
-        for (std::thread& t : th) t.join();
-    }
     pdipc_status download_vec(const V4<TC>* src, double* dst, int n, std::string& err) {
         launch_pack(raw_, src, n, s_);
-        volatile char* page = reinterpret_cast<volatile char*>(dst);
-        for (size_t b = 0; b < sizeof(double) * 3 * (size_t)n; b += 4096) page[b] = 0;
+        map_pages(dst, sizeof(double) * 3 * (size_t)n);
         PD_CK(cudaMemcpyAsync(dst, raw_, sizeof(double) * 3 * (size_t)n, cudaMemcpyDeviceToHost, s_));
         PD_CK(cudaStreamSynchronize(s_));
         return PDIPC_OK;
