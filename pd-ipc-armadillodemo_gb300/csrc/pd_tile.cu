@@ -38,6 +38,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "smem_limit.h"
 #include "svd3.cuh"
 #include "tile_device.cuh"
 
@@ -892,12 +893,7 @@ int tile_residents(int R, bool tets, bool pairs, int threads, size_t smem, int s
     const void* f = tile_kernel<T, S>(R, tets, pairs);
     if (!f || threads > kTileMaxWarps * 32) return 0;
     smem = cta_smem(pairs, smem);
-    // the kernel's limit is raised only: other contexts may hold larger tiles
-    cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) return 0;
-    if ((size_t)fa.maxDynamicSharedSizeBytes < smem &&
-        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return 0;
+    if (allow_smem(f, smem) != cudaSuccess) return 0;
     int per_sm = 0;
     const int per_cta = pairs ? kPairTiles : 1;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads * per_cta, smem) != cudaSuccess)
@@ -945,11 +941,7 @@ bool tile_cluster_fits(int tiles, int threads, size_t smem) {
     } else {
         const void* f = cluster_kernel<T, S>();
         if (threads > kTileMaxWarps * 32 || tiles > kTileCluster) return false;
-        cudaFuncAttributes fa;
-        if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) return false;
-        if ((size_t)fa.maxDynamicSharedSizeBytes < smem &&
-            cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return false;
+        if (allow_smem(f, smem) != cudaSuccess) return false;
         if (cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return false;
         cudaLaunchAttribute at;
         const cudaLaunchConfig_t c = cluster_config(tiles, threads, smem, nullptr, &at);

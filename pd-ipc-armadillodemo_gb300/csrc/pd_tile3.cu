@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "smem_limit.h"
 #include "tile_device.cuh"
 
 namespace pdipc {
@@ -255,11 +256,7 @@ __global__ void __launch_bounds__(kTile3Warps * 96, 1) k_pd_tile3(const __grid_c
 int tile3_residents(int threads, size_t smem, int sms) {
     const void* f = (const void*)k_pd_tile3;
     if (threads > kTile3Warps * 96) return 0;
-    cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) return 0;
-    if ((size_t)fa.maxDynamicSharedSizeBytes < smem &&
-        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return 0;
+    if (allow_smem(f, smem) != cudaSuccess) return 0;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, threads, smem) != cudaSuccess) return 0;
     return per_sm * sms;

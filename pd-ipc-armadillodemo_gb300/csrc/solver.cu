@@ -26,6 +26,7 @@
 #include "host_copy.h"
 #include "kernels.cuh"
 #include "persistent.h"
+#include "smem_limit.h"
 #include "solver.h"
 #include "tile.h"
 
@@ -1628,10 +1629,7 @@ private:
                     const void* f =
                         persistent_kernel(kCorrection, smem_mat, c.ch.band, c.band_param, c.ch.l1_gather, R, H.ntet > 0);
                     if (!f) continue;
-                    cudaFuncAttributes fa;  // the kernel's limit is raised only: other contexts may need more
-                    PD_CK(cudaFuncGetAttributes(&fa, f));
-                    if ((size_t)fa.maxDynamicSharedSizeBytes < c.sm)
-                        PD_CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.sm));
+                    PD_CK(allow_smem(f, c.sm));
                     int per_sm = 0;
                     PD_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, c.threads, c.sm));
                     if (per_sm < 1) continue;
