@@ -522,17 +522,25 @@ private:
     // by timing every candidate with CUDA events at initialize, on the
     // predicted first step of the current state (restored afterwards).  The
     // choice is cached by shape for the process: later contexts of the same
-    // shape take it without timing.  Every candidate computes the same
+    // shape, with the same configurations to choose from, take it without timing.  Every candidate computes the same
     // iteration; they differ in launch shape and, on the band path, in where a
     // row's sum splits between own and halo entries.
     pdipc_status autotune(const HostTables& H, std::string& err) {
         static std::mutex mu;
         static std::map<std::string, Tuned> cache;
-        const std::string key = std::to_string(sizeof(T)) + "/" + std::to_string(sizeof(TC)) + "/" +
-                                std::to_string(d_.nsim) + "/" + std::to_string(d_.ntot) + "/" +
-                                std::to_string(d_.npatch) + "/" + std::to_string(sell_entries_) + "/" +
-                                std::to_string(c_.lg) + "/" + std::to_string(c_.cheby) + "/" +
-                                std::to_string(prm_.persistent) + "/" + std::to_string(d_.ntet);
+        std::string key = std::to_string(sizeof(T)) + "/" + std::to_string(sizeof(TC)) + "/" +
+                          std::to_string(d_.nsim) + "/" + std::to_string(d_.ntot) + "/" +
+                          std::to_string(d_.npatch) + "/" + std::to_string(sell_entries_) + "/" +
+                          std::to_string(c_.lg) + "/" + std::to_string(c_.cheby) + "/" +
+                          std::to_string(prm_.persistent) + "/" + std::to_string(d_.ntet) + "/" +
+                          std::to_string(prm_.pd_group_ctas) + "/" + std::to_string(prm_.instance_stop);
+        // and the configurations that fit: a numbering of the same mesh, for one, may
+        // leave out some that another has
+        if (tile_.ok)
+            key += "/t" + std::to_string(tile_.tiles.size()) + "," + std::to_string(tile_.rows_per_thread) + "," +
+                   std::to_string(tile_.groups.size());
+        for (const PlanChoice& c : plan_choices_)
+            key += "/" + std::to_string(c.rows_per_thread * 8 + c.band * 4 + c.l1_gather * 2 + c.local_sync);
         Tuned best{current_choice(), c_.cand_grid, c_.trav_block, c_.expand_block};
         bool cached = false;
         {
