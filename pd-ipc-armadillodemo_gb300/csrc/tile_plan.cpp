@@ -10,9 +10,9 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <new>
 #include <numeric>
-#include <system_error>
 #include <thread>
 #include <unordered_map>
 
@@ -541,8 +541,8 @@ void try_plan(const HostTables& H, const TileLimits& lim, int order_block, bool 
         for (int k = std::min({nt / 16, 7, (int)std::thread::hardware_concurrency() - 1}); k > 0; --k) {
             try {
                 team.emplace_back(work);
-            } catch (const std::system_error&) {
-                break;  // fewer threads
+            } catch (const std::exception&) {  // no thread or no memory for one (those that run are joined below)
+                break;
             }
         }
         work();
