@@ -168,9 +168,12 @@ typedef struct {
     int32_t pd_rows_per_thread; /* persistent PD solve: rows per thread (slices per warp); 0: one launch
                                    per sweep */
     int32_t pd_ctas;            /* tiles or CTAs of the persistent solve */
-    int32_t pd_band;            /* 1: the iterate's column band in shared memory */
-    int32_t pd_l1_gather;       /* 1: gathers through L1 */
-    int32_t pd_local_sync;      /* 1: neighbour waits, 0: grid barriers */
+    int32_t pd_band;            /* 1: the iterate in shared memory: row blocks with their column band, tiles
+                                   in mixed precision */
+    int32_t pd_l1_gather;       /* row blocks: 1: gathers through L1 (tiles, which gather from shared
+                                   memory: 1) */
+    int32_t pd_local_sync;      /* row blocks: 1: neighbour waits, 0: grid barriers (tiles, which wait for
+                                   the words they read: 1) */
     int32_t cand_grid;          /* blocks of the time-of-impact and contact kernels (grid-stride) */
     int32_t traverse_block;     /* threads per block of the broad-phase traversal */
     int32_t expand_block;       /* threads per block of the candidate expansion */
@@ -180,7 +183,8 @@ typedef struct {
     double pd_default_ms;       /* the same with the default configuration */
     double collision_ms;        /* broad phase + time of impact + contact, chosen shapes */
     double collision_default_ms;/* the same with the default shapes */
-    int32_t reserved[8];
+    int32_t pd_tiles;           /* 1: the persistent solve runs over tiles, 0: over row blocks (or not at all) */
+    int32_t reserved[7];
 } pdipc_tuning;
 
 /* Fill *p with the reference defaults listed beside each field. */

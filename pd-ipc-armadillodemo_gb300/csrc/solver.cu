@@ -426,6 +426,7 @@ private:
     };
 
     void fill_tuning_record() {
+        tuning_.pd_tiles = tile_on_;
         tuning_.pd_rows_per_thread = tile_on_ ? tile_.rows_per_thread : plan_.enabled ? plan_.rows_per_thread : 0;
         tuning_.pd_ctas = tile_on_ ? (int)tile_.tiles.size() : plan_.enabled ? plan_.ctas : 0;
         tuning_.pd_launches = tile_on_ ? (int)tile_.groups.size() : plan_.enabled ? (int)groups_.size() : 0;

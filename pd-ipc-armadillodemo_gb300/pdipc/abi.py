@@ -183,7 +183,8 @@ class Tuning(C.Structure):
         ("pd_default_ms", C.c_double),
         ("collision_ms", C.c_double),
         ("collision_default_ms", C.c_double),
-        ("reserved", C.c_int32 * 8),
+        ("pd_tiles", C.c_int32),
+        ("reserved", C.c_int32 * 7),
     ]
 
     def as_dict(self) -> dict:
