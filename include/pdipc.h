@@ -90,10 +90,13 @@ typedef struct {
                                 and mixed only: 2 neighbour waits, L2-only
                                 gathers; 3 grid-wide barriers, gathers through L1; 4 neighbour waits,
                                 gathers through L1 (no band); 0 one launch per sweep */
-    int wait_limit_us;       /* limit of every device-side wait of the persistent solve (exchanged rows,
-                                neighbour flags, grid barrier, halo copies), in microseconds at the maximum SM clock; past
-                                it the launch ends and the step returns PDIPC_ERR_CUDA; 0 = 2 s.  The
-                                reference has no device-side waits (one launch per kernel). */
+    int wait_limit_us;       /* limit of the device-side waits of the persistent solve (polls of exchanged
+                                rows, neighbour flags, grid barrier, halo copies), in microseconds at the
+                                maximum SM clock; past it the launch ends and the step returns
+                                PDIPC_ERR_CUDA; 0 = 2 s.  Without effect where the tiles form one
+                                thread-block cluster (a single launch of 16 tiles or fewer, FP32 arithmetic):
+                                nothing is polled there, the sweeps end at the cluster's hardware barrier.
+                                The reference has no device-side waits (one launch per kernel). */
     int autotune;            /* 1: choose launch shapes by timing candidates at pdipc_initialize (see
                                 pdipc_get_tuning); 0: the built-in defaults */
     int ccd_mode;            /* 0: the reference's additive CCD (PdIpcGpuFunc.cu:2460-2607); 1: plus an FP64
@@ -321,8 +324,8 @@ pdipc_status pdipc_initialize(pdipc_ctx* ctx);
 pdipc_status pdipc_step(pdipc_ctx* ctx, int nsteps);
 
 /* Change pdipc_params.wait_limit_us of an initialised context (no counterpart in
- * the reference, whose kernels never wait on one another).  A launch whose wait
- * runs past the limit ends early, the step returns PDIPC_ERR_CUDA with the state
+ * the reference, whose kernels never wait on one another).  A launch whose polls
+ * run past the limit ends early, the step returns PDIPC_ERR_CUDA with the state
  * of a partial step, and the context stays usable: set the state again
  * (pdipc_set_state / pdipc_load / pdipc_reset) and step on. */
 pdipc_status pdipc_set_wait_limit(pdipc_ctx* ctx, int wait_limit_us);

@@ -32,9 +32,10 @@
 // phase p (the plan makes reading mutual).  In a cluster no tile starts a phase
 // before all have ended the one before, so two copies of the iterate do.
 //
-// Every wait is clock-bounded: past the limit it raises kErrBarrier, the tile
-// leaves together at its next barrier, and the others' waits end on the error
-// or their own limit.
+// Every poll of a word or a count is clock-bounded: past the limit it raises
+// kErrBarrier, the tile leaves together at its next barrier, and the others' waits end
+// on the error or their own limit.  A cluster polls nothing and has no such limit: its
+// CTAs run together, each comes to every barrier, and none leaves before the last.
 #include <algorithm>
 #include <type_traits>
 

@@ -42,7 +42,7 @@ struct TileArgs {
     int cheby;
     T relax;
     T omega[kMaxCheby];
-    long long timeout;  // limit of a wait in clock cycles
+    long long timeout;  // limit of a poll in clock cycles (a cluster polls nothing)
     // state, as in PersistArgs
     V4<S>* P;
     V4<T>* Ph;

@@ -37,7 +37,8 @@ __device__ __forceinline__ void st_word(TileWord* p, unsigned long long lo, unsi
         : "memory");
 }
 // ---- thread-block cluster: the same place in another CTA's shared memory, and the
-// barrier of all its threads (release, acquire: it orders the remote writes) ----
+// barrier of all its threads (release, acquire: it orders the remote writes; without a
+// limit, since the hardware runs the CTAs together and none leaves early) ----
 __device__ __forceinline__ unsigned remote_addr(const void* p, unsigned rank) {
     unsigned r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
