@@ -1951,7 +1951,6 @@ private:
                 lim.cluster_rows = kTileClusterRows;
             }
             lim.pairs = !fp64;
-            lim.pairs = !fp64;
             lim.pair_rows = kPairRows;
             build_tile_plan(H, lim, order_block, tile_);
             tile_.smem_bytes = (tile_.smem_bytes + 15) / 16 * 16;

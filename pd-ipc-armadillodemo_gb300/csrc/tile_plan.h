@@ -1,5 +1,5 @@
 // tile_plan.h — partition of the simulated rows into tiles for the tiled
-// persistent solve (pd_tile.cuh) and every table a tile reads.  Host only.
+// persistent solve (pd_tile.cu, pd_tile3.cu) and every table a tile reads.  Host only.
 #pragma once
 
 #include <cstdint>
