@@ -97,7 +97,8 @@ __global__ void k_adj_weights(int nsim, int nt, T relax, const AdjScales<T> sc, 
 // One component of a row per thread, a block's three warps the x, y and z of the
 // same 32 rows (as k_sweep3: with a row per thread an FP64 sweep of few rows is
 // one long chain per scheduler; a 128x128 rollout of two steps and its
-// gradients 70.4 ms, split 56.3).
+// gradients 70.4 ms, split 56.3).  13.9 us a sweep at 128x128, twice a forward sweep:
+// the columns of N^T and N and the spring neighbours are all gathered.
 constexpr int kRows3 = 32;
 template <typename T>
 __global__ void __launch_bounds__(3 * kRows3) k_adj_sweep(
