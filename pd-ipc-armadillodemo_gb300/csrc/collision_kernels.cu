@@ -575,9 +575,12 @@ __device__ __forceinline__ void toi_rel(const int* ids, const V4<T>* __restrict_
 // rounding, |low| <= 2^-24 |x| and the roundings here: < 2^-18 of the largest
 // coordinate; then the CCD's box-gap exit).  A NaN or infinite coordinate goes on
 // to the exact test.
-template <typename T, bool kPT>
+// kSteps: the exact test takes a conservative step (max_iter > 0).  A parameter of the
+// kernels: as a test at run time it cost 7% of the pass (40 cloths in flight 0.624 ->
+// 0.668 ms a step).
+template <typename T, bool kPT, bool kSteps>
 __device__ __forceinline__ bool toi_maybe(const int* ids, const V4<T>* __restrict__ X0h, const V4<T>* __restrict__ X1h,
-                                          T slack, int max_iter) {
+                                          T slack) {
     T xh[4][3], dh[4][3], m = T(0);
     const V4<T> o = ld4(X0h, ids[0]);
 #pragma unroll
@@ -599,7 +602,7 @@ __device__ __forceinline__ bool toi_maybe(const int* ids, const V4<T>* __restric
     // (m bounds |x|), so the margins below keep it conservative; most pairs
     // settle here without loading anything more
     const T eps = m * T(1.0 / 1048576.0);
-    return !geo::ccd_trivial_approx<T, kPT>(xh, dh, T(4) * eps, T(8) * eps, max_iter > 0);
+    return !geo::ccd_trivial_approx<T, kPT>(xh, dh, T(4) * eps, T(8) * eps, kSteps);
 }
 
 template <bool kPT>
@@ -610,13 +613,12 @@ __device__ __forceinline__ bool shares_vertex(const int4 c) {
 // Mixed mode, stage 1 of a candidate: false when its time of impact is 1
 // without any CCD iteration (shared vertex; the filters above on the high
 // parts, then exactly; no motion, or the CCD's box-gap exit).
-template <typename T, bool kPT>
+template <typename T, bool kPT, bool kSteps>
 __device__ __forceinline__ bool toi_needs_ccd(const int4 c, const V4<T>* __restrict__ X0h, const V4<T>* __restrict__ X0l,
-                                              const V4<T>* __restrict__ X1h, const V4<T>* __restrict__ X1l, T slack,
-                                              int max_iter) {
+                                              const V4<T>* __restrict__ X1h, const V4<T>* __restrict__ X1l, T slack) {
     if (shares_vertex<kPT>(c)) return false;
     const int ids[4] = {c.x, c.y, c.z, c.w};
-    if (!toi_maybe<T, kPT>(ids, X0h, X1h, slack, max_iter)) return false;
+    if (!toi_maybe<T, kPT, kSteps>(ids, X0h, X1h, slack)) return false;
     T x[4][3], dx[4][3];
     toi_rel<T>(ids, X0h, X0l, X1h, X1l, x, dx);
     if (!(kPT ? geo::pt_ccd_broad<T>(x, dx, slack) : geo::ee_ccd_broad<T>(x, dx, slack))) return false;
@@ -673,7 +675,7 @@ __global__ void k_round(int n, const V4<double>* __restrict__ A, V4<float>* __re
 // FP32 filters on rounded positions settle those, warps queue the rest and run
 // the FP64 test on 32 at a time.  A filter only drops candidates whose FP64
 // test gives 1, so the minimum and every per-candidate time keep their bits.
-template <bool kPT>
+template <bool kPT, bool kSteps>
 __global__ void __launch_bounds__(kBlock, 4) k_toi_f64(int64_t n, const int4* __restrict__ cand,
                                                        const V4<double>* __restrict__ X0,
                                                        const V4<double>* __restrict__ X1,
@@ -700,7 +702,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_toi_f64(int64_t n, const int4* __
         if (t < n) {
             const int4 c = cand[t];
             const int ids[4] = {c.x, c.y, c.z, c.w};
-            need = !shares_vertex<kPT>(c) && toi_maybe<float, kPT>(ids, X0h, X1h, wide, max_iter);
+            need = !shares_vertex<kPT>(c) && toi_maybe<float, kPT, kSteps>(ids, X0h, X1h, wide);
             if (!need && per) per[t] = 1.0;
         }
         const unsigned m = __ballot_sync(0xffffffffu, need);
@@ -729,7 +731,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_toi_f64(int64_t n, const int4* __
 // FP64 time of impact.  The stage-1 tests settle most candidates; each warp
 // queues the rest in shared memory and runs the CCD iterations on 32 of them
 // at a time, so they run on full warps.
-template <typename T, typename TC, bool kPT, bool kRel>
+template <typename T, typename TC, bool kPT, bool kRel, bool kSteps>
 __global__ void __launch_bounds__(kBlock, kCandBlocks<T>) k_toi(int64_t n, const int4* __restrict__ cand,
                                                 const V4<TC>* __restrict__ X0, const V4<TC>* __restrict__ X1,
                                                 const V4<T>* __restrict__ X0h, const V4<T>* __restrict__ X0l,
@@ -745,7 +747,7 @@ __global__ void __launch_bounds__(kBlock, kCandBlocks<T>) k_toi(int64_t n, const
         const int64_t step = (int64_t)gridDim.x * (kBlock / 32) * 32;
         for (int64_t base = ((int64_t)blockIdx.x * (kBlock / 32) + w) * 32; base < n; base += step) {
             const int64_t t = base + lane;
-            const bool need = t < n && toi_needs_ccd<T, kPT>(cand[t], X0h, X0l, X1h, X1l, (T)slack, max_iter);
+            const bool need = t < n && toi_needs_ccd<T, kPT, kSteps>(cand[t], X0h, X0l, X1h, X1l, (T)slack);
             if (t < n && !need && per) per[t] = TC(1);
             const unsigned m = __ballot_sync(0xffffffffu, need);
             if (need) queue[w][qn + __popc(m & ((1u << lane) - 1u))] = t;
@@ -1225,31 +1227,41 @@ void launch_expand(const Dev<T, TC>& d, const int64_t* opt, const int64_t* oee, 
     k_expand<<<blocks_for(d.nPairs, b), b, 0, s>>>(d.nPairs, d.Pairs, d.pfPtr, d.pfIdx, d.ppPtr, d.ppIdx, d.pePtr,
                                                    d.peIdx, d.Faces, d.Edges, opt, oee, d.PT, d.EE);
 }
-template <typename T, typename TC>
-void launch_toi(const Dev<T, TC>& d, Pos<T, TC> X0, Pos<T, TC> X1, const SolverConsts& c, TC* per_pt,
-                TC* per_ee, cudaStream_t s) {
+// the reference's additive CCD over both lists
+template <typename T, typename TC, bool kSteps>
+static void launch_toi_additive(const Dev<T, TC>& d, Pos<T, TC> X0, Pos<T, TC> X1, const SolverConsts& c, TC* per_pt,
+                                TC* per_ee, cudaStream_t s) {
     constexpr bool kRel = sizeof(T) == 4 && sizeof(TC) == 8;
     if constexpr (std::is_same<T, double>::value) {
-        if (c.ccd_mode != 2 && d.nPT + d.nEE > 0) {
+        if (d.nPT + d.nEE > 0) {
             k_round<<<blocks_for(d.ntot), kBlock, 0, s>>>(d.ntot, X0.x, d.F0, X1.x, d.F1, d.Gate);
             if (d.nPT > 0)
-                k_toi_f64<true><<<grid_cap(d.nPT, kBlock, c.cand_grid), kBlock, 0, s>>>(
+                k_toi_f64<true, kSteps><<<grid_cap(d.nPT, kBlock, c.cand_grid), kBlock, 0, s>>>(
                     d.nPT, d.PT, X0.x, X1.x, d.F0, d.F1, c.ccd_slack, c.ccd_eta, c.ccd_max_iter, per_pt, d.ToiMin,
                     d.Gate);
             if (d.nEE > 0)
-                k_toi_f64<false><<<grid_cap(d.nEE, kBlock, c.cand_grid), kBlock, 0, s>>>(
+                k_toi_f64<false, kSteps><<<grid_cap(d.nEE, kBlock, c.cand_grid), kBlock, 0, s>>>(
                     d.nEE, d.EE, X0.x, X1.x, d.F0, d.F1, c.ccd_slack, c.ccd_eta, c.ccd_max_iter, per_ee, d.ToiMin,
                     d.Gate);
         }
-    } else if (c.ccd_mode != 2) {  // the reference's additive CCD
+    } else {
+        constexpr bool kS = kSteps || !kRel;  // (the FP32 mode has no filter that depends on it)
         if (d.nPT > 0)
-            k_toi<T, TC, true, kRel><<<grid_cap(d.nPT, kBlock, c.cand_grid), kBlock, 0, s>>>(
+            k_toi<T, TC, true, kRel, kS><<<grid_cap(d.nPT, kBlock, c.cand_grid), kBlock, 0, s>>>(
                 d.nPT, d.PT, X0.x, X1.x, X0.hi, X0.lo, X1.hi, X1.lo, (TC)c.ccd_slack, (TC)c.ccd_eta,
                 c.ccd_max_iter, per_pt, d.ToiMin, d.Gate);
         if (d.nEE > 0)
-            k_toi<T, TC, false, kRel><<<grid_cap(d.nEE, kBlock, c.cand_grid), kBlock, 0, s>>>(
+            k_toi<T, TC, false, kRel, kS><<<grid_cap(d.nEE, kBlock, c.cand_grid), kBlock, 0, s>>>(
                 d.nEE, d.EE, X0.x, X1.x, X0.hi, X0.lo, X1.hi, X1.lo, (TC)c.ccd_slack, (TC)c.ccd_eta,
                 c.ccd_max_iter, per_ee, d.ToiMin, d.Gate);
+    }
+}
+template <typename T, typename TC>
+void launch_toi(const Dev<T, TC>& d, Pos<T, TC> X0, Pos<T, TC> X1, const SolverConsts& c, TC* per_pt,
+                TC* per_ee, cudaStream_t s) {
+    if (c.ccd_mode != 2) {
+        if (c.ccd_max_iter > 0) launch_toi_additive<T, TC, true>(d, X0, X1, c, per_pt, per_ee, s);
+        else launch_toi_additive<T, TC, false>(d, X0, X1, c, per_pt, per_ee, s);
     }
     if (c.ccd_mode == 1) {  // the FP64 cubic may lower it
         if (d.nPT > 0)
